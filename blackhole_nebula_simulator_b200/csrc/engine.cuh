@@ -19,6 +19,7 @@ constexpr int MAX_LEVELS = 16;
 // perm[k] of the caller's order; entries are sorted positions.
 struct Lists {
   int64_t n = 0, total = 0;
+  int64_t longest = 0;          // entries of the longest row
   int64_t gen = 0;              // builds so far (the sorted order changes with every build)
   int32_t* perm = nullptr;      // sorted position -> caller index
   int32_t* inv_perm = nullptr;  // caller index -> sorted position

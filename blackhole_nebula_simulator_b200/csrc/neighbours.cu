@@ -710,14 +710,120 @@ __global__ void k_export_counts(int64_t n, const int32_t* __restrict__ inv_perm,
   cnt_o[i] = off_s[k + 1] - off_s[k];
 }
 
-__global__ void k_export_fill(int64_t n, const int32_t* __restrict__ perm,
-                              const int64_t* __restrict__ off_s, const int32_t* __restrict__ idx_s,
-                              const int64_t* __restrict__ off_o, int64_t* __restrict__ idx_o) {
-  int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  int64_t i = perm[k];
-  int64_t dst = off_o[i];
-  for (int64_t e = off_s[k]; e < off_s[k + 1]; ++e) idx_o[dst++] = perm[idx_s[e]];
+// Ascending sort of 32 K keys held by one warp, K per lane (element lane K + r in v[r]): a bitonic
+// network whose merges start with the mirrored comparison (element e against e ^ (size - 1)), so
+// that every comparison is ascending.  Strides below K stay within a lane, the others are
+// shuffles.
+template <int K>
+__device__ __forceinline__ void warp_sort(int32_t (&v)[K], int lane) {
+  const unsigned FULL = 0xffffffffu;
+#pragma unroll
+  for (int size = 2; size <= 32 * K; size *= 2) {
+    if (size <= K) {
+#pragma unroll
+      for (int r = 0; r < K; ++r) {
+        const int o = r ^ (size - 1);
+        if (o > r) {
+          const int32_t a = v[r], b = v[o];
+          v[r] = min(a, b);
+          v[o] = max(a, b);
+        }
+      }
+    } else {
+      const int m = size / K - 1;
+      const bool low = lane < (lane ^ m);
+      int32_t w[K];
+#pragma unroll
+      for (int r = 0; r < K; ++r) w[r] = __shfl_xor_sync(FULL, v[K - 1 - r], m);
+#pragma unroll
+      for (int r = 0; r < K; ++r) v[r] = low ? min(v[r], w[r]) : max(v[r], w[r]);
+    }
+#pragma unroll
+    for (int stride = size / 4; stride > 0; stride /= 2) {
+      if (stride < K) {
+#pragma unroll
+        for (int r = 0; r < K; ++r)
+          if ((r & stride) == 0) {
+            const int32_t a = v[r], b = v[r | stride];
+            v[r] = min(a, b);
+            v[r | stride] = max(a, b);
+          }
+      } else {
+        const int m = stride / K;
+        const bool low = (lane & m) == 0;
+#pragma unroll
+        for (int r = 0; r < K; ++r) {
+          const int32_t o = __shfl_xor_sync(FULL, v[r], m);
+          v[r] = low ? min(v[r], o) : max(v[r], o);
+        }
+      }
+    }
+  }
+}
+
+// One row of at most 32 K entries: sorted positions to caller indices, sorted, written 32
+// consecutive entries a store through `stage` (33 words of 32, so both sides are conflict-free).
+template <int K>
+__device__ __forceinline__ void export_row(const int32_t* __restrict__ src, int len,
+                                           const int32_t* __restrict__ perm, int32_t* stage,
+                                           int64_t* __restrict__ dst, int lane) {
+  int32_t v[K];
+#pragma unroll
+  for (int r = 0; r < K; ++r) v[r] = 32 * r + lane < len ? ld_stream(src + 32 * r + lane) : -1;
+#pragma unroll
+  for (int r = 0; r < K; ++r) v[r] = v[r] >= 0 ? perm[v[r]] : INT32_MAX;
+  warp_sort<K>(v, lane);
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    const int e = lane * K + r;
+    stage[e + (e >> 5)] = v[r];
+  }
+  __syncwarp();
+  for (int t = lane; t < len; t += 32) dst[t] = stage[t + (t >> 5)];
+  __syncwarp();
+}
+
+// Rows in the caller's order and numbering, each ascending: one warp per row, sorted in registers.
+// Bound by the network's shuffles and minima; the entries are read and written once.  Building
+// and exporting the lists of the 1M torus (160M entries) takes 5.56 ms, of a 4,096-particle
+// cloud 0.52 ms; with rows filled by one thread each and sorted as 64-bit keys by a segmented
+// device sort it was 76.5 and 0.90 ms.  The network is chosen by the row's length; a row over
+// EXPORT_MAX entries (the registers of the largest network) goes unsorted to `keys` and into the
+// segment list, for the device sort.
+constexpr int EXPORT_MAX = 1024;
+constexpr int EXPORT_WARPS = 8;
+
+__global__ void __launch_bounds__(EXPORT_WARPS * 32) k_export_rows(
+    int64_t n, const int32_t* __restrict__ perm, const int64_t* __restrict__ off_s,
+    const int32_t* __restrict__ idx_s, const int64_t* __restrict__ off_o,
+    int64_t* __restrict__ idx_o, int64_t* __restrict__ keys, int64_t* __restrict__ seg_beg,
+    int64_t* __restrict__ seg_end, unsigned long long* __restrict__ nseg) {
+  __shared__ int32_t stage_s[EXPORT_WARPS][EXPORT_MAX + EXPORT_MAX / 32];
+  const int64_t k = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (k >= n) return;  // warp-uniform
+  int32_t* stage = stage_s[threadIdx.x >> 5];
+  const int64_t e0 = off_s[k];
+  const int64_t len = off_s[k + 1] - e0;
+  const int64_t at = off_o[perm[k]];
+  const int32_t* src = idx_s + e0;
+  int64_t* dst = idx_o + at;
+  if (len <= 128)
+    export_row<4>(src, (int)len, perm, stage, dst, lane);
+  else if (len <= 256)
+    export_row<8>(src, (int)len, perm, stage, dst, lane);
+  else if (len <= 512)
+    export_row<16>(src, (int)len, perm, stage, dst, lane);
+  else if (len <= EXPORT_MAX)
+    export_row<32>(src, (int)len, perm, stage, dst, lane);
+  else {
+    for (int64_t t = lane; t < len; t += 32) keys[at + t] = perm[src[t]];
+    if (lane == 0) {
+      const unsigned long long s = atomicAdd(nseg, 1ull);
+      seg_beg[s] = at;
+      seg_end[s] = at + len;
+    }
+  }
 }
 
 // ---------------------------------------------------------------- host orchestration
@@ -747,6 +853,7 @@ int build_lists(Engine& E, int64_t n, const double* pos, const double* hs, cudaS
   if (n == 0) {
     E.lists.n = 0;
     E.lists.total = 0;
+    E.lists.longest = 0;
     NB_CUDA(cudaMemsetAsync(E.lists.off, 0, sizeof(int64_t), st));
     return 0;
   }
@@ -833,7 +940,7 @@ int build_lists(Engine& E, int64_t n, const double* pos, const double* hs, cudaS
   NB_CUDA(cudaMemcpyAsync(E.h_build, L.off + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   NB_CUDA(cudaMemcpyAsync(E.h_build + 1, E.d_rowmax, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   NB_TRY(pending_check(E, st));
-  const int64_t total = E.h_build[0];
+  const int64_t total = E.h_build[0], longest = E.h_build[1];
   NB_TRY(E.ensure_list_capacity(total));
   // masks -> entries at the rows' offsets
   count_launch(), k_lists_expand<<<grid_for(nleaf * 32, EXPAND_WARPS * 32), EXPAND_WARPS * 32, 0, st>>>(
@@ -841,6 +948,7 @@ int build_lists(Engine& E, int64_t n, const double* pos, const double* hs, cudaS
   E.prof.end(PROF_LISTS, st, (double)n, (double)total);
   L.n = n;
   L.total = total;
+  L.longest = longest;
   return check_device_error(E, st);
 }
 
@@ -862,15 +970,22 @@ int export_lists(Engine& E, int64_t* off_out, int64_t* idx_out, cudaStream_t st)
   Lists& L = E.lists;
   int64_t n = L.n;
   if (n == 0) return 0;
-  size_t tmp = E.cub_bytes;
-  count_launch(), k_export_fill<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, L.off, L.idx, off_out, idx_out);
-  if (L.total > 0) {
+  const bool long_rows = L.longest > EXPORT_MAX;
+  unsigned long long* nseg = E.d_rowmax + 7;
+  int64_t* seg_beg = E.counts;  // scratch of at least n entries each, free between builds
+  int64_t* seg_end = reinterpret_cast<int64_t*>(E.keys_b);
+  if (long_rows) {
     NB_TRY(E.ensure_sort_keys(L.total));
-    NB_CUDA(cudaMemcpyAsync(E.sort_keys, idx_out, sizeof(int64_t) * L.total,
-                            cudaMemcpyDeviceToDevice, st));
-    tmp = E.cub_bytes;
+    NB_CUDA(cudaMemsetAsync(nseg, 0, sizeof(unsigned long long), st));
+  }
+  count_launch(), k_export_rows<<<grid_for(n * 32, EXPORT_WARPS * 32), EXPORT_WARPS * 32, 0, st>>>(
+      n, L.perm, L.off, L.idx, off_out, idx_out, E.sort_keys, seg_beg, seg_end, nseg);
+  if (long_rows) {
+    NB_CUDA(cudaMemcpyAsync(E.h_build, nseg, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    NB_CUDA(host_sync(st));
+    size_t tmp = E.cub_bytes;
     NB_CUDA(cub::DeviceSegmentedSort::SortKeys(E.cub_tmp, tmp, E.sort_keys, idx_out, L.total,
-                                                (int)n, off_out, off_out + 1, st));
+                                                (int)E.h_build[0], seg_beg, seg_end, st));
   }
   return check_device_error(E, st);
 }
