@@ -5,6 +5,8 @@
 
 namespace nbk {
 
+struct Engine;
+
 constexpr int DEP_FIELDS = 6;  // m, m T, m T^4, m vx, m vy, m vz per cell
 
 struct LogGeom {
@@ -17,10 +19,11 @@ void launch_deposit_log(int64_t n, const double* x, const double* h, const doubl
                         const double* t, const double* v, const LogGeom& g, int kid,
                         double* acc, double* outside, unsigned long long* n_tri,
                         cudaStream_t st);
-void launch_deposit_box(int64_t n, const double* x, const double* h, const double* m,
-                        const double* t, const double* v, double x0, double y0, double z0,
-                        double dx, int nb, int kid, double* acc, double* outside,
-                        unsigned long long* n_tri, cudaStream_t st);
+// the box' sums (acc, *outside and *n_tri zeroed by the caller); waits for the stream once
+int deposit_box(Engine& E, int64_t n, const double* x, const double* h, const double* m,
+                const double* t, const double* v, double x0, double y0, double z0, double dx,
+                int nb, int kid, double* acc, double* outside, unsigned long long* n_tri,
+                cudaStream_t st);
 void launch_grid_finish(int64_t ncell, const double* acc, const double* vol, int64_t per,
                         double* mass, float* rho, float* t_mass, float* t_em, float* vel,
                         cudaStream_t st);
@@ -29,9 +32,8 @@ void launch_refine_sums(const double* acc_c, const double* vol_c, int nrc, int n
                         const double* vol_f, int nr, int nth, int nph, int cr, int ct, int cp,
                         double* out, double* sums2, cudaStream_t st);
 
-// spatial order of the particles (grid_kind 0: log grid g, 1: box): keys and identity indices
-void launch_deposit_keys(int64_t n, const double* x, int grid_kind, const LogGeom& g, double x0,
-                         double y0, double z0, double dx, int nb, unsigned long long* keys,
+// spatial order of the particles on the log grid: keys and identity indices
+void launch_deposit_keys(int64_t n, const double* x, const LogGeom& g, unsigned long long* keys,
                          int32_t* idx, cudaStream_t st);
 // out (9 n doubles): x (3n), h, m, t, v (3n) gathered in idx order
 void launch_deposit_gather(int64_t n, const int32_t* idx, const double* x, const double* h,

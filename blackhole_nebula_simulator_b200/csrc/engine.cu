@@ -160,7 +160,7 @@ int Engine::ensure_deposit(int64_t n) {
     NB_CUDA(cudaMalloc((void**)&dep_k1, sizeof(unsigned long long) * c));
     NB_CUDA(cudaMalloc((void**)&dep_i0, sizeof(int32_t) * c));
     NB_CUDA(cudaMalloc((void**)&dep_i1, sizeof(int32_t) * c));
-    NB_CUDA(cudaMalloc((void**)&dep_buf, sizeof(double) * 9 * c));
+    NB_CUDA(cudaMalloc((void**)&dep_buf, sizeof(double) * 12 * c));
     dep_cap = c;
   }
   size_t b = 0;
@@ -168,6 +168,26 @@ int Engine::ensure_deposit(int64_t n) {
                                   (unsigned long long*)nullptr, (int32_t*)nullptr,
                                   (int32_t*)nullptr, (int)dep_cap);
   return ensure_cub(b);
+}
+
+int Engine::ensure_bricks(int64_t nbricks) {
+  Engine& E = *this;
+  if (!dep_count) NB_CUDA(cudaMalloc((void**)&dep_count, 4 * sizeof(int64_t)));
+  if (nbricks <= cap_bricks && brick_off) return 0;
+  int64_t c = 0;
+  NB_TRY(grow(E, brick_count, c, nbricks));
+  c = 0;
+  NB_TRY(grow(E, brick_cursor, c, nbricks));
+  c = 0;
+  NB_TRY(grow(E, brick_off, c, nbricks + 1));
+  cap_bricks = nbricks;
+  return 0;
+}
+
+int Engine::ensure_brick_lists(int64_t pairs, int64_t tasks) {
+  Engine& E = *this;
+  NB_TRY(grow(E, brick_pairs, cap_brick_pairs, pairs));
+  return grow(E, brick_tasks, cap_brick_tasks, tasks);
 }
 
 int Engine::ensure_sort_keys(int64_t m) {
@@ -179,7 +199,8 @@ int Engine::ensure_sort_keys(int64_t m) {
 void Engine::release() {
   void* ps[] = {dep_k0, dep_k1, dep_i0, dep_i1, dep_buf, d_err, bbox, bbox_part, keys_a, keys_b, vals_a, counts, node_lo, node_hi, sub_lo, sub_hi,
                 cub_tmp, sort_keys, red, lists.perm, lists.inv_perm, lists.spos, lists.off,
-                lists.idx, d_rowmax, tidx, leaf_cbase, leaf_bbase, leaf_ncand, cands, masks};
+                lists.idx, d_rowmax, tidx, leaf_cbase, leaf_bbase, leaf_ncand, cands, masks,
+                dep_count, brick_count, brick_cursor, brick_off, brick_pairs, brick_tasks};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (h_err) cudaFreeHost(h_err);

@@ -171,12 +171,24 @@ struct Engine {
   size_t cub_bytes = 0;
   int64_t* sort_keys = nullptr;
   // particle -> grid deposition: spatial sort keys / indices (double buffers) and the gathered
-  // particle data (9 doubles per particle)
+  // particle data (9 doubles per particle) of the log grid; the box' work list (in dep_i0) and
+  // records (12 doubles per particle, in dep_buf)
   unsigned long long *dep_k0 = nullptr, *dep_k1 = nullptr;
   int32_t *dep_i0 = nullptr, *dep_i1 = nullptr;
   double* dep_buf = nullptr;
   int64_t dep_cap = 0;
   int ensure_deposit(int64_t n);
+  // the box' bricks of cells: counters, particles per brick, lists, tasks
+  int64_t* dep_count = nullptr;
+  unsigned long long* brick_count = nullptr;
+  unsigned* brick_cursor = nullptr;
+  int64_t* brick_off = nullptr;
+  int64_t cap_bricks = 0;
+  int32_t* brick_pairs = nullptr;
+  int2* brick_tasks = nullptr;
+  int64_t cap_brick_pairs = 0, cap_brick_tasks = 0;
+  int ensure_bricks(int64_t nbricks);
+  int ensure_brick_lists(int64_t pairs, int64_t tasks);
   int64_t list_slots = 0, cand_slots = 0;  // resident warps of the persistent list passes
   int32_t* tidx = nullptr;  // interacting entries of the active rows, in the lists' layout
   int64_t cap_tidx = 0;
