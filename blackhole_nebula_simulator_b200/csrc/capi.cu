@@ -218,7 +218,7 @@ int nb_density(nb_ctx* ctx, int64_t n, const double* pos, const double* mass,
   Engine& E = ctx->E;
   if (kernel_id != 0 && kernel_id != 1) return nbk::set_host_error(E, "bad kernel_id"), NB_ERR_INPUT;
   NB_TRY(E.ws.ensure(E, n));
-  nbk::pack_pos(n, pos, nullptr, E.ws.pk0, S(stream));
+  nbk::pack_pos(n, pos, mass, E.ws.pk0, S(stream));
   nbk::DensityParams dp{kernel_id, cnorm_of(kernel_id), eta, tol, h_max};
   nbk::launch_density64<int64_t>(rows ? nrows : n, rows, E.ws.pk0, mass, h_start, h_search,
                                  offset, index, dp, nullptr, h_out, rho, omega, iters, flags,

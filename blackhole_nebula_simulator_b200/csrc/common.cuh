@@ -73,6 +73,21 @@ __device__ __forceinline__ I ld_stream(const I* p) {
     return (I)__ldcs(reinterpret_cast<const long long*>(p));
 }
 
+// One 32-byte record in one load (the packed per-particle records lie on 32-byte boundaries and
+// are read-only in the pass that gathers them).
+__device__ __forceinline__ double4 ld_rec(const double4* p) {
+  double4 v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+      : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void ld_rec(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
 // Kahan-compensated accumulator for the FP32 pair sums.
 struct Kahan {
   float s, c;

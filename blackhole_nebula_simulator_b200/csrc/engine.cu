@@ -417,20 +417,17 @@ __global__ void k_pack_sorted(int64_t n, const int32_t* __restrict__ perm,
   out[k] = make_double4(x[3 * i], x[3 * i + 1], x[3 * i + 2], w ? w[i] : 0.0);
 }
 
-// the density pass's per-particle inputs in sorted order (masses also as floats when asked)
+// the density pass's per-particle inputs in sorted order
 __global__ void k_gather_density(int64_t n, const int32_t* __restrict__ perm,
                                  const double* __restrict__ mass, const double* __restrict__ h0,
                                  const double* __restrict__ hs, double* __restrict__ mass_s,
-                                 double* __restrict__ h0_s, double* __restrict__ hs_s,
-                                 float* __restrict__ massf_s) {
+                                 double* __restrict__ h0_s, double* __restrict__ hs_s) {
   int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int32_t i = perm[k];
-  const double m = mass[i];
-  mass_s[k] = m;
+  mass_s[k] = mass[i];
   h0_s[k] = h0[i];
   hs_s[k] = hs[i];
-  if (massf_s) massf_s[k] = (float)m;
 }
 
 __global__ void k_to_float(int64_t n, const double* __restrict__ a, float* __restrict__ out) {
@@ -702,7 +699,6 @@ int Workspace::ensure(Engine& E, int64_t n) {
   double4** d4[] = {&pk0, &pk1, &pk2, &pk3};
   for (double4** p : d4) NB_CUDA(cudaMalloc((void**)p, sizeof(double4) * c));
   NB_CUDA(cudaMalloc((void**)&pk32, sizeof(float4) * 2 * c));
-  NB_CUDA(cudaMalloc((void**)&f_mass, sizeof(float) * c));
   float4** f4s[] = {&pf1, &pf2, &pf3};
   for (float4** p : f4s) NB_CUDA(cudaMalloc((void**)p, sizeof(float4) * c));
   int64_t** i8[] = {&rows, &rows_s, &rows2, &iters, &flags, &need, &i_tmp, &pairs, &i_lvl, &i_tmp2};
@@ -765,7 +761,7 @@ int Workspace::ensure_grad(Engine& E, int64_t n) {
 void Workspace::release() {
   void* ps[] = {pk4, gvel, gvel32, d_a, d_b, d_c, d_hg, d_hs, d_heff, d_hlim, d_disp, d_P, d_cs, d_vsig, d_ddudt,
                 d_dm, d_tmp, d_uh, v_flow, v_pred, v_eval, v_dacc, v_tmp, pk0, pk1, pk2, pk3, pk32,
-                pf1, pf2, pf3, m_x, m_sorted, m_smark, f_mass,
+                pf1, pf2, pf3, m_x, m_sorted, m_smark,
                 rows, rows_s, rows2, iters, flags, need, i_tmp, pairs, i_lvl, i_tmp2, m_rows, m_done, m_need,
                 m_tmp, i32a, i32b, dk_b, d_int, d_i64, tk_key0, tk_key1, tk_idx0, tk_idx1, d_scal_i};
   for (void* p : ps)
@@ -921,8 +917,8 @@ static int density_on_lists(Engine& E, int64_t n, const double* x, const double*
                               E.prof.on ? W.pairs : nullptr, st);
   } else {
     count_launch(), k_gather_density<<<grid_for(n), NB_THREADS, 0, st>>>(
-        n, L.perm, mass, h_start, h_search, W.d_a, W.d_b, W.d_c, nullptr);
-    count_launch(), k_pack_sorted<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, x, nullptr, W.pk0);
+        n, L.perm, mass, h_start, h_search, W.d_a, W.d_b, W.d_c);
+    count_launch(), k_pack_sorted<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, x, mass, W.pk0);
     E.prof.begin(st);
     launch_density64<int32_t>(nrows, W.rows_s, W.pk0, W.d_a, W.d_b, W.d_c, L.off, L.idx, dp,
                               L.perm, h_out, rho, omega, W.iters, W.flags,

@@ -3,7 +3,7 @@
 // pre-planned run that must not allocate once set up.  It needs no context (nb_create allocates)
 // and calls no cudaMalloc, cudaFree or allocating library routine.
 //
-// Its only scratch, the packed (x, y, z) positions the density kernel reads, lives in the
+// Its only scratch, the packed (x, y, z, mass) records the density kernel reads, lives in the
 // file-scope array below, of a fixed maximum of NB_NOALLOC_MAX_N particles (8 MiB).  Every GPU
 // that loads the library holds that array until the process exits.  All calls share it and it
 // keeps the last call's contents; each call overwrites the first n entries before reading them,
@@ -85,7 +85,7 @@ int nb_density_noalloc(int64_t n, const double* pos, const double* mass, const d
   int r = scratch_for_current_device(&scratch, g_msg, sizeof(g_msg));
   if (r != 0) return r;
   cudaStream_t st = (cudaStream_t)stream;
-  nbk::pack_pos(n, pos, nullptr, scratch, st);
+  nbk::pack_pos(n, pos, mass, scratch, st);
   double cn = kernel_id == 0 ? 1.0 / M_PI : 495.0 / (256.0 * M_PI);
   nbk::DensityParams dp{kernel_id, cn, eta, tol, h_max};
   nbk::launch_density64<int64_t>(rows ? nrows : n, rows, scratch, mass, h_start, h_search, offset,

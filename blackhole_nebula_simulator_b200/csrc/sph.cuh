@@ -8,7 +8,6 @@ namespace nbk {
 struct DensityParams {
   int kid;
   double cnorm, eta, tol, h_max;
-  const float* massf = nullptr;  // FP32 form: neighbour masses as floats (sorted order), or null
 };
 
 struct ForceParams {
@@ -72,6 +71,7 @@ struct ForceOut {
   int64_t* pairs = nullptr; // interacting pairs per row
 };
 
+// pos: (x, y, z, mass) records, 32-byte aligned
 template <typename I>
 void launch_density64(int64_t nrows, const int64_t* rows, const double4* pos, const double* mass,
                       const double* h_start, const double* h_search, const int64_t* off,

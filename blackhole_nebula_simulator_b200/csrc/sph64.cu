@@ -1,5 +1,7 @@
 // FP64 instantiations of the pair passes (compiled without fused multiply-add: the FP64 path
 // rounds like the reference).
+#include <type_traits>
+
 #include "sph_impl.cuh"
 
 namespace nbk {
@@ -12,9 +14,24 @@ void launch_density64(int64_t nrows, const int64_t* rows, const double4* pos, co
                       cudaStream_t st) {
   if (nrows <= 0) return;
   Pos64 geo{pos};
-  count_launch(), k_density_thread<double, Pos64, I><<<grid_for(nrows), NB_THREADS, 0, st>>>(
-      nrows, rows, geo, mass, h_start, h_search, off, idx, prm, out_map, h_out, rho, omega, iters,
-      flags, work);
+  auto run = [&](auto kid, auto lanes) {
+    constexpr int KID = decltype(kid)::value, L = decltype(lanes)::value;
+    count_launch(), k_density64<KID, L, I><<<grid_for(nrows * L, DENSITY_THREADS), DENSITY_THREADS, 0, st>>>(
+        nrows, rows, geo, mass, h_start, h_search, off, idx, prm, out_map, h_out, rho, omega,
+        iters, flags, work);
+  };
+  using std::integral_constant;
+  // Cubic: 8 lanes per row once the rows fill the GPU (262,144 cloud rows 447 us against 646 with
+  // 32 lanes; 300,000 torus rows 607 against 721), 32 for fewer (30,000 rows 150 us against 186,
+  // 3,000 rows 84 against 113).  Wendland C4: 32 lanes at any size, whose block keeps 4 rows'
+  // caches (11 KB) instead of 16 rows' (43 KB) out of L1 (200,001 torus rows 0.98 ms against
+  // 1.24 with 16 lanes and 1.94 with 8).
+  if (prm.kid != 0)
+    run(integral_constant<int, 1>{}, integral_constant<int, 32>{});
+  else if (nrows >= 65536)
+    run(integral_constant<int, 0>{}, integral_constant<int, 8>{});
+  else
+    run(integral_constant<int, 0>{}, integral_constant<int, 32>{});
 }
 
 template <typename I>

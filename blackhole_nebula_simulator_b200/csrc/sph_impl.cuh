@@ -1,8 +1,8 @@
 // SPH pair passes on neighbour lists (implementation, included by sph64.cu and sph32.cu): the h-rho Newton solve and the fused pressure + artificial
 // viscosity (+ conductivity, + disc viscosity) force and du/dt pass.
 //
-// The density solve runs eight lanes per row with a shared-memory cache of the in-range entries
-// (FP32) or one thread per row (FP64); the force pass eight lanes per row.  Both walk CSR lists.  They are templated on the list index type so the
+// The density solve runs 8 (FP32) or 16 (FP64) lanes per row with a shared-memory cache of the
+// inner entries; the force pass eight lanes per row.  Both walk CSR lists.  They are templated on the list index type so the
 // same code serves the caller-order int64 lists of the operator API and the engine's sorted int32
 // lists, and on the arithmetic: FP64 (every pair term in double) or FP32 (positions as float
 // offsets from cell centres, float pair terms, Kahan-compensated sums, the Newton update and all
@@ -18,7 +18,6 @@ namespace nbk {
 // FP64: packed (x, y, z, w) doubles.  dx = x_j - x_i as the reference forms it.
 struct Pos64 {
   const double4* p;
-  static constexpr bool has_mass = false;
   struct Own {
     double4 a;
   };
@@ -34,6 +33,15 @@ struct Pos64 {
   __device__ __forceinline__ void diff(int64_t i, int64_t j, double& dx, double& dy,
                                        double& dz) const {
     diff(own(i), j, dx, dy, dz);
+  }
+  // the difference and particle j's mass (the record's w, where the pass packs it there)
+  __device__ __forceinline__ void diff_m(const Own& o, int64_t j, double& dx, double& dy,
+                                         double& dz, double& m) const {
+    const double4 b = ld_rec(p + j);
+    dx = b.x - o.a.x;
+    dy = b.y - o.a.y;
+    dz = b.z - o.a.z;
+    m = b.w;
   }
   // the difference and particle j's smoothing length (from the hydro record)
   template <typename V4>
@@ -58,7 +66,6 @@ struct Pos32 {
   const float4* p;
   float cell;
   const double* box6 = nullptr;  // grid corner and far corner; the edge is derived on the device
-  static constexpr bool has_mass = true;
   struct Own {
     float4 a, c;
   };
@@ -123,173 +130,24 @@ struct Acc<float> {
 // Reference sim/sph.py:215-297 (_sums, _distances, _density_kernel): Newton-Raphson on
 // f(h) = sum_j m_j W(r_ij, h) - m_i (eta/h)^3 inside a bisection bracket, tol * h0, at most 50
 // iterations; the cap test near the search limit; Omega = 1 + h/(3 rho) sum m dW/dh (1 at h_max).
-template <typename R, typename PosT, typename I>
-__device__ void density_sums(const PosT& geo, int64_t i, const int64_t* off, const I* idx,
-                             const double* mass, R r2max, R h, int kid, R cnorm, double& rs_out,
-                             double& dws_out, int64_t& work) {
-  Acc<R> rs, dws;
-  R inv_h = R(1) / h;
-  R ih2 = inv_h * inv_h;
-  R ih3 = ih2 * inv_h;
-  R ih4 = ih2 * ih2;
-  for (int64_t e = off[i]; e < off[i + 1]; ++e) {
-    int64_t j = (int64_t)idx[e];
-    R dx, dy, dz;
-    geo.diff(i, j, dx, dy, dz);
-    R d2 = sqdist(dx, dy, dz);
-    if (!(d2 < r2max)) continue;
-    R q = sqrt(d2) * inv_h;
-    if (q < R(2)) {
-      work += 1;
-      R fq = kernel_f<R>(q, kid);
-      R m = (R)mass[j];
-      rs.add(m * cnorm * ih3 * fq);
-      dws.add(m * (-cnorm * ih4 * (R(3) * fq + q * kernel_df<R>(q, kid))));
-    }
-  }
-  rs_out = rs.get();
-  dws_out = dws.get();
-}
 
-// Sums over the cached in-range entries (r, m) of one row.
-template <typename R>
-__device__ __forceinline__ void cached_sums(const R* rr, const R* mm, int cnt, R h, int kid,
-                                            R cnorm, double& rs_out, double& dws_out,
-                                            int64_t& work) {
-  Acc<R> rs, dws;
-  R inv_h = R(1) / h;
-  R ih2 = inv_h * inv_h;
-  R ih3 = ih2 * inv_h;
-  R ih4 = ih2 * ih2;
-  for (int k = 0; k < cnt; ++k) {
-    R q = rr[k] * inv_h;
-    if (q < R(2)) {
-      work += 1;
-      R fq = kernel_f<R>(q, kid);
-      R m = mm[k];
-      rs.add(m * cnorm * ih3 * fq);
-      dws.add(m * (-cnorm * ih4 * (R(3) * fq + q * kernel_df<R>(q, kid))));
-    }
-  }
-  rs_out = rs.get();
-  dws_out = dws.get();
-}
-
-// In-range entries a row may cache in its thread's local array (0: every sum walks the list; a
-// per-thread cache in local memory measured slower than re-walking the curve-local list).
-constexpr int DENSITY_CACHE = 0;
-
-// One thread per row (the FP64 form: its shared-memory cache of (r, m) in double would hold
-// occupancy too low for the row-group kernel below to pay off).
-
-template <typename R, typename PosT, typename I>
-__global__ void __launch_bounds__(NB_THREADS)
-    k_density_thread(int64_t nrows, const int64_t* __restrict__ rows, PosT geo_in,
-              const double* __restrict__ mass, const double* __restrict__ h_start,
-              const double* __restrict__ h_search, const int64_t* __restrict__ off,
-              const I* __restrict__ idx, DensityParams prm, const int32_t* __restrict__ out_map,
-              double* __restrict__ h_out, double* __restrict__ rho, double* __restrict__ omega,
-              int64_t* __restrict__ iters, int64_t* __restrict__ flags, int64_t* __restrict__ work) {
-  PosT geo = geo_in;
-  geo.ready();
-  int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (q >= nrows) return;
-  int64_t i = rows ? rows[q] : q;
-  int64_t o = out_map ? (int64_t)out_map[i] : q;
-  double m_i = mass[i];
-  double hs = fmin(h_search[i], prm.h_max);
-  double r_max = 2.0 * hs;
-  R r2max = (R)(r_max * r_max);
-  const int kid = prm.kid;
-  const R cn = (R)prm.cnorm;
-  int64_t evals = 0;
-  // distances and masses of the entries inside r_max (sim/sph.py:231-248): cached when
-  // DENSITY_CACHE > 0, else recomputed from the list by every sum
-  constexpr int CAP = DENSITY_CACHE > 0 ? DENSITY_CACHE : 1;
-  R rr[CAP], mm[CAP];
-  int cnt = 0;
-  bool cached = DENSITY_CACHE > 0;
-  if (DENSITY_CACHE > 0) {
-    for (int64_t e = off[i]; e < off[i + 1]; ++e) {
-      int64_t j = (int64_t)idx[e];
-      R dx, dy, dz;
-      geo.diff(i, j, dx, dy, dz);
-      R d2 = sqdist(dx, dy, dz);
-      if (!(d2 < r2max)) continue;
-      if (cnt < DENSITY_CACHE) {
-        rr[cnt] = sqrt(d2);
-        mm[cnt] = (R)mass[j];
-      } else {
-        cached = false;
-      }
-      cnt += 1;
-    }
-  }
-  auto sums = [&](R h, double& rs, double& dws) {
-    if (cached)
-      cached_sums<R>(rr, mm, cnt, h, kid, cn, rs, dws, evals);
-    else
-      density_sums<R>(geo, i, off, idx, mass, r2max, h, kid, cn, rs, dws, evals);
-  };
-  double lo = 0.0, hi = hs;
-  double h = fmin(h_start[i], hi);
-  double h0 = h;
-  int flag = 3, it = 0;
-  const double eta = prm.eta, e3 = eta * eta * eta;
-  while (it < 50) {
-    it += 1;
-    double rs, dws;
-    sums((R)h, rs, dws);
-    double t = eta / h;
-    double f = rs - m_i * (t * t * t);
-    double h2 = h * h;
-    double df = dws + 3.0 * m_i * e3 / (h2 * h2);
-    if (f > 0)
-      hi = h;
-    else
-      lo = h;
-    double h_new = df > 0 ? h - f / df : 0.5 * (lo + hi);
-    if (!(lo <= h_new && h_new <= hi)) h_new = 0.5 * (lo + hi);
-    if (fabs(h_new - h) < prm.tol * h0) {
-      h = h_new;
-      flag = 0;
-      break;
-    }
-    h = h_new;
-  }
-  if (h >= hs * (1 - 1e-3)) {
-    double rs_lim, dummy;
-    sums((R)hs, rs_lim, dummy);
-    double t = eta / hs;
-    if (rs_lim - m_i * (t * t * t) < 0) {
-      h = hs;
-      flag = hs >= prm.h_max ? 1 : 2;
-    }
-  }
-  double rs, dws;
-  sums((R)h, rs, dws);
-  h_out[o] = h;
-  rho[o] = rs;
-  omega[o] = flag == 1 ? 1.0 : 1.0 + h / (3.0 * rs) * dws;
-  if (iters) iters[o] = it;
-  if (flags) flags[o] = flag;
-  if (work) work[o] = evals;
-}
-
-// Sums over the 8 lanes of a row group (lanes 8g .. 8g+7 of a warp).  Every lane of the group ends
-// with the same value (each butterfly step adds the same two operands on both lanes).  FP64: plain
-// sums.  FP32: each lane's Kahan partial (s, -c) is combined pairwise with an exact two-sum, the
-// rounding errors and the lanes' compensations carried in a second float.
+// Sums over the L lanes of a row group (lanes L g .. L g + L - 1 of a warp).  Every lane of the
+// group ends with the same value (each butterfly step adds the same two operands on both lanes).
+// FP64: plain sums.  FP32: each lane's Kahan partial (s, -c) is combined pairwise with an exact
+// two-sum, the rounding errors and the lanes' compensations carried in a second float.
+template <int L = 8>
 __device__ __forceinline__ double group_total(double v) {
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ __forceinline__ double group_total(const Acc<double>& a) { return group_total(a.s); }
+template <int L = 8>
+__device__ __forceinline__ double group_total(const Acc<double>& a) { return group_total<L>(a.s); }
+template <int L = 8>
 __device__ __forceinline__ double group_total(const Acc<float>& a) {
   float s = a.k.s, k = -a.k.c;
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) {
+  for (int o = L / 2; o > 0; o >>= 1) {
     float s2 = __shfl_xor_sync(0xffffffffu, s, o);
     float k2 = __shfl_xor_sync(0xffffffffu, k, o);
     float t = __fadd_rn(s, s2);
@@ -313,12 +171,6 @@ struct DensityEntry<float> {
   // 8 resident blocks (the register limit) leave most of the SM's L1 to the gathered records
   static constexpr int CAP = DENSITY_CAP;
   static constexpr int BLOCKS = 8;
-};
-template <>
-struct DensityEntry<double> {
-  using T = double2;
-  static constexpr int CAP = 192;
-  static constexpr int BLOCKS = 4;
 };
 constexpr int DENSITY_THREADS = 128;  // 16 rows per block
 // rounds of 8 entries the list walk loads at once: 4 measured 3.55 ms per density launch on the
@@ -364,12 +216,7 @@ __global__ void __launch_bounds__(DENSITY_THREADS, DensityEntry<R>::BLOCKS)
     e1 = off[i + 1];
   }
   const typename PosT::Own me_rec = geo.own(i);  // the row's own record, loaded once
-  auto mass_of = [&](int64_t j) -> R {
-    if constexpr (PosT::has_mass)
-      return (R)geo.mass(j);
-    else
-      return prm.massf ? (R)prm.massf[j] : (R)mass[j];
-  };
+  auto mass_of = [&](int64_t j) -> R { return (R)geo.mass(j); };
   const double r_max = 2.0 * hs;
   const R r2max = (R)(r_max * r_max);
   const int kid = prm.kid;
@@ -522,6 +369,240 @@ __global__ void __launch_bounds__(DENSITY_THREADS, DensityEntry<R>::BLOCKS)
   sums((R)h, live, rs, dws);
 #pragma unroll
   for (int of = 4; of > 0; of >>= 1) evals += __shfl_xor_sync(FULL, evals, of);
+  if (live && gl == 0) {
+    h_out[o] = h;
+    rho[o] = rs;
+    omega[o] = flag == 1 ? 1.0 : 1.0 + h / (3.0 * rs) * dws;
+    if (iters) iters[o] = it;
+    if (flags) flags[o] = flag;
+    if (work) work[o] = evals;
+  }
+}
+
+// Terms of one entry (r, m) at 1/h, FP64: m f and m (3 f + q f') with the powers of 1/h factored
+// out of the sums.
+template <int KID>
+struct DensityTerm {
+  double inv_h, cn;
+  __device__ __forceinline__ DensityTerm(double h, double cn_) : inv_h(1.0 / h), cn(cn_) {}
+  __device__ __forceinline__ int add(double r, double m, double& rs, double& dws) const {
+    const double q = r * inv_h;
+    if (!(q < 2.0)) return 0;
+    double f, g;  // f(q) and 3 f + q f'
+    if (KID == 0) {
+      if (q < 1.0) {
+        const double q2 = q * q;
+        f = fma(q2, fma(0.75, q, -1.5), 1.0);
+        g = fma(q2, fma(4.5, q, -7.5), 3.0);
+      } else {
+        const double t = 2.0 - q, t2 = t * t;
+        f = 0.25 * t2 * t;
+        g = 1.5 * t2 * (1.0 - q);
+      }
+    } else {
+      const double x = fma(-0.5, q, 1.0), x2 = x * x, x5 = x2 * x2 * x;
+      f = x5 * x * fma(fma(35.0 / 12.0, q, 3.0), q, 1.0);
+      g = fma(3.0, f, (-7.0 / 3.0) * (q * q) * x5 * fma(5.0, q, 2.0));
+    }
+    rs = fma(m, f, rs);
+    dws = fma(m, g, dws);
+    return 1;
+  }
+  __device__ __forceinline__ double rho(double s) const { return cn * (inv_h * inv_h * inv_h) * s; }
+  __device__ __forceinline__ double drho(double s) const {
+    const double i2 = inv_h * inv_h;
+    return -cn * (i2 * i2) * s;
+  }
+};
+
+// FP64 form.  L lanes per row.  The lanes of a row split its list (entry e to lane e mod L,
+// coalesced index loads) and keep the squared distance and the index of every entry inside r_in =
+// 2.1 h in shared memory, in list order; the Newton sums run over that cache and reduce across
+// the lanes, so the lanes of a row take the same Newton steps.  The first sum over a filled cache
+// turns the squares into distances (two thirds of the entries are not worth a square root); a
+// cached entry's mass is the row's own where all of them are equal, else gathered again.  The
+// iterates stay near the start h where it is the last step's; where h leaves the cached range
+// (2 h > r_in), or has shrunk enough that the entries of a row too long for the cache may fit, the
+// cache is filled again at the present h.  A row with more entries inside 2.1 h than the cache
+// holds walks its list in every sum.
+// Bound by issue and by the gathers' latency (54 % issue active, L1 54 %, FP64 pipe 35 % at 16
+// lanes; a row needs about 800 warp instructions with 8 lanes).  With one thread per row, the list
+// read uncoalesced and walked again in every sum, 262,144 cloud particles took 1.69 ms per call;
+// 0.45 ms now.
+// Entries kept: about 67 lie inside 2.1 h with the cubic kernel, 159 with Wendland C4.
+template <int KID>
+constexpr int D64_CAP = KID == 0 ? 128 : 224;
+// 8 lanes share the Newton arithmetic among four rows of a warp, 32 give a row all the loads in
+// flight at once: see launch_density64 for where each is the faster.
+constexpr int D64_UNROLL = 3;  // rounds loaded at once (2, 4, 5 measured up to 10 % slower)
+
+template <int KID, int L, typename I>
+__global__ void __launch_bounds__(DENSITY_THREADS, 6)
+    k_density64(int64_t nrows, const int64_t* __restrict__ rows, Pos64 geo,
+              const double* __restrict__ mass, const double* __restrict__ h_start,
+              const double* __restrict__ h_search, const int64_t* __restrict__ off,
+              const I* __restrict__ idx, DensityParams prm,
+              const int32_t* __restrict__ out_map, double* __restrict__ h_out,
+              double* __restrict__ rho, double* __restrict__ omega, int64_t* __restrict__ iters,
+              int64_t* __restrict__ flags, int64_t* __restrict__ work) {
+  constexpr int CAP = D64_CAP<KID>;
+  __shared__ double cache_r[DENSITY_THREADS / L][CAP];
+  __shared__ int32_t cache_j[DENSITY_THREADS / L][CAP];
+  const unsigned FULL = 0xffffffffu;
+  const unsigned GROUP = (unsigned)((1ull << L) - 1ull);
+  const int lane = threadIdx.x & 31, gl = lane & (L - 1), g = lane / L;
+  const int64_t q = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * (32 / L) + g;
+  const bool live = q < nrows;
+  if (!__any_sync(FULL, live)) return;  // warp-uniform
+  double* cr = cache_r[threadIdx.x / L];
+  int32_t* cj = cache_j[threadIdx.x / L];
+  int64_t i = 0, o = 0, e0 = 0;
+  unsigned len = 0;
+  double m_i = 1.0, hs = 1.0;
+  if (live) {
+    i = rows ? rows[q] : q;
+    o = out_map ? (int64_t)out_map[i] : q;
+    m_i = mass[i];
+    hs = fmin(h_search[i], prm.h_max);
+    e0 = off[i];
+    len = (unsigned)(off[i + 1] - e0);
+  }
+  const I* list = idx + e0;
+  const Pos64::Own me_rec = geo.own(i);  // the row's own record, loaded once
+  const double r_max = 2.0 * hs;
+  const double r2max = r_max * r_max;
+  double r_in = 0.0;  // radius of the cached entries
+  int cnt = 0;
+  bool cached = false, squared = false, uniform = false;
+  int evals = 0;
+  // The entries inside rin of the rows whose `need` is set, appended in list order.  D64_UNROLL
+  // rounds of L entries per pass: their index and record loads are issued together (the walk is
+  // bound by the latency of those dependent gathers), then the rounds are appended one after the
+  // other.
+  constexpr int U = D64_UNROLL;
+  auto fill = [&](bool need, double rin) {
+    const unsigned mylen = need ? len : 0u;
+    const unsigned maxlen = __reduce_max_sync(FULL, mylen);
+    const double r2in = fmin(rin * rin, r2max);
+    int c = 0;
+    bool same = true;
+    __syncwarp();
+    for (unsigned b = 0; b < maxlen; b += L * U) {
+      int jj[U];
+      double d2[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned e = b + L * u + gl;
+        jj[u] = e < mylen ? (int)ld_stream(list + e) : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        d2[u] = INFINITY;
+        if (jj[u] >= 0) {
+          double dx, dy, dz, m;
+          geo.diff_m(me_rec, jj[u], dx, dy, dz, m);
+          d2[u] = sqdist(dx, dy, dz);
+          if (d2[u] < r2in && m != m_i) same = false;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool inner = d2[u] < r2in;
+        const unsigned seg = (__ballot_sync(FULL, inner) >> (L * g)) & GROUP;
+        const int pos = c + __popc(seg & ((1u << gl) - 1u));
+        if (inner && pos < CAP) {  // overflow: the walk in `sums` instead
+          cr[pos] = d2[u];
+          cj[pos] = jj[u];
+        }
+        c += __popc(seg);
+      }
+    }
+    const unsigned differ = (__ballot_sync(FULL, !same) >> (L * g)) & GROUP;
+    __syncwarp();
+    if (need) {
+      r_in = rin;
+      cnt = c;
+      cached = c <= CAP;
+      squared = true;
+      uniform = differ == 0;
+    }
+  };
+  // kernel sums at h of the rows whose `active` is set; every lane takes part in the reductions
+  auto sums = [&](double h, bool active, double& rs_out, double& dws_out) {
+    const DensityTerm<KID> term(h, prm.cnorm);
+    const bool outgrown = !(r_in * term.inv_h >= 2.0);
+    const bool need = active && (cached ? outgrown : r_in == 0.0 || 2.1 * h < 0.85 * r_in);
+    if (__any_sync(FULL, need)) fill(need, 2.1 * h);
+    double rs = 0.0, dws = 0.0;
+    if (active) {
+      if (cached) {
+        for (int t = gl; t < cnt; t += L) {
+          double r = cr[t];
+          if (squared) {
+            r = sqrt(r);
+            cr[t] = r;  // only this lane reads it
+          }
+          evals += term.add(r, uniform ? m_i : geo.p[cj[t]].w, rs, dws);
+        }
+        squared = false;
+      } else {
+        for (unsigned e = gl; e < len; e += L) {
+          double dx, dy, dz, m;
+          geo.diff_m(me_rec, (int)list[e], dx, dy, dz, m);
+          const double d2 = sqdist(dx, dy, dz);
+          if (d2 < r2max) evals += term.add(sqrt(d2), m, rs, dws);
+        }
+      }
+    }
+    rs_out = term.rho(group_total<L>(rs));
+    dws_out = term.drho(group_total<L>(dws));
+  };
+  double lo = 0.0, hi = hs;
+  double h = live ? fmin(h_start[i], hi) : 1.0;
+  double h0 = h;
+  int flag = 3, it = 0;
+  bool done = !live;
+  const double eta = prm.eta, e3 = eta * eta * eta;
+  while (__any_sync(FULL, !done)) {
+    double rs, dws;
+    sums(h, !done, rs, dws);
+    if (!done) {
+      it += 1;
+      double t = eta / h;
+      double f = rs - m_i * (t * t * t);
+      double h2 = h * h;
+      double df = dws + 3.0 * m_i * e3 / (h2 * h2);
+      if (f > 0)
+        hi = h;
+      else
+        lo = h;
+      double h_new = df > 0 ? h - f / df : 0.5 * (lo + hi);
+      if (!(lo <= h_new && h_new <= hi)) h_new = 0.5 * (lo + hi);
+      if (fabs(h_new - h) < prm.tol * h0) {
+        flag = 0;
+        done = true;
+      } else if (it >= 50) {
+        done = true;
+      }
+      h = h_new;
+    }
+  }
+  const bool cap_test = live && h >= hs * (1 - 1e-3);
+  if (__any_sync(FULL, cap_test)) {
+    double rs_lim, dummy;
+    sums(cap_test ? hs : h, cap_test, rs_lim, dummy);
+    double t = eta / hs;
+    if (cap_test && rs_lim - m_i * (t * t * t) < 0) {
+      h = hs;
+      flag = hs >= prm.h_max ? 1 : 2;
+    }
+  }
+  double rs, dws;
+  sums(h, live, rs, dws);
+  if (work) {
+#pragma unroll
+    for (int of = L / 2; of > 0; of >>= 1) evals += __shfl_xor_sync(FULL, evals, of);
+  }
   if (live && gl == 0) {
     h_out[o] = h;
     rho[o] = rs;
