@@ -276,10 +276,8 @@ static int forces_impl(nb_ctx* ctx, int64_t n, const double* pos, const double* 
   NB_TRY(E.ws.ensure(E, n));
   nbk::Workspace& W = E.ws;
   cudaStream_t st = S(stream);
-  nbk::pack_pos(n, pos, nullptr, W.pk0, st);
-  nbk::pack_vm(n, vel, mass, W.pk1, st);
-  nbk::pack4(n, h, rho, omega, pressure, W.pk2, st);
-  nbk::pack4(n, u, c_s, alpha, nullptr, W.pk3, st);
+  nbk::pack_forces64(n, pos, vel, mass, h, rho, omega, pressure, u, c_s, alpha, W.pk0, W.pk1,
+                     W.pk2, W.pk3, st);
   nbk::ForceParams fp{};
   fp.kid = kernel_id;
   fp.cnorm = cnorm_of(kernel_id);
@@ -298,7 +296,9 @@ static int forces_impl(nb_ctx* ctx, int64_t n, const double* pos, const double* 
     fp.eta_crit = eta_crit;
     fp.eta_fold = eta_fold;
     fp.gate = gate;
-    fp.gv64 = grad_v;
+    NB_TRY(W.ensure_grad(E, n));
+    nbk::pack_sym(n, grad_v, reinterpret_cast<double4*>(W.gvel), st);
+    fp.gs64 = reinterpret_cast<const double4*>(W.gvel);
   }
   nbk::ForceOut fo;
   fo.acc = acc;
@@ -352,17 +352,15 @@ int nb_gradients(nb_ctx* ctx, int64_t n, const double* pos, const double* vel,
   NB_TRY(E.ws.ensure(E, std::max<int64_t>(n, 1)));
   nbk::Workspace& W = E.ws;
   cudaStream_t st = S(stream);
-  nbk::pack_pos(n, pos, nullptr, W.pk0, st);
+  nbk::pack_pos(n, pos, h, W.pk0, st);
   nbk::pack_vm(n, vel, mass, W.pk1, st);
-  nbk::pack4(n, h, nullptr, nullptr, nullptr, W.pk2, st);
   nbk::pack_pos(n, acc, nullptr, W.pk3, st);
-  nbk::GradParams gp{kernel_id, cnorm_of(kernel_id), 0};
   nbk::GradOut go;
   go.div = div_v;
   go.curl = curl_v;
   go.ddiv = ddivv_dt;
-  nbk::launch_gradients<int64_t>(rows ? nrows : n, rows, W.pk0, W.pk1, W.pk2, W.pk3, offset,
-                                 index, gp, nullptr, go, st);
+  nbk::launch_gradients(rows ? nrows : n, rows, W.pk0, W.pk1, W.pk3, offset, index, kernel_id,
+                        cnorm_of(kernel_id), go, st);
   NB_CUDA(cudaGetLastError());
   return nbk::check_device_error(E, st);
 }
@@ -377,14 +375,12 @@ int nb_velocity_gradients(nb_ctx* ctx, int64_t n, const double* pos, const doubl
   NB_TRY(E.ws.ensure(E, std::max<int64_t>(n, 1)));
   nbk::Workspace& W = E.ws;
   cudaStream_t st = S(stream);
-  nbk::pack_pos(n, pos, nullptr, W.pk0, st);
+  nbk::pack_pos(n, pos, h, W.pk0, st);
   nbk::pack_vm(n, vel, mass, W.pk1, st);
-  nbk::pack4(n, h, nullptr, nullptr, nullptr, W.pk2, st);
-  nbk::GradParams gp{kernel_id, cnorm_of(kernel_id), 0};
   nbk::GradOut go;
   go.gv = out;
-  nbk::launch_gradients<int64_t>(rows ? nrows : n, rows, W.pk0, W.pk1, W.pk2, nullptr, offset,
-                                 index, gp, nullptr, go, st);
+  nbk::launch_gradients(rows ? nrows : n, rows, W.pk0, W.pk1, nullptr, offset, index, kernel_id,
+                        cnorm_of(kernel_id), go, st);
   NB_CUDA(cudaGetLastError());
   return nbk::check_device_error(E, st);
 }
@@ -400,10 +396,8 @@ int nb_disc_forces(nb_ctx* ctx, int64_t n, const double* pos, const double* vel,
   NB_TRY(E.ws.ensure(E, n));
   nbk::Workspace& W = E.ws;
   cudaStream_t st = S(stream);
-  nbk::pack_pos(n, pos, nullptr, W.pk0, st);
-  nbk::pack_vm(n, vel, mass, W.pk1, st);
-  nbk::pack4(n, h, rho, omega, nullptr, W.pk2, st);
-  nbk::pack4(n, nullptr, c_s, nullptr, nullptr, W.pk3, st);
+  nbk::pack_forces64(n, pos, vel, mass, h, rho, omega, nullptr, nullptr, c_s, nullptr, W.pk0,
+                     W.pk1, W.pk2, W.pk3, st);
   nbk::ForceParams fp{};
   fp.kid = kernel_id;
   fp.cnorm = cnorm_of(kernel_id);

@@ -444,6 +444,18 @@ __global__ void k_pack_sorted4(int64_t n, const int32_t* __restrict__ perm, cons
   out[k] = make_double4(a ? a[i] : 0.0, b ? b[i] : 0.0, c ? c[i] : 0.0, d ? d[i] : 0.0);
 }
 
+// the FP64 force pass's hydro record (1/h, rho, 1/(Omega rho^2), P)
+__global__ void k_pack_hydro64(int64_t n, const int32_t* __restrict__ perm,
+                               const double* __restrict__ h, const double* __restrict__ rho,
+                               const double* __restrict__ omega, const double* __restrict__ P,
+                               double4* __restrict__ out) {
+  int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int64_t i = perm[k];
+  const double r = rho[i];
+  out[k] = make_double4(1.0 / h[i], r, 1.0 / (omega[i] * r * r), P[i]);
+}
+
 // FP32 positions: the cell of a uniform grid (edge `cell`, at most 1024 per axis, corner lo) and
 // the float offset from the cell centre, as two float4 per particle: (offset, mass) and (cell
 // coordinates as exact floats, h); mass and h 0 when not given.
@@ -1159,13 +1171,12 @@ int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, in
   }
   if (prm->precision != 1 || sw_on || recon) {
     // FP64 packs (the FP32 form needs them only for the gradient passes)
-    count_launch(), k_pack_sorted<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, vel, s->mass, W.pk1);
-    count_launch(), k_pack_sorted4<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, s->h, s->rho, s->omega, W.d_P, W.pk2);
-  }
-  if (sw_on || recon) {
-    NB_TRY(W.ensure_grad(E, n));
     count_launch(), k_pack_sorted<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, s->x, s->h, W.pk0);
+    count_launch(), k_pack_sorted<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, vel, s->mass, W.pk1);
   }
+  if (prm->precision != 1)
+    count_launch(), k_pack_hydro64<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, s->h, s->rho, s->omega, W.d_P, W.pk2);
+  if (sw_on || recon) NB_TRY(W.ensure_grad(E, n));
   if (sw_on || recon) {
     // Cullen-Dehnen switch (sim/blocks.py:261-266, sim/coupled.py:159-162): corrected gradients
     // of the rows over their interacting pairs with the previous accelerations, then alpha of
@@ -1176,7 +1187,10 @@ int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, in
     if (sw_on)
       count_launch(), k_pack_sorted<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, s->a_hydro, nullptr, W.pk4);
     GradOut go;
-    go.gv = W.gvel;
+    if (prm->precision == 1)
+      go.gv = W.gvel;
+    else
+      go.gs = reinterpret_cast<double4*>(W.gvel);
     go.alpha = s->alpha;
     go.cs = W.d_cs;
     go.h = s->h;
@@ -1185,7 +1199,7 @@ int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, in
     go.n_end = sk.n_end;
     go.tick = sk.tick;
     E.prof.begin(st);
-    launch_shock_gradients(n, W.pk0, W.pk1, W.pk2, W.pk4, L.off, L.idx, prm->kernel_id,
+    launch_shock_gradients(n, W.pk0, W.pk1, W.pk4, L.off, L.idx, prm->kernel_id,
                            prm->cnorm, recon ? 1 : 0, sk.recon_full,
                            sk.recon_full ? touched : nullptr, sw_on ? W.m_sorted : nullptr,
                            L.perm, go, st);
@@ -1222,8 +1236,7 @@ int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, in
     fp.tcnt = W.i32a;
   }
   if (want_tight && prm->precision == 1) {
-    if (!fused_pack) count_launch(), k_pack_sorted<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, s->x, s->h, W.pk0);
-    fp.pos64 = W.pk0;
+    fp.pos64 = W.pk0;  // packed above, or with the other FP32 records below
   }
   if (recon) {
     fp.use_recon = 1;
@@ -1231,7 +1244,7 @@ int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, in
     fp.gate = prm->recon_gate;
     fp.eta_crit = prm->recon_eta_crit;
     fp.eta_fold = prm->recon_eta_fold;
-    fp.gv64 = W.gvel;
+    fp.gs64 = reinterpret_cast<const double4*>(W.gvel);
     fp.gv32 = W.gvel32;
   }
   ForceOut fo;
@@ -1254,7 +1267,6 @@ int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, in
     launch_forces32<int32_t>(nrows, W.rows_s, W.pk32, E.bbox, W.pf1, W.pf2, W.pf3, L.off,
                              L.idx, fp, L.perm, fo, st);
   } else {
-    count_launch(), k_pack_sorted<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, s->x, nullptr, W.pk0);
     E.prof.begin(st);
     launch_forces64<int32_t>(nrows, W.rows_s, W.pk0, W.pk1, W.pk2, W.pk3, L.off, L.idx, fp,
                              L.perm, fo, st);

@@ -39,54 +39,53 @@ void launch_forces64(int64_t nrows, const int64_t* rows, const double4* pos, con
                      const double4* hydro, const double4* aux, const int64_t* off, const I* idx,
                      ForceParams prm, const int32_t* out_map, ForceOut out, cudaStream_t st) {
   if (nrows <= 0) return;
-  Pos64 geo{pos};
-  if (prm.use_recon && prm.use_visc)
-    count_launch(), k_forces_g<double, Pos64, I, double4, true><<<grid_for(nrows * 8), NB_THREADS, 0, st>>>(
-        nrows, rows, geo, vm, hydro, aux, off, idx, prm, out_map, out);
+  auto run = [&](auto sph, auto disc, auto recon) {
+    constexpr bool S = decltype(sph)::value, D = decltype(disc)::value, R = decltype(recon)::value;
+    // the caller-order lists come tightened, the engine's sorted lists are tested by the walk
+    constexpr bool T = sizeof(I) == 4;
+    count_launch(), k_forces64<S, D, R, T, I><<<grid_for(nrows * 8, F64_THREADS), F64_THREADS, 0, st>>>(
+        nrows, rows, pos, vm, hydro, aux, prm.gs64, off, idx, prm, out_map, out);
+  };
+  const std::true_type yes;
+  const std::false_type no;
+  const bool recon = prm.use_recon && prm.use_visc;
+  if (!prm.use_sph)
+    run(no, yes, no);
+  else if (recon && prm.use_disc)
+    run(yes, yes, yes);
+  else if (recon)
+    run(yes, no, yes);
+  else if (prm.use_disc)
+    run(yes, yes, no);
   else
-    count_launch(), k_forces_g<double, Pos64, I, double4, false><<<grid_for(nrows * 8), NB_THREADS, 0, st>>>(
-        nrows, rows, geo, vm, hydro, aux, off, idx, prm, out_map, out);
+    run(yes, no, no);
 }
 
-template <typename I>
 void launch_gradients(int64_t nrows, const int64_t* rows, const double4* pos, const double4* vm,
-                      const double4* hydro, const double4* acc, const int64_t* off, const I* idx,
-                      GradParams prm, const int32_t* out_map, GradOut out, cudaStream_t st) {
+                      const double4* acc, const int64_t* off, const int64_t* idx, int kid,
+                      double cnorm, GradOut out, cudaStream_t st) {
   if (nrows <= 0) return;
-  Pos64 geo{pos};
   if (acc)
-    count_launch(), k_gradients<I, true><<<grid_for(nrows * 8), NB_THREADS, 0, st>>>(
-        nrows, rows, geo, vm, hydro, acc, off, idx, prm, out_map, out);
+    count_launch(), k_gradients<int64_t, true><<<grid_for(nrows * 8), NB_THREADS, 0, st>>>(
+        nrows, rows, pos, vm, acc, off, idx, kid, cnorm, out);
   else
-    count_launch(), k_gradients<I, false><<<grid_for(nrows * 8), NB_THREADS, 0, st>>>(
-        nrows, rows, geo, vm, hydro, acc, off, idx, prm, out_map, out);
+    count_launch(), k_gradients<int64_t, false><<<grid_for(nrows * 8), NB_THREADS, 0, st>>>(
+        nrows, rows, pos, vm, acc, off, idx, kid, cnorm, out);
 }
 
-void launch_shock_gradients(int64_t n, const double4* pos, const double4* vm,
-                            const double4* hydro, const double4* acc, const int64_t* off,
-                            const int32_t* idx, int kid, double cnorm, int recon, int recon_full,
-                            const uint8_t* live_mask, const uint8_t* row_sorted,
-                            const int32_t* perm, GradOut out, cudaStream_t st) {
+void launch_shock_gradients(int64_t n, const double4* pos, const double4* vm, const double4* acc,
+                            const int64_t* off, const int32_t* idx, int kid, double cnorm,
+                            int recon, int recon_full, const uint8_t* live_mask,
+                            const uint8_t* row_sorted, const int32_t* perm, GradOut out,
+                            cudaStream_t st) {
   if (n <= 0) return;
-  Pos64 geo{pos};
   if (row_sorted)
     count_launch(), k_shock_grad<int32_t, true><<<grid_for(n * 8), NB_THREADS, 0, st>>>(
-        n, geo, vm, hydro, acc, off, idx, kid, cnorm, recon, recon_full, live_mask, row_sorted,
-        perm, out);
+        n, pos, vm, acc, off, idx, kid, cnorm, recon, recon_full, live_mask, row_sorted, perm, out);
   else
     count_launch(), k_shock_grad<int32_t, false><<<grid_for(n * 8), NB_THREADS, 0, st>>>(
-        n, geo, vm, hydro, acc, off, idx, kid, cnorm, recon, recon_full, live_mask, row_sorted,
-        perm, out);
+        n, pos, vm, acc, off, idx, kid, cnorm, recon, recon_full, live_mask, row_sorted, perm, out);
 }
-
-template void launch_gradients<int64_t>(int64_t, const int64_t*, const double4*, const double4*,
-                                        const double4*, const double4*, const int64_t*,
-                                        const int64_t*, GradParams, const int32_t*, GradOut,
-                                        cudaStream_t);
-template void launch_gradients<int32_t>(int64_t, const int64_t*, const double4*, const double4*,
-                                        const double4*, const double4*, const int64_t*,
-                                        const int32_t*, GradParams, const int32_t*, GradOut,
-                                        cudaStream_t);
 
 template void launch_density64<int64_t>(int64_t, const int64_t*, const double4*, const double*,
                                         const double*, const double*, const int64_t*,
@@ -115,12 +114,26 @@ __global__ void k_pack_pos(int64_t n, const double* __restrict__ pos, const doub
   out[i] = make_double4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], w ? w[i] : 0.0);
 }
 
-__global__ void k_pack4(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
-                        const double* __restrict__ c, const double* __restrict__ d,
-                        double4* __restrict__ out) {
+__global__ void k_pack_forces64(int64_t n, const double* __restrict__ pos,
+                                const double* __restrict__ vel, const double* __restrict__ m,
+                                const double* __restrict__ h, const double* __restrict__ rho,
+                                const double* __restrict__ omega, const double* __restrict__ P,
+                                const double* __restrict__ u, const double* __restrict__ cs,
+                                const double* __restrict__ alpha, double4* __restrict__ pk0,
+                                double4* __restrict__ pk1, double4* __restrict__ pk2,
+                                double4* __restrict__ pk3) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[i] = make_double4(a ? a[i] : 0.0, b ? b[i] : 0.0, c ? c[i] : 0.0, d ? d[i] : 0.0);
+  const double hi = h[i], ri = rho[i];
+  pk0[i] = make_double4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], hi);
+  pk1[i] = make_double4(vel[3 * i], vel[3 * i + 1], vel[3 * i + 2], m[i]);
+  pk2[i] = make_double4(1.0 / hi, ri, 1.0 / (omega[i] * ri * ri), P ? P[i] : 0.0);
+  pk3[i] = make_double4(u ? u[i] : 0.0, cs ? cs[i] : 0.0, alpha ? alpha[i] : 0.0, 0.0);
+}
+
+__global__ void k_pack_sym(int64_t n, const double* __restrict__ gv, double4* __restrict__ out) {
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) store_sym(out + 2 * i, gv + 9 * i);
 }
 
 __global__ void k_pack_vm(int64_t n, const double* __restrict__ vel, const double* __restrict__ m,
@@ -134,9 +147,16 @@ __global__ void k_pack_vm(int64_t n, const double* __restrict__ vel, const doubl
 void pack_pos(int64_t n, const double* pos, const double* w, double4* out, cudaStream_t st) {
   if (n > 0) count_launch(), k_pack_pos<<<grid_for(n), NB_THREADS, 0, st>>>(n, pos, w, out);
 }
-void pack4(int64_t n, const double* a, const double* b, const double* c, const double* d,
-           double4* out, cudaStream_t st) {
-  if (n > 0) count_launch(), k_pack4<<<grid_for(n), NB_THREADS, 0, st>>>(n, a, b, c, d, out);
+void pack_forces64(int64_t n, const double* pos, const double* vel, const double* mass,
+                   const double* h, const double* rho, const double* omega, const double* P,
+                   const double* u, const double* cs, const double* alpha, double4* pk0,
+                   double4* pk1, double4* pk2, double4* pk3, cudaStream_t st) {
+  if (n > 0)
+    count_launch(), k_pack_forces64<<<grid_for(n), NB_THREADS, 0, st>>>(
+        n, pos, vel, mass, h, rho, omega, P, u, cs, alpha, pk0, pk1, pk2, pk3);
+}
+void pack_sym(int64_t n, const double* gv, double4* out, cudaStream_t st) {
+  if (n > 0) count_launch(), k_pack_sym<<<grid_for(n), NB_THREADS, 0, st>>>(n, gv, out);
 }
 void pack_vm(int64_t n, const double* vel, const double* m, double4* out, cudaStream_t st) {
   if (n > 0) count_launch(), k_pack_vm<<<grid_for(n), NB_THREADS, 0, st>>>(n, vel, m, out);

@@ -15,26 +15,14 @@
 namespace nbk {
 
 // ---------------------------------------------------------------- position differences
-// FP64: packed (x, y, z, w) doubles.  dx = x_j - x_i as the reference forms it.
+// FP64 density: packed (x, y, z, mass) doubles.
 struct Pos64 {
   const double4* p;
   struct Own {
     double4 a;
   };
-  __device__ __forceinline__ void ready() {}
   __device__ __forceinline__ Own own(int64_t i) const { return Own{p[i]}; }
-  __device__ __forceinline__ void diff(const Own& o, int64_t j, double& dx, double& dy,
-                                       double& dz) const {
-    const double4 b = p[j];
-    dx = b.x - o.a.x;
-    dy = b.y - o.a.y;
-    dz = b.z - o.a.z;
-  }
-  __device__ __forceinline__ void diff(int64_t i, int64_t j, double& dx, double& dy,
-                                       double& dz) const {
-    diff(own(i), j, dx, dy, dz);
-  }
-  // the difference and particle j's mass (the record's w, where the pass packs it there)
+  // the difference x_j - x_i and particle j's mass (the record's w)
   __device__ __forceinline__ void diff_m(const Own& o, int64_t j, double& dx, double& dy,
                                          double& dz, double& m) const {
     const double4 b = ld_rec(p + j);
@@ -42,18 +30,6 @@ struct Pos64 {
     dy = b.y - o.a.y;
     dz = b.z - o.a.z;
     m = b.w;
-  }
-  // the difference and particle j's smoothing length (from the hydro record)
-  template <typename V4>
-  __device__ __forceinline__ void diff_h(const Own& o, int64_t j, const V4* __restrict__ hydro,
-                                         double& dx, double& dy, double& dz, double& hj) const {
-    diff(o, j, dx, dy, dz);
-    hj = (double)hydro[j].x;
-  }
-  template <typename V4>
-  __device__ __forceinline__ void diff_h(int64_t i, int64_t j, const V4* __restrict__ hydro,
-                                         double& dx, double& dy, double& dz, double& hj) const {
-    diff_h(own(i), j, hydro, dx, dy, dz, hj);
   }
 };
 
@@ -652,15 +628,13 @@ constexpr int FORCE_QUEUE = 64;  // interacting entries a row queues before its 
 // interacting entries (self included, list order) to prm.tidx / prm.tcnt, with few registers
 // and so many resident warps to hide the walk's dependent loads; MODE 2 then reads those
 // entries, every lane busy on pair terms, with no walk state alive beside the accumulators.
-template <int MODE, typename R, bool RECON>
+template <int MODE, bool RECON>
 struct ForceBlocks {
-  static constexpr int value = MODE == 1 ? WALK_BLOCKS
-                               : sizeof(R) == 4 ? (RECON ? 2 : FORCE_BLOCKS_PER_SM_FP32)
-                                                : (RECON ? 1 : 2);
+  static constexpr int value = MODE == 1 ? WALK_BLOCKS : RECON ? 2 : FORCE_BLOCKS_PER_SM_FP32;
 };
 
 template <typename R, typename PosT, typename I, typename V4, bool RECON, int MODE = 0>
-__global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, R, RECON>::value))
+__global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, RECON>::value))
     k_forces_g(int64_t nrows, const int64_t* __restrict__ rows, PosT geo_in,
              const V4* __restrict__ vm,    // (vx, vy, vz, mass)
              const V4* __restrict__ hydro, // (h, rho, omega, P)
@@ -710,22 +684,15 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, R, RECON>::valu
   for (int e = 0; e < 9; ++e) {
     if constexpr (!RECON)
       Ga[e] = R(0);
-    else if constexpr (sizeof(R) == 4)
-      Ga[e] = prm.gv32[9 * a + e];
     else
-      Ga[e] = (R)prm.gv64[9 * a + e];
+      Ga[e] = prm.gv32[9 * a + e];
   }
   const R eta_crit = (R)prm.eta_crit, eta_fold = (R)prm.eta_fold;
   auto recon_visc = [&](int64_t b, R dx0, R dx1, R dx2, R r, R rx, R ry, R rz, R h_b, R vdotr,
                         const V4& vb, const V4& xb, R rho_b, R m_b, R fa, R& num_a, R& num_b) {
     R Gb[9];
 #pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      if constexpr (sizeof(R) == 4)
-        Gb[e] = prm.gv32[9 * b + e];
-      else
-        Gb[e] = (R)prm.gv64[9 * b + e];
-    }
+    for (int e = 0; e < 9; ++e) Gb[e] = prm.gv32[9 * b + e];
     const R ga0 = Ga[0] * dx0 + Ga[1] * dx1 + Ga[2] * dx2;
     const R ga1 = Ga[3] * dx0 + Ga[4] * dx1 + Ga[5] * dx2;
     const R ga2 = Ga[6] * dx0 + Ga[7] * dx1 + Ga[8] * dx2;
@@ -771,78 +738,6 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, R, RECON>::valu
       vheat.add(-dh);
     }
   };
-  auto pair = [&](int64_t b) {
-    R ddx, ddy, ddz;
-    geo.diff(a, b, ddx, ddy, ddz);  // x_b - x_a
-    const V4 hb4 = hydro[b];
-    const R h_b = (R)hb4.x;
-    R d2 = sqdist(ddx, ddy, ddz);
-    npairs += 1;
-    const V4 vb = vm[b];
-    const R rho_b = (R)hb4.y, om_b = (R)hb4.z, P_b = (R)hb4.w;
-    const R m_b = (R)vb.w;
-    R r = sqrt(d2);
-    R rx = -ddx / r, ry = -ddy / r, rz = -ddz / r;  // r_hat of x_a - x_b
-    R fa = dwdr<R>(r, h_a, kid, cn);
-    R fb = dwdr<R>(r, h_b, kid, cn);
-    // velocity differences are formed in double before rounding, so a large common (orbital)
-    // velocity costs the FP32 path no precision
-    const R dvx = (R)(va.x - vb.x), dvy = (R)(va.y - vb.y), dvz = (R)(va.z - vb.z);
-    R vdotr = dvx * rx + dvy * ry + dvz * rz;
-    R num_a = P_a, num_b = P_b;
-    R inv_orr_b = R(1) / (om_b * rho_b * rho_b);
-    if (prm.use_sph) {
-      if (prm.use_visc) {
-        const V4 xb = aux[b];
-        if constexpr (RECON) {
-          recon_visc(b, -ddx, -ddy, -ddz, r, rx, ry, rz, h_b, vdotr, vb, xb, rho_b, m_b, fa,
-                     num_a, num_b);
-        } else {
-          R vsig_a = al_a * cs_a + beta * fabs(vdotr);
-          R vsig_b = (R)xb.z * (R)xb.y + beta * fabs(vdotr);
-          if (vsig_a > vmax) vmax = vsig_a;
-          if (vdotr < R(0)) {
-            num_a += R(-0.5) * rho_a * vsig_a * vdotr;
-            num_b += R(-0.5) * rho_b * vsig_b * vdotr;
-            R dh = m_b * vsig_a * R(0.5) * vdotr * vdotr * fa * inv_or_a;
-            heat.add(-dh);
-            vheat.add(-dh);
-          }
-        }
-        if (prm.use_cond) {
-          R vu;
-          if (prm.cond_signal == 0)
-            vu = sqrt(fabs(P_a - P_b) / (R(0.5) * (rho_a + rho_b)));
-          else
-            vu = fabs(vdotr);
-          R dc = m_b * alpha_u * vu * (R)(xa.x - xb.x) * R(0.5) *
-                 (fa * inv_or_a + fb / (om_b * rho_b));
-          heat.add(dc);
-          cheat.add(dc);
-        }
-      }
-      R f = m_b * (num_a * inv_orr_a * fa + num_b * inv_orr_b * fb);
-      ax.add(-f * rx);
-      ay.add(-f * ry);
-      az.add(-f * rz);
-      work.add(m_b * vdotr * fa);
-    }
-    if (prm.use_disc) {
-      // the reference's disc kernel forms its terms in its own order (sim/sph.py:1097-1114)
-      const V4 xb = aux[b];
-      R ex = -ddx, ey = -ddy, ez = -ddz;  // x_a - x_b
-      R vdr = dvx * ex / r;
-      vdr = vdr + dvy * ey / r;
-      vdr = vdr + dvz * ez / r;
-      R qa = -rho_a * h_a / (R(2) * r) * aav * cs_a * vdr * (R(1) / (om_a * rho_a * rho_a));
-      R qb = -rho_b * h_b / (R(2) * r) * aav * (R)xb.y * vdr / (om_b * rho_b * rho_b);
-      R f = m_b * (qa * fa + qb * fb);
-      dax.add(-(f * ex / r));
-      day.add(-(f * ey / r));
-      daz.add(-(f * ez / r));
-      dheat.add(m_b * qa * vdr * fa);
-    }
-    };
   // FP32 form: the same terms with one reciprocal square root per pair and reciprocals of the
   // per-particle denominators instead of divisions (rounding differs from the FP64 form by a few
   // float ulps, far inside the FP32 tolerances)
@@ -918,10 +813,7 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, R, RECON>::valu
   };
   auto drain = [&]() {
     for (int k2 = gl; k2 < pc; k2 += 8) {
-      if constexpr (sizeof(R) == 4)
-        pair_fast((int64_t)pq[k2]);
-      else
-        pair((int64_t)pq[k2]);
+      pair_fast((int64_t)pq[k2]);
     }
     __syncwarp();
     pc = 0;
@@ -936,10 +828,7 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, R, RECON>::valu
     for (int k2 = gl; k2 < cnt; k2 += 8) {
       const int64_t b = (int64_t)ld_stream(prm.tidx + e_beg + k2);
       if (b == a) continue;
-      if constexpr (sizeof(R) == 4)
-        pair_fast(b);
-      else
-        pair(b);
+      pair_fast(b);
     }
   }
   // FORCE_UNROLL rounds of eight entries at a time: their index and position loads are issued
@@ -971,13 +860,11 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, R, RECON>::valu
             R rr = R(2) * (h_a > h_b ? h_a : h_b);
             const R d2 = sqdist(ddx, ddy, ddz), r2 = rr * rr;
             tk = d2 < r2;
-            if constexpr (sizeof(R) == 4) {
-              if (prm.pos64 && d2 > r2 * R(1.0 - 1e-5) && d2 < r2 * R(1.0 + 1e-5)) {
-                const double4 pa = prm.pos64[a], pb = prm.pos64[b];
-                const double e2 = d2_exact(pb.x - pa.x, pb.y - pa.y, pb.z - pa.z);
-                const double er = 2.0 * fmax(pa.w, pb.w);
-                tk = e2 < er * er;
-              }
+            if (prm.pos64 && d2 > r2 * R(1.0 - 1e-5) && d2 < r2 * R(1.0 + 1e-5)) {
+              const double4 pa = prm.pos64[a], pb = prm.pos64[b];
+              const double e2 = d2_exact(pb.x - pa.x, pb.y - pa.y, pb.z - pa.z);
+              const double er = 2.0 * fmax(pa.w, pb.w);
+              tk = e2 < er * er;
             }
           }
           take[u] = tk;
@@ -1054,6 +941,250 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, R, RECON>::valu
   if (out.pairs) out.pairs[o] = npairs;
 }
 
+// ---------------------------------------------------------------- forces, FP64
+// The same pass in double (sim/sph.py:519-652, 568-609, 1084-1117).  What a division would give per
+// pair is precomputed per particle: the records are (x, y, z, h), (v, m), (1/h, rho, 1/(Omega
+// rho^2), P), (u, c_s, alpha, -) and, with the reconstruction, the symmetric part of the velocity
+// gradient (xx, yy, zz, xy, xz, yz, -, -), each fetched in one 32-byte load; a pair needs one
+// reciprocal square root, and one division more with the reconstruction.
+//   SPH   pressure, viscosity, conductivity, P dV;  DISC  disc viscosity
+//   RECON velocity reconstruction (the jump only enters through its projections on the pair
+//         axis: with pa = dx.Ga dx and pb = dx.Gb dx the jump is v_ab . r_hat - phi/2 (pa + pb) / r,
+//         and the limiter 4 x / (1 + x)^2 of x = pa / pb is 4 pa pb / (pa + pb)^2)
+//   TIGHT the list holds entries beyond 2 max(h_a, h_b): the walk tests them, queues the
+//         interacting ones in shared memory and drains full queues with all lanes busy; without
+//         it every entry is a pair and the lanes take them straight from the list
+// Bound by the FP64 pipe and the gathers' latency at 12 to 24 resident warps (128 B per pair).
+// 148,000 torus rows of 58 pairs: 207 us with viscosity and conductivity, 165 us disc viscosity
+// (about 385 each with a division per term); 100,000 rows of 137 pairs with the reconstruction:
+// 423 us (898 with 3x3 gradients and 210 registers).
+constexpr int F64_THREADS = 128;
+
+template <bool SPH, bool DISC, bool RECON>
+struct F64Blocks {
+  // 4 and 5 blocks with the reconstruction spill (5: 1.40 ms against 1.08 for its case), 6 and 8
+  // without it gain nothing more
+  static constexpr int value = RECON ? 3 : !SPH ? 6 : DISC ? 4 : 5;
+};
+
+template <bool SPH, bool DISC, bool RECON, bool TIGHT, typename I>
+__global__ void __launch_bounds__(F64_THREADS, (F64Blocks<SPH, DISC, RECON>::value))
+    k_forces64(int64_t nrows, const int64_t* __restrict__ rows, const double4* __restrict__ pos,
+               const double4* __restrict__ vm, const double4* __restrict__ hyd,
+               const double4* __restrict__ aux, const double4* __restrict__ sym,
+               const int64_t* __restrict__ off, const I* __restrict__ idx, ForceParams prm,
+               const int32_t* __restrict__ out_map, ForceOut out) {
+  const unsigned FULL = 0xffffffffu;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t q = t >> 3;
+  const int gl = (int)(t & 7), g = (threadIdx.x & 31) >> 3;
+  const bool live = q < nrows;
+  if (!__any_sync(FULL, live)) return;  // warp-uniform
+  const int64_t a = live ? (rows ? rows[q] : q) : 0;
+  const double4 xa = pos[a], va = vm[a], ha = hyd[a], ua = aux[a];
+  const double ih_a = ha.x, rho_a = ha.y, iorr_a = ha.z, P_a = ha.w, cs_a = ua.y, al_a = ua.z;
+  const double cn4_a = prm.cnorm * (ih_a * ih_a) * (ih_a * ih_a);
+  const double ior_a = iorr_a * rho_a;  // 1 / (Omega rho)
+  const double beta = prm.beta;
+  // disc viscosity: q_a = k_a (v . r_hat) / r, with the pair's side b alike
+  const double disc_a = -0.5 * rho_a * xa.w * prm.disc_alpha_av * cs_a * iorr_a;
+  double4 sa0 = make_double4(0, 0, 0, 0), sa1 = sa0;
+  if constexpr (RECON) {
+    sa0 = sym[2 * a];
+    sa1 = sym[2 * a + 1];
+  }
+  double ax = 0, ay = 0, az = 0, work = 0, vheat = 0, cheat = 0;
+  double dax = 0, day = 0, daz = 0, dheat = 0;
+  double vmax = SPH && prm.use_visc ? cs_a : 0.0;
+  int npairs = 0;
+  auto pair = [&](int b) {
+    const double4 xb = ld_rec(pos + b), vb = ld_rec(vm + b), hb = ld_rec(hyd + b);
+    double4 ub = make_double4(0, 0, 0, 0);
+    if (DISC || prm.use_visc) ub = ld_rec(aux + b);
+    npairs += 1;
+    const double dx = xa.x - xb.x, dy = xa.y - xb.y, dz = xa.z - xb.z;
+    const double d2 = fma(dz, dz, fma(dy, dy, dx * dx));
+    const double ir = rsqrt(d2);
+    double r = d2 * ir;
+    if (!(r > 0.0)) r = d2;  // 0 and infinity, as a square root gives them
+    const double rx = dx * ir, ry = dy * ir, rz = dz * ir;
+    const double ih_b = hb.x, ih2 = ih_b * ih_b;
+    const double fa = cn4_a * kernel_df<double>(r * ih_a, prm.kid);
+    const double fb = prm.cnorm * (ih2 * ih2) * kernel_df<double>(r * ih_b, prm.kid);
+    const double m = vb.w;
+    const double vr = fma(va.z - vb.z, rz, fma(va.y - vb.y, ry, (va.x - vb.x) * rx));
+    if constexpr (SPH) {
+      double na = P_a, nb = hb.w;
+      if (prm.use_visc) {
+        double jump = vr;  // drives the viscosity
+        bool on = vr < 0.0;
+        if constexpr (RECON) {
+          const double4 sb0 = ld_rec(sym + 2 * (int64_t)b), sb1 = ld_rec(sym + 2 * (int64_t)b + 1);
+          const double xx = dx * dx, yy = dy * dy, zz = dz * dz;
+          const double xy = 2.0 * dx * dy, xz = 2.0 * dx * dz, yz = 2.0 * dy * dz;
+          const double pa = fma(sa1.y, yz, fma(sa1.x, xz, fma(sa0.w, xy, fma(sa0.z, zz, fma(sa0.y, yy, sa0.x * xx)))));
+          const double pb = fma(sb1.y, yz, fma(sb1.x, xz, fma(sb0.w, xy, fma(sb0.z, zz, fma(sb0.y, yy, sb0.x * xx)))));
+          double phi = 0.0;
+          const double pp = pa * pb;
+          if (pp > 0.0) {
+            const double s = pa + pb;
+            phi = fmin(4.0 * pp / (s * s), 1.0);
+            if (prm.closeness) {
+              const double eta_ab = r * fmin(ih_a, ih_b);
+              if (eta_ab < prm.eta_crit) {
+                const double c = (eta_ab - prm.eta_crit) / prm.eta_fold;
+                phi *= exp(-c * c);
+              }
+            }
+          }
+          jump = fma(-0.5 * phi * (pa + pb), ir, vr);
+          on = jump < 0.0 && vr < 0.0;
+          if (prm.gate == 1)
+            on = jump < 0.0;
+          else if (prm.gate == 2 && vr > jump)
+            jump = vr;
+        }
+        const double aj = fabs(jump);
+        const double vs_a = fma(beta, aj, al_a * cs_a), vs_b = fma(beta, aj, ub.z * ub.y);
+        const double cfl = RECON ? fma(beta, fabs(vr), al_a * cs_a) : vs_a;
+        if (cfl > vmax) vmax = cfl;
+        if (on) {
+          const double hj = -0.5 * jump;
+          na = fma(rho_a * vs_a, hj, na);
+          nb = fma(hb.y * vs_b, hj, nb);
+          vheat = fma(m * vs_a * hj * vr, fa * ior_a, vheat);
+        }
+        if (prm.use_cond) {
+          const double vu = prm.cond_signal == 0
+                                ? sqrt(fabs(P_a - hb.w) / (0.5 * (rho_a + hb.y)))
+                                : fabs(vr);
+          cheat = fma(m * prm.alpha_u * vu * (ua.x - ub.x) * 0.5,
+                      fma(fb, hb.z * hb.y, fa * ior_a), cheat);
+        }
+      }
+      const double f = -m * fma(nb * hb.z, fb, na * iorr_a * fa);
+      ax = fma(f, rx, ax);
+      ay = fma(f, ry, ay);
+      az = fma(f, rz, az);
+      work = fma(m * vr, fa, work);
+    }
+    if constexpr (DISC) {
+      const double s = vr * ir;
+      const double qa = disc_a * s;
+      const double qb = -0.5 * hb.y * xb.w * prm.disc_alpha_av * ub.y * hb.z * s;
+      const double f = -m * fma(qb, fb, qa * fa);
+      dax = fma(f, rx, dax);
+      day = fma(f, ry, day);
+      daz = fma(f, rz, daz);
+      dheat = fma(m * qa * vr, fa, dheat);
+    }
+  };
+  const int64_t e0 = live ? off[a] : 0;
+  const unsigned len = live ? (unsigned)(off[a + 1] - e0) : 0u;
+  const I* list = idx + e0;
+  if constexpr (!TIGHT) {
+    int next = gl < len ? (int)ld_stream(list + gl) : -1;
+    for (unsigned e = gl; e < len; e += 8) {
+      const int b = next;
+      next = e + 8 < len ? (int)ld_stream(list + e + 8) : -1;
+      if (b != (int)a) pair(b);
+    }
+  } else {
+    // rounds of eight entries, FORCE_UNROLL of them with their loads issued together; with
+    // prm.tidx the interacting entries (self included, list order) are also written out for the
+    // level limiter
+    constexpr int U = FORCE_UNROLL;
+    __shared__ int32_t queue_s[F64_THREADS / 8][FORCE_QUEUE + 8 * U];
+    int32_t* pq = queue_s[threadIdx.x >> 3];
+    int pc = 0, m_tot = 0;
+    auto drain = [&]() {
+      __syncwarp();
+      for (int k = gl; k < pc; k += 8) pair(pq[k]);
+      __syncwarp();
+      pc = 0;
+    };
+    const unsigned maxlen = __reduce_max_sync(FULL, len);
+    for (unsigned base = 0; base < maxlen; base += 8 * U) {
+      int bb[U];
+      bool near[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned e = base + 8 * u + gl;
+        bb[u] = e < len ? (int)ld_stream(list + e) : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        near[u] = false;
+        if (bb[u] >= 0) {
+          const double4 o = ld_rec(pos + bb[u]);
+          const double d2 = d2_exact(o.x - xa.x, o.y - xa.y, o.z - xa.z);
+          const double rr = 2.0 * (xa.w > o.w ? xa.w : o.w);
+          near[u] = bb[u] == (int)a || d2 < rr * rr;
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool take = near[u] && bb[u] != (int)a;
+        const unsigned below = (1u << gl) - 1u;
+        const unsigned seg = (__ballot_sync(FULL, take) >> (8 * g)) & 0xffu;
+        if (take) pq[pc + __popc(seg & below)] = bb[u];
+        pc += __popc(seg);
+        if (prm.tidx) {
+          const unsigned tseg = (__ballot_sync(FULL, near[u]) >> (8 * g)) & 0xffu;
+          if (near[u]) prm.tidx[e0 + m_tot + __popc(tseg & below)] = bb[u];
+          m_tot += __popc(tseg);
+        }
+      }
+      if (__any_sync(FULL, pc > FORCE_QUEUE - 8)) drain();
+    }
+    drain();
+    if (prm.tcnt && live && gl == 0) prm.tcnt[q] = m_tot;
+  }
+  if constexpr (SPH) {
+    ax = group_total(ax);
+    ay = group_total(ay);
+    az = group_total(az);
+    work = group_total(work);
+    vheat = group_total(vheat);
+    cheat = group_total(cheat);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      const double vo = __shfl_xor_sync(FULL, vmax, o);
+      vmax = vo > vmax ? vo : vmax;
+    }
+  }
+  if constexpr (DISC) {
+    dax = group_total(dax);
+    day = group_total(day);
+    daz = group_total(daz);
+    dheat = group_total(dheat);
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) npairs += __shfl_xor_sync(FULL, npairs, o);
+  if (!live || gl != 0) return;
+  const int64_t o = out_map ? (int64_t)out_map[a] : q;
+  if constexpr (SPH) {
+    if (out.acc) {
+      out.acc[3 * o + 0] = ax;
+      out.acc[3 * o + 1] = ay;
+      out.acc[3 * o + 2] = az;
+    }
+    if (out.dudt) out.dudt[o] = fma(P_a * iorr_a, work, vheat + cheat);
+    if (out.vsig) out.vsig[o] = vmax;
+    if (out.vheat) out.vheat[o] = vheat;
+    if (out.cheat) out.cheat[o] = cheat;
+  }
+  if constexpr (DISC) {
+    if (out.dacc) {
+      out.dacc[3 * o + 0] = dax;
+      out.dacc[3 * o + 1] = day;
+      out.dacc[3 * o + 2] = daz;
+    }
+    if (out.ddudt) out.ddudt[o] = dheat;
+  }
+  if (out.pairs) out.pairs[o] = npairs;
+}
+
 // ---------------------------------------------------------------- corrected gradients
 // Reference sim/sph.py:693-902 (_near_singular, _velocity_gradient_kernel, _gradients_kernel):
 //     R_lj = sum_b m_b (x_b - x_a)^l dW_ab(h_a)/dx_a^j,  G_kj = sum_b m_b (v_b - v_a)^k dW/dx_a^j,
@@ -1063,16 +1194,14 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, R, RECON>::valu
 // the adjugate over the determinant.  Eight lanes per row, FP64 only (the FP32 form converts).
 constexpr double SINGULAR_TOL = 1e-6;
 
-__device__ __forceinline__ double det3(const double* m) {
-  return m[0] * (m[4] * m[8] - m[5] * m[7]) - m[1] * (m[3] * m[8] - m[5] * m[6]) +
-         m[2] * (m[3] * m[7] - m[4] * m[6]);
-}
-
-// g <- g R^-1 (or the fallback) for the gradient sums g (3x3 row-major)
+// R is symmetric, (xx, yy, zz, xy, xz, yz); g <- g R^-1 (or the fallback) for the 3x3 row-major
+// gradient sums g
 template <int NG>
 __device__ __forceinline__ void corrected_gradients(const double* rm, int64_t cnt, double (*g)[9]) {
-  const double scale = (rm[0] + rm[4] + rm[8]) / 3.0;
-  const double det = det3(rm);
+  const double scale = (rm[0] + rm[1] + rm[2]) / 3.0;
+  const double c00 = rm[1] * rm[2] - rm[5] * rm[5], c01 = rm[5] * rm[4] - rm[3] * rm[2],
+               c02 = rm[3] * rm[5] - rm[1] * rm[4];
+  const double det = rm[0] * c00 + rm[3] * c01 + rm[4] * c02;
   const bool singular =
       cnt < 4 || !(scale > 0.0) || !(fabs(det) >= SINGULAR_TOL * scale * scale * scale);
   if (singular) {
@@ -1084,15 +1213,12 @@ __device__ __forceinline__ void corrected_gradients(const double* rm, int64_t cn
     return;
   }
   double ri[9];
-  ri[0] = (rm[4] * rm[8] - rm[5] * rm[7]) / det;
-  ri[1] = (rm[2] * rm[7] - rm[1] * rm[8]) / det;
-  ri[2] = (rm[1] * rm[5] - rm[2] * rm[4]) / det;
-  ri[3] = (rm[5] * rm[6] - rm[3] * rm[8]) / det;
-  ri[4] = (rm[0] * rm[8] - rm[2] * rm[6]) / det;
-  ri[5] = (rm[2] * rm[3] - rm[0] * rm[5]) / det;
-  ri[6] = (rm[3] * rm[7] - rm[4] * rm[6]) / det;
-  ri[7] = (rm[1] * rm[6] - rm[0] * rm[7]) / det;
-  ri[8] = (rm[0] * rm[4] - rm[1] * rm[3]) / det;
+  ri[0] = c00 / det;
+  ri[1] = ri[3] = c01 / det;
+  ri[2] = ri[6] = c02 / det;
+  ri[4] = (rm[0] * rm[2] - rm[4] * rm[4]) / det;
+  ri[5] = ri[7] = (rm[4] * rm[3] - rm[0] * rm[5]) / det;
+  ri[8] = (rm[0] * rm[1] - rm[3] * rm[3]) / det;
 #pragma unroll
   for (int k = 0; k < NG; ++k) {
     double o[9];
@@ -1105,6 +1231,73 @@ __device__ __forceinline__ void corrected_gradients(const double* rm, int64_t cn
 #pragma unroll
     for (int e = 0; e < 9; ++e) g[k][e] = o[e];
   }
+}
+
+// 100,000 rows of 137 entries: 197 us for the velocity gradients, 226 us with the accelerations
+// (299 and 333 with a square root and divisions per entry and all nine sums of R).
+// The sums R (symmetric) and G of one row (and of the accelerations, with ACC) over the entries of
+// a pass, each one rsqrt and fused adds: F(r, h_a) / r = cn4 f'(r / h_a) / r.
+// SKIP: entries with F(r, h_a) = 0 are passed over (the step's untightened lists hold many); without
+// it they add their zeros, as the operators' reference does.
+template <bool ACC, bool SKIP>
+struct GradSums {
+  double rm[6] = {0, 0, 0, 0, 0, 0}, gv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0},
+         ga[ACC ? 9 : 1] = {0};
+  // (dx, dy, dz) = x_a - x_b
+  __device__ __forceinline__ void add(double dx, double dy, double dz, double d2, double ih_a,
+                                      double cn4, int kid, const double4& va,
+                                      const double4* __restrict__ vm, const double4& aa,
+                                      const double4* __restrict__ acc, int64_t b, bool use_acc) {
+    const double ir = rsqrt(d2);
+    double r = d2 * ir;
+    if (!(r > 0.0)) r = d2;  // 0 and infinity, as a square root gives them
+    const double q = r * ih_a;
+    if (SKIP && !(q < 2.0)) return;
+    const double4 vb = ld_rec(vm + b);
+    const double mf = vb.w * (cn4 * kernel_df<double>(q, kid) * ir);
+    const double gx = mf * dx, gy = mf * dy, gz = mf * dz;
+    rm[0] = fma(-dx, gx, rm[0]);
+    rm[1] = fma(-dy, gy, rm[1]);
+    rm[2] = fma(-dz, gz, rm[2]);
+    rm[3] = fma(-dx, gy, rm[3]);
+    rm[4] = fma(-dx, gz, rm[4]);
+    rm[5] = fma(-dy, gz, rm[5]);
+    const double dv[3] = {vb.x - va.x, vb.y - va.y, vb.z - va.z};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      gv[3 * i] = fma(dv[i], gx, gv[3 * i]);
+      gv[3 * i + 1] = fma(dv[i], gy, gv[3 * i + 1]);
+      gv[3 * i + 2] = fma(dv[i], gz, gv[3 * i + 2]);
+    }
+    if constexpr (ACC) {
+      if (use_acc) {
+        const double4 ab = ld_rec(acc + b);
+        const double da[3] = {ab.x - aa.x, ab.y - aa.y, ab.z - aa.z};
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          ga[3 * i] = fma(da[i], gx, ga[3 * i]);
+          ga[3 * i + 1] = fma(da[i], gy, ga[3 * i + 1]);
+          ga[3 * i + 2] = fma(da[i], gz, ga[3 * i + 2]);
+        }
+      }
+    }
+  }
+  // sums over the row's eight lanes
+  __device__ __forceinline__ void total() {
+#pragma unroll
+    for (int e = 0; e < 6; ++e) rm[e] = group_total(rm[e]);
+#pragma unroll
+    for (int e = 0; e < 9; ++e) {
+      gv[e] = group_total(gv[e]);
+      if (ACC) ga[ACC ? e : 0] = group_total(ga[ACC ? e : 0]);
+    }
+  }
+};
+
+// the symmetric part of a velocity gradient as the force pass reads it (8 doubles)
+__device__ __forceinline__ void store_sym(double4* out, const double* g) {
+  out[0] = make_double4(g[0], g[4], g[8], 0.5 * (g[1] + g[3]));
+  out[1] = make_double4(0.5 * (g[2] + g[6]), 0.5 * (g[5] + g[7]), 0.0, 0.0);
 }
 
 // physics/viscosity.py:83-113: xi (Balsara), alpha_loc, decay time, then the jump to alpha_loc
@@ -1126,107 +1319,76 @@ __device__ __forceinline__ void switch_update(const GradOut& out, int64_t o, dou
   out.alpha[o] = a_loc > alpha ? a_loc : decayed;
 }
 
-template <typename I, bool ACC>
-__global__ void __launch_bounds__(NB_THREADS)
-    k_gradients(int64_t nrows, const int64_t* __restrict__ rows, Pos64 geo,
-                const double4* __restrict__ vm,     // (vx, vy, vz, mass)
-                const double4* __restrict__ hydro,  // (h, ...)
-                const double4* __restrict__ acc,    // (ax, ay, az, -), with ACC
-                const int64_t* __restrict__ off, const I* __restrict__ idx, GradParams prm,
-                const int32_t* __restrict__ out_map, GradOut out) {
-  const unsigned FULL = 0xffffffffu;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t q = t >> 3;
-  const int gl = (int)(t & 7);
-  bool live = q < nrows;
-  int64_t a = 0, o = 0;
-  if (live) {
-    a = rows ? rows[q] : q;
-    o = out_map ? (int64_t)out_map[a] : q;
-    if (!rows && prm.mask && !prm.mask[o]) live = false;
-  }
-  if (!__any_sync(FULL, live)) return;  // warp-uniform
-  const double4 va = vm[a];
-  const double h_a = hydro[a].x;
-  double4 aa = make_double4(0.0, 0.0, 0.0, 0.0);
-  if (ACC) aa = acc[a];
-  double rm[9], g[ACC ? 2 : 1][9];
-#pragma unroll
-  for (int e = 0; e < 9; ++e) {
-    rm[e] = 0.0;
-    g[0][e] = 0.0;
-    if (ACC) g[ACC ? 1 : 0][e] = 0.0;
-  }
-  int cnt = 0;
-  // eight lanes per row, each taking every eighth list entry; the sums are then added over
-  // the row's lanes
-  const int64_t e0 = live ? off[a] : 0, e1 = live ? off[a + 1] : 0;
-  for (int64_t k = e0 + gl; k < e1; k += 8) {
-    const int64_t b = (int64_t)ld_stream(idx + k);
-    if (b == a) continue;
-    double ddx, ddy, ddz;
-    geo.diff(a, b, ddx, ddy, ddz);  // x_b - x_a
-    if (prm.tighten) {
-      const double h_b = hydro[b].x;
-      const double rr = 2.0 * (h_a > h_b ? h_a : h_b);
-      if (!(sqdist(ddx, ddy, ddz) < rr * rr)) continue;
-    }
-    cnt += 1;
-    const double dx[3] = {-ddx, -ddy, -ddz};  // x_a - x_b
-    const double r = sqrt(dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2]);
-    const double f = dwdr<double>(r, h_a, prm.kid, prm.cnorm) / r;
-    const double4 vb = vm[b];
-    const double dv[3] = {vb.x - va.x, vb.y - va.y, vb.z - va.z};
-    double da[3] = {0.0, 0.0, 0.0};
-    if (ACC) {
-      const double4 ab = acc[b];
-      da[0] = ab.x - aa.x;
-      da[1] = ab.y - aa.y;
-      da[2] = ab.z - aa.z;
-    }
-    const double mf = vb.w * f;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const double gj = mf * dx[j];
-        rm[3 * i + j] -= dx[i] * gj;
-        g[0][3 * i + j] += dv[i] * gj;
-        if (ACC) g[ACC ? 1 : 0][3 * i + j] += da[i] * gj;
-      }
-  }
-#pragma unroll
-  for (int of = 4; of > 0; of >>= 1) {
-    cnt += __shfl_xor_sync(FULL, cnt, of);
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      rm[e] += __shfl_xor_sync(FULL, rm[e], of);
-      g[0][e] += __shfl_xor_sync(FULL, g[0][e], of);
-      if (ACC) g[ACC ? 1 : 0][e] += __shfl_xor_sync(FULL, g[ACC ? 1 : 0][e], of);
-    }
-  }
-  if (!live || gl != 0) return;
-  corrected_gradients<ACC ? 2 : 1>(rm, cnt, g);
-  const double* dv = g[0];
-  if (out.gv) {
-#pragma unroll
-    for (int e = 0; e < 9; ++e) out.gv[9 * a + e] = dv[e];
-  }
-  if (!ACC) return;
-  const double* dacc = g[ACC ? 1 : 0];
-  const double div = dv[0] + dv[4] + dv[8];
-  const double c0 = dv[7] - dv[5], c1 = dv[2] - dv[6], c2 = dv[3] - dv[1];
-  const double curl = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
+// div v, |curl v| and d(div v)/dt from the gradients of v and of the acceleration
+__device__ __forceinline__ void switch_scalars(const double (*g)[9], double& div, double& curl,
+                                               double& ddiv) {
+  const double* v = g[0];
+  div = v[0] + v[4] + v[8];
+  const double c0 = v[7] - v[5], c1 = v[2] - v[6], c2 = v[3] - v[1];
+  curl = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
   double sdd = 0.0;
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) sdd += dv[3 * i + j] * dv[3 * j + i];
-  const double ddiv = dacc[0] + dacc[4] + dacc[8] - sdd;
-  if (out.div) out.div[o] = div;
-  if (out.curl) out.curl[o] = curl;
-  if (out.ddiv) out.ddiv[o] = ddiv;
-  if (out.alpha) switch_update(out, o, div, curl, ddiv);
+    for (int j = 0; j < 3; ++j) sdd += v[3 * i + j] * v[3 * j + i];
+  ddiv = g[1][0] + g[1][4] + g[1][8] - sdd;
+}
+
+template <typename I, bool ACC>
+__global__ void __launch_bounds__(NB_THREADS, 2)
+    k_gradients(int64_t nrows, const int64_t* __restrict__ rows, const double4* __restrict__ pos,
+                const double4* __restrict__ vm,   // (vx, vy, vz, mass); pos: (x, y, z, h)
+                const double4* __restrict__ acc,  // (ax, ay, az, -), with ACC
+                const int64_t* __restrict__ off, const I* __restrict__ idx, int kid, double cnorm,
+                GradOut out) {
+  const unsigned FULL = 0xffffffffu;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t q = t >> 3;
+  const int gl = (int)(t & 7);
+  const bool live = q < nrows;
+  if (!__any_sync(FULL, live)) return;  // warp-uniform
+  const int64_t a = live ? (rows ? rows[q] : q) : 0;
+  const double4 xa = pos[a], va = vm[a];
+  const double4 aa = ACC ? acc[a] : make_double4(0.0, 0.0, 0.0, 0.0);
+  const double ih_a = 1.0 / xa.w, cn4 = cnorm * (ih_a * ih_a) * (ih_a * ih_a);
+  GradSums<ACC, false> s;
+  int cnt = 0;
+  // eight lanes per row, each taking every eighth list entry (the next one's index is on its way
+  // while an entry is summed); the sums are then added over the row's lanes
+  const int64_t e0 = live ? off[a] : 0, e1 = live ? off[a + 1] : 0;
+  int64_t next = e0 + gl < e1 ? (int64_t)ld_stream(idx + e0 + gl) : -1;
+  for (int64_t k = e0 + gl; k < e1; k += 8) {
+    const int64_t b = next;
+    next = k + 8 < e1 ? (int64_t)ld_stream(idx + k + 8) : -1;
+    if (b == a) continue;
+    cnt += 1;
+    const double4 xb = ld_rec(pos + b);
+    const double dx = xa.x - xb.x, dy = xa.y - xb.y, dz = xa.z - xb.z;
+    const double d2 = fma(dz, dz, fma(dy, dy, dx * dx));
+    s.add(dx, dy, dz, d2, ih_a, cn4, kid, va, vm, aa, acc, b, true);
+  }
+  s.total();
+#pragma unroll
+  for (int of = 4; of > 0; of >>= 1) cnt += __shfl_xor_sync(FULL, cnt, of);
+  if (!live || gl != 0) return;
+  double g[ACC ? 2 : 1][9];
+#pragma unroll
+  for (int e = 0; e < 9; ++e) {
+    g[0][e] = s.gv[e];
+    if (ACC) g[ACC ? 1 : 0][e] = s.ga[ACC ? e : 0];
+  }
+  corrected_gradients<ACC ? 2 : 1>(s.rm, cnt, g);
+  if (out.gv) {
+#pragma unroll
+    for (int e = 0; e < 9; ++e) out.gv[9 * a + e] = g[0][e];
+  }
+  if constexpr (ACC) {
+    double div, curl, ddiv;
+    switch_scalars(g, div, curl, ddiv);
+    if (out.div) out.div[q] = div;
+    if (out.curl) out.curl[q] = curl;
+    if (out.ddiv) out.ddiv[q] = ddiv;
+  }
 }
 
 // The switch and the reconstruction's gradients of a step in one walk of the cached lists
@@ -1238,14 +1400,14 @@ __global__ void __launch_bounds__(NB_THREADS)
 // the same order, and only the entry counts of the singular-matrix test differ: both are kept.
 //   live: particles whose gradient the reconstruction needs (mask, caller order; null = all),
 //         or none without it; rows: the switch's rows (sorted mask; null = no switch)
+//   pos: (x, y, z, h) records; out.gs (8 doubles per particle, for the FP64 force pass) or out.gv
 template <typename I, bool SW>
 __global__ void __launch_bounds__(NB_THREADS)
-    k_shock_grad(int64_t n, Pos64 geo, const double4* __restrict__ vm,
-                 const double4* __restrict__ hydro, const double4* __restrict__ acc,
-                 const int64_t* __restrict__ off, const I* __restrict__ idx, int kid,
-                 double cnorm, int recon, int recon_full, const uint8_t* __restrict__ live_mask,
-                 const uint8_t* __restrict__ row_sorted, const int32_t* __restrict__ perm,
-                 GradOut out) {
+    k_shock_grad(int64_t n, const double4* __restrict__ pos, const double4* __restrict__ vm,
+                 const double4* __restrict__ acc, const int64_t* __restrict__ off,
+                 const I* __restrict__ idx, int kid, double cnorm, int recon, int recon_full,
+                 const uint8_t* __restrict__ live_mask, const uint8_t* __restrict__ row_sorted,
+                 const int32_t* __restrict__ perm, GradOut out) {
   const unsigned FULL = 0xffffffffu;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t a = t >> 3;
@@ -1259,92 +1421,55 @@ __global__ void __launch_bounds__(NB_THREADS)
   }
   const bool live = need_g || is_row;
   if (!__any_sync(FULL, live)) return;  // warp-uniform
-  const double4 va = vm[live ? a : 0];
-  const double h_a = hydro[live ? a : 0].x;
+  const double4 xa = pos[live ? a : 0], va = vm[live ? a : 0];
   double4 aa = make_double4(0.0, 0.0, 0.0, 0.0);
   if (SW && is_row) aa = acc[a];
-  double rm[9], gv[9], ga[SW ? 9 : 1];
-#pragma unroll
-  for (int e = 0; e < 9; ++e) {
-    rm[e] = 0.0;
-    gv[e] = 0.0;
-    if (SW) ga[SW ? e : 0] = 0.0;
-  }
+  const double h_a = xa.w, ih_a = 1.0 / h_a, cn4 = cnorm * (ih_a * ih_a) * (ih_a * ih_a);
+  GradSums<SW, true> s;
   int cnt_f = 0, cnt_t = 0;
   const int64_t e0 = live ? off[a] : 0, e1 = live ? off[a + 1] : 0;
+  int64_t next = e0 + gl < e1 ? (int64_t)ld_stream(idx + e0 + gl) : -1;
   for (int64_t k = e0 + gl; k < e1; k += 8) {
-    const int64_t b = (int64_t)ld_stream(idx + k);
+    const int64_t b = next;
+    next = k + 8 < e1 ? (int64_t)ld_stream(idx + k + 8) : -1;
     if (b == a) continue;
     cnt_f += 1;
-    double ddx, ddy, ddz;
-    geo.diff(a, b, ddx, ddy, ddz);  // x_b - x_a
-    const double d2 = sqdist(ddx, ddy, ddz);
-    const double h_b = hydro[b].x;
-    const double rr = 2.0 * (h_a > h_b ? h_a : h_b);
+    const double4 xb = ld_rec(pos + b);
+    const double dx = xa.x - xb.x, dy = xa.y - xb.y, dz = xa.z - xb.z;
+    const double d2 = d2_exact(dx, dy, dz);
+    const double rr = 2.0 * (h_a > xb.w ? h_a : xb.w);
     if (d2 < rr * rr) cnt_t += 1;
-    const double dx[3] = {-ddx, -ddy, -ddz};  // x_a - x_b
-    const double r = sqrt(dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2]);
-    if (!(r / h_a < 2.0)) continue;  // F(r, h_a) = 0: every term below is an exact zero
-    const double f = dwdr<double>(r, h_a, kid, cnorm) / r;
-    const double4 vb = vm[b];
-    const double dv[3] = {vb.x - va.x, vb.y - va.y, vb.z - va.z};
-    double da[3] = {0.0, 0.0, 0.0};
-    if (SW && is_row) {
-      const double4 ab = acc[b];
-      da[0] = ab.x - aa.x;
-      da[1] = ab.y - aa.y;
-      da[2] = ab.z - aa.z;
-    }
-    const double mf = vb.w * f;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const double gj = mf * dx[j];
-        rm[3 * i + j] -= dx[i] * gj;
-        gv[3 * i + j] += dv[i] * gj;
-        if (SW) ga[SW ? 3 * i + j : 0] += da[i] * gj;
-      }
+    s.add(dx, dy, dz, d2, ih_a, cn4, kid, va, vm, aa, acc, b, is_row);
   }
+  s.total();
 #pragma unroll
   for (int of = 4; of > 0; of >>= 1) {
     cnt_f += __shfl_xor_sync(FULL, cnt_f, of);
     cnt_t += __shfl_xor_sync(FULL, cnt_t, of);
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {
-      rm[e] += __shfl_xor_sync(FULL, rm[e], of);
-      gv[e] += __shfl_xor_sync(FULL, gv[e], of);
-      if (SW) ga[SW ? e : 0] += __shfl_xor_sync(FULL, ga[SW ? e : 0], of);
-    }
   }
   if (!live || gl != 0) return;
   if (need_g) {
     double g1[1][9];
 #pragma unroll
-    for (int e = 0; e < 9; ++e) g1[0][e] = gv[e];
-    corrected_gradients<1>(rm, recon_full ? cnt_f : cnt_t, g1);
+    for (int e = 0; e < 9; ++e) g1[0][e] = s.gv[e];
+    corrected_gradients<1>(s.rm, recon_full ? cnt_f : cnt_t, g1);
+    if (out.gs)
+      store_sym(out.gs + 2 * a, g1[0]);
+    else {
 #pragma unroll
-    for (int e = 0; e < 9; ++e) out.gv[9 * a + e] = g1[0][e];
+      for (int e = 0; e < 9; ++e) out.gv[9 * a + e] = g1[0][e];
+    }
   }
   if (SW && is_row) {
     double g2[2][9];
 #pragma unroll
     for (int e = 0; e < 9; ++e) {
-      g2[0][e] = gv[e];
-      g2[1][e] = ga[SW ? e : 0];
+      g2[0][e] = s.gv[e];
+      g2[1][e] = s.ga[SW ? e : 0];
     }
-    corrected_gradients<2>(rm, cnt_t, g2);
-    const double* dvm = g2[0];
-    const double* dam = g2[1];
-    const double div = dvm[0] + dvm[4] + dvm[8];
-    const double c0 = dvm[7] - dvm[5], c1 = dvm[2] - dvm[6], c2 = dvm[3] - dvm[1];
-    const double curl = sqrt(c0 * c0 + c1 * c1 + c2 * c2);
-    double sdd = 0.0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-      for (int j = 0; j < 3; ++j) sdd += dvm[3 * i + j] * dvm[3 * j + i];
-    const double ddiv = dam[0] + dam[4] + dam[8] - sdd;
+    corrected_gradients<2>(s.rm, cnt_t, g2);
+    double div, curl, ddiv;
+    switch_scalars(g2, div, curl, ddiv);
     switch_update(out, o, div, curl, ddiv);
   }
 }
