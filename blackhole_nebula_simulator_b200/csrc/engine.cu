@@ -56,8 +56,8 @@ int Engine::ensure_n(int64_t n) {
     NB_CUDA(cudaMallocHost((void**)&h_err, sizeof(int) * 4));
     NB_CUDA(cudaMalloc((void**)&bbox, sizeof(double) * 8));
     NB_CUDA(cudaMallocHost((void**)&h_red, sizeof(double) * 64));
-    NB_CUDA(cudaMalloc((void**)&d_rowmax, 8 * sizeof(unsigned long long)));
-    NB_CUDA(cudaMallocHost((void**)&h_build, sizeof(int64_t) * 2));
+    NB_CUDA(cudaMalloc((void**)&d_rowmax, 16 * sizeof(unsigned long long)));
+    NB_CUDA(cudaMallocHost((void**)&h_build, sizeof(int64_t) * 4));
   }
   if (n <= cap_n && keys_a) return 0;
   int64_t c = std::max<int64_t>(n + n / 4, 1024);
@@ -98,6 +98,8 @@ int Engine::grow2(int64_t m) {
   int64_t c = std::max<int64_t>(m + m / 4, 256);
   if (node_lo) cudaFree(node_lo);
   if (node_hi) cudaFree(node_hi);
+  if (node_q) cudaFree(node_q);
+  NB_CUDA(cudaMalloc(&node_q, 32 * c));
   NB_CUDA(cudaMalloc((void**)&node_lo, sizeof(double4) * c));
   NB_CUDA(cudaMalloc((void**)&node_hi, sizeof(double4) * c));
   cap_nodes = c;
@@ -110,6 +112,8 @@ int Engine::ensure_sub(int64_t m) {
   int64_t c = std::max<int64_t>(m + m / 4, 256);
   if (sub_lo) cudaFree(sub_lo);
   if (sub_hi) cudaFree(sub_hi);
+  if (sub_q) cudaFree(sub_q);
+  NB_CUDA(cudaMalloc(&sub_q, 32 * c));
   NB_CUDA(cudaMalloc((void**)&sub_lo, sizeof(double4) * c));
   NB_CUDA(cudaMalloc((void**)&sub_hi, sizeof(double4) * c));
   cap_sub = c;
@@ -135,15 +139,23 @@ int Engine::ensure_leaves(int64_t m) {
   c = 0;
   NB_TRY(grow(E, leaf_bbase, c, m));
   c = 0;
+  NB_TRY(grow(E, leaf_ibase, c, m));
+  c = 0;
   NB_TRY(grow(E, leaf_ncand, c, m));
   cap_leaf = c;
   return 0;
 }
 
-int Engine::ensure_tiles(int64_t ncand, int64_t nbatch) {
+int Engine::ensure_tiles(int64_t ncand, int64_t nbatch, int64_t nitem) {
   Engine& E = *this;
   NB_TRY(grow(E, cands, cap_cands, std::max<int64_t>(ncand, 1)));
-  return grow(E, masks, cap_masks, std::max<int64_t>(nbatch * 32, 32));
+  NB_TRY(grow(E, masks, cap_masks, std::max<int64_t>(nbatch * 32, 32)));
+  if (nitem <= cap_items && items) return 0;
+  int64_t c = 0;
+  NB_TRY(grow(E, items, c, nitem));
+  cap_items = c;
+  c = 0;
+  return grow(E, part_count, c, cap_items * 32);
 }
 
 int Engine::ensure_deposit(int64_t n) {
@@ -197,9 +209,9 @@ int Engine::ensure_sort_keys(int64_t m) {
 }
 
 void Engine::release() {
-  void* ps[] = {dep_k0, dep_k1, dep_i0, dep_i1, dep_buf, d_err, bbox, bbox_part, keys_a, keys_b, vals_a, counts, node_lo, node_hi, sub_lo, sub_hi,
+  void* ps[] = {dep_k0, dep_k1, dep_i0, dep_i1, dep_buf, d_err, bbox, bbox_part, keys_a, keys_b, vals_a, counts, node_lo, node_hi, sub_lo, sub_hi, node_q, sub_q,
                 cub_tmp, sort_keys, red, lists.perm, lists.inv_perm, lists.spos, lists.off,
-                lists.idx, d_rowmax, tidx, leaf_cbase, leaf_bbase, leaf_ncand, cands, masks,
+                lists.idx, d_rowmax, tidx, leaf_cbase, leaf_bbase, leaf_ibase, leaf_ncand, cands, masks, items, part_count,
                 dep_count, brick_count, brick_cursor, brick_off, brick_pairs, brick_tasks};
   for (void* p : ps)
     if (p) cudaFree(p);

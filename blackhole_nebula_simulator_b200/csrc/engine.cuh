@@ -165,6 +165,7 @@ struct Engine {
   double4* node_hi = nullptr;
   double4* sub_lo = nullptr;  // sub-leaf boxes
   double4* sub_hi = nullptr;
+  void *node_q = nullptr, *sub_q = nullptr;  // the boxes' 32-byte records of the candidate walk
   int64_t cap_sub = 0;
   void* cub_tmp = nullptr;
   size_t cub_bytes = 0;
@@ -189,14 +190,16 @@ struct Engine {
   int ensure_bricks(int64_t nbricks);
   int ensure_brick_lists(int64_t pairs, int64_t tasks);
   int64_t list_slots = 0, cand_slots = 0;  // resident warps of the persistent list passes
+  int64_t wide_slots = 0;                  // blocks for the leaves with large frontiers
   int32_t* tidx = nullptr;  // interacting entries of the active rows, in the lists' layout
   int64_t cap_tidx = 0;
-  // list build: the longest row of the last build [0], the passes' work counters [2, 3] and the
-  // candidate and batch cursors [4, 5]
+  // list build: the longest row of the last build [0], the passes' work counters [2, 3], the
+  // candidate, batch and item cursors [4, 5, 6], the leaves with large frontiers [8]; the export's
+  // long rows [9]
   unsigned long long* d_rowmax = nullptr;
   // list build: per query leaf the start of its candidate list and of its masks and its number
   // of candidate sub-leaves; the candidate lists and the tests' hit masks (32 per batch)
-  int64_t *leaf_cbase = nullptr, *leaf_bbase = nullptr;
+  int64_t *leaf_cbase = nullptr, *leaf_bbase = nullptr, *leaf_ibase = nullptr;
   int32_t* leaf_ncand = nullptr;
   int64_t cap_leaf = 0;
   int32_t* cands = nullptr;
@@ -205,7 +208,11 @@ struct Engine {
   int64_t cap_masks = 0;
   int64_t last_cands = 0, last_batches = 0;
   int ensure_leaves(int64_t m);
-  int ensure_tiles(int64_t ncand, int64_t nbatch);
+  int ensure_tiles(int64_t ncand, int64_t nbatch, int64_t nitem);
+  // the tests' work items ((part << 32) | leaf) and their entries per row (32 per item)
+  uint64_t* items = nullptr;
+  uint32_t* part_count = nullptr;
+  int64_t cap_items = 0;
   int64_t* h_build = nullptr;  // pinned: total entries and longest row of the last build
   double* red = nullptr;      // reduction partials (doubles)
   double* h_red = nullptr;    // pinned host copy of small reductions

@@ -146,8 +146,57 @@ __global__ void k_gather_sorted(int64_t n, const int32_t* __restrict__ perm,
 }
 
 // ---------------------------------------------------------------- tree of boxes
+// A box as the candidate walk reads it, one 32-byte record: its corners on a 2^32 grid over the
+// particles' bounding box, rounded outward, and twice its largest h in units of that grid, rounded
+// up with 1e-6 to spare, so that a test on the records can only keep more than the exact one.
+struct Box32 {
+  uint32_t lx, ly, lz;
+  float reach;
+  uint32_t hx, hy, hz, pad;
+};
+
+// grid cells per unit length; 0 where the bounding box has no extent or is not finite
+__device__ __forceinline__ double box_scale(const double* __restrict__ box6) {
+  const double span = fmax(fmax(box6[3] - box6[0], box6[4] - box6[1]), box6[5] - box6[2]);
+  return span > 0.0 && isfinite(span) ? 4294967040.0 / span : 0.0;
+}
+
+__device__ __forceinline__ Box32 box32(const double4& lo, const double4& hi,
+                                       const double* __restrict__ box6) {
+  const double s = box_scale(box6);
+  Box32 b;
+  b.lx = __double2uint_rd(__dmul_rd(__dsub_rd(lo.x, box6[0]), s));
+  b.ly = __double2uint_rd(__dmul_rd(__dsub_rd(lo.y, box6[1]), s));
+  b.lz = __double2uint_rd(__dmul_rd(__dsub_rd(lo.z, box6[2]), s));
+  b.hx = __double2uint_ru(__dmul_ru(__dsub_ru(hi.x, box6[0]), s));
+  b.hy = __double2uint_ru(__dmul_ru(__dsub_ru(hi.y, box6[1]), s));
+  b.hz = __double2uint_ru(__dmul_ru(__dsub_ru(hi.z, box6[2]), s));
+  b.reach = __double2float_ru(2.0 * lo.w * s * (1.0 + 1e-6));
+  b.pad = 0;
+  return b;
+}
+
+__device__ __forceinline__ Box32 ld_box(const Box32* p) {
+  Box32 b;
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(b.lx), "=r"(b.ly), "=r"(b.lz), "=f"(b.reach), "=r"(b.hx), "=r"(b.hy), "=r"(b.hz),
+        "=r"(b.pad)
+      : "l"(p));
+  return b;
+}
+
+// whether two boxes may hold a pair within reach (every rounding on the keeping side)
+__device__ __forceinline__ bool box_near(const Box32& a, const Box32& b) {
+  const float gx = __uint2float_rd((max(b.lx, a.hx) - a.hx) + (max(a.lx, b.hx) - b.hx));
+  const float gy = __uint2float_rd((max(b.ly, a.hy) - a.hy) + (max(a.ly, b.hy) - b.hy));
+  const float gz = __uint2float_rd((max(b.lz, a.hz) - a.hz) + (max(a.lz, b.hz) - b.hz));
+  const float r = fmaxf(a.reach, b.reach);
+  return __fmaf_rd(gz, gz, __fmaf_rd(gy, gy, __fmul_rd(gx, gx))) <= __fmul_ru(r, r);
+}
+
 __global__ void k_leaf_boxes(int64_t n, int64_t nleaf, const double4* __restrict__ spos,
-                             double4* __restrict__ lo, double4* __restrict__ hi) {
+                             const double* __restrict__ box6, double4* __restrict__ lo,
+                             double4* __restrict__ hi, Box32* __restrict__ q) {
   int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (l >= nleaf) return;
   int64_t a = l * LEAF, b = min(a + LEAF, n);
@@ -164,11 +213,13 @@ __global__ void k_leaf_boxes(int64_t n, int64_t nleaf, const double4* __restrict
   }
   lo[l] = mn;
   hi[l] = mx;
+  q[l] = box32(mn, mx, box6);
 }
 
 // Boxes (and largest h) of the sub-leaves of SUB consecutive sorted particles.
 __global__ void k_sub_boxes(int64_t n, int64_t nsub, const double4* __restrict__ spos,
-                            double4* __restrict__ lo, double4* __restrict__ hi) {
+                            const double* __restrict__ box6, double4* __restrict__ lo,
+                            double4* __restrict__ hi, Box32* __restrict__ q) {
   int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (l >= nsub) return;
   int64_t a = l * SUB, b = min(a + SUB, n);
@@ -185,11 +236,13 @@ __global__ void k_sub_boxes(int64_t n, int64_t nsub, const double4* __restrict__
   }
   lo[l] = mn;
   hi[l] = mx;
+  q[l] = box32(mn, mx, box6);
 }
 
 __global__ void k_level_up(int64_t nchild, int64_t nparent, const double4* __restrict__ clo,
-                           const double4* __restrict__ chi, double4* __restrict__ plo,
-                           double4* __restrict__ phi) {
+                           const double4* __restrict__ chi, const double* __restrict__ box6,
+                           double4* __restrict__ plo, double4* __restrict__ phi,
+                           Box32* __restrict__ q) {
   int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= nparent) return;
   double4 mn = make_double4(1e308, 1e308, 1e308, 0.0), mx = make_double4(-1e308, -1e308, -1e308, 0.0);
@@ -205,11 +258,13 @@ __global__ void k_level_up(int64_t nchild, int64_t nparent, const double4* __res
   }
   plo[p] = mn;
   phi[p] = mx;
+  q[p] = box32(mn, mx, box6);
 }
 
 struct TreeView {
   const double4* lo;
   const double4* hi;
+  const Box32* q;  // the same boxes as the walk's records
   int64_t level_off[MAX_LEVELS + 1];
   int64_t level_size[MAX_LEVELS];
   int nlevels;
@@ -219,13 +274,6 @@ __device__ __forceinline__ double box_gap2(double4 alo, double4 ahi, double4 blo
   double gx = fmax(fmax(blo.x - ahi.x, alo.x - bhi.x), 0.0);
   double gy = fmax(fmax(blo.y - ahi.y, alo.y - bhi.y), 0.0);
   double gz = fmax(fmax(blo.z - ahi.z, alo.z - bhi.z), 0.0);
-  return gx * gx + gy * gy + gz * gz;
-}
-
-__device__ __forceinline__ double point_gap2(double x, double y, double z, double4 blo, double4 bhi) {
-  double gx = fmax(fmax(blo.x - x, x - bhi.x), 0.0);
-  double gy = fmax(fmax(blo.y - y, y - bhi.y), 0.0);
-  double gz = fmax(fmax(blo.z - z, z - bhi.z), 0.0);
   return gx * gx + gy * gy + gz * gz;
 }
 
@@ -333,43 +381,75 @@ __device__ __forceinline__ bool walk_candidates(int64_t n, const TreeView& tv, c
   return true;
 }
 
+// Where each query leaf's candidates, batches and work items lie, and the cursors that place them.
+// A work item is a stretch of at most `chunk` batches of one leaf, so that a leaf in reach of much
+// more than the others (a large h beside a dense region) is shared by as many warps as it needs.
+struct ListSlices {
+  int64_t *cbase, *bbase, *ibase;  // per leaf: first candidate, batch and item
+  int32_t* ncand;                  // per leaf: candidate sub-leaves
+  uint64_t* items;                 // (part << 32) | leaf
+  unsigned long long* cursor;      // candidates, batches, items taken so far
+  int64_t cap_cands, cap_batches, cap_items;
+  int chunk;
+};
+
+// One thread takes a leaf's slices with three atomic adds (so slices of different leaves lie in
+// any order).  Returns the first candidate, or -1 if a slice would pass its buffer's capacity:
+// nothing is written then; the host grows the buffers from the cursors' final values and runs
+// the pass again.
+__device__ __forceinline__ int64_t take_slices(const ListSlices& ls, int64_t leaf, int64_t count) {
+  const int64_t nbat = (count + 3) / 4;
+  const int64_t nit = nbat > ls.chunk ? (nbat + ls.chunk - 1) / ls.chunk : 1;
+  const int64_t cb = (int64_t)atomicAdd(ls.cursor, (unsigned long long)count);
+  const int64_t bb = (int64_t)atomicAdd(ls.cursor + 1, (unsigned long long)nbat);
+  const int64_t ib = (int64_t)atomicAdd(ls.cursor + 2, (unsigned long long)nit);
+  ls.cbase[leaf] = cb;
+  ls.bbase[leaf] = bb;
+  ls.ibase[leaf] = ib;
+  ls.ncand[leaf] = (int32_t)count;
+  if (cb + count > ls.cap_cands || bb + nbat > ls.cap_batches || ib + nit > ls.cap_items) return -1;
+  for (int64_t p = 0; p < nit; ++p) ls.items[ib + p] = ((uint64_t)p << 32) | (uint64_t)leaf;
+  return cb;
+}
+
+// whether child `c` of a level (its boxes at clo, chi, cq) is within reach of the query leaf
+__device__ __forceinline__ bool child_near(bool records, const QueryLeaf& q, const Box32& qb,
+                                           const double4* clo, const double4* chi,
+                                           const Box32* cq, int64_t c) {
+  if (records) return box_near(qb, ld_box(cq + c));
+  const double4 blo = clo[c], bhi = chi[c];
+  const double reach = 2.0 * fmax(q.lo.w, blo.w);
+  return box_gap2(q.lo, q.hi, blo, bhi) < reach * reach * (1.0 + 1e-12);
+}
+
 // Pass 1: the candidate sub-leaves of each query leaf, in ascending order, into its own slice of
 // the candidate buffer.  The walk goes level by level: the nodes within reach of the query box at
 // one level (a frontier in shared memory, ascending) give the next level's nodes to test, 32 at
 // a time, one per lane; the leaves within reach give the sub-leaves to test the same way, and the
 // sub-leaves within reach are the leaf's candidate list (ascending, since every frontier is).  A
-// frontier larger than its buffer sends the leaf to the depth-first walk instead, which counts
-// first and writes in a second walk.  The leaf takes its slices of the candidate and mask
-// buffers with two atomic adds (cand_at / batch_at, so slices of different leaves lie in any
-// order).  A slice that would pass the buffers' capacity is not written; the host then grows the
-// buffers from the cursors' final values and runs the pass again.
+// leaf whose frontier outgrows its buffer goes to the list `wide`, for k_lists_wide.
+// Latency bound (a dependent chain of box loads per level): 0.14 ms on the 1M torus, 0.54 on the
+// 4M torus, 0.04 on the 262,144-particle cloud.  With 64-byte boxes in double, and the few leaves
+// with large frontiers walked node by node by their warps, twice, 1.34, 2.3 and 0.04 ms.
 constexpr int CAND_WARPS = 4;
 #ifndef CAND_SMEM
 #define CAND_SMEM 1024  // entries of a frontier buffer
 #endif
 
-__global__ void __launch_bounds__(CAND_WARPS * 32) k_lists_cand(int64_t n, int64_t nwork,
-                                                           const uint64_t* __restrict__ order,
-                                                           unsigned long long* __restrict__ next,
-                                                           TreeView tv,
-                                                           const double4* __restrict__ slo,
-                                                           const double4* __restrict__ shi,
-                                                           unsigned long long* __restrict__ cand_at,
-                                                           unsigned long long* __restrict__ batch_at,
-                                                           int64_t cap_cands, int64_t cap_batches,
-                                                           int32_t* __restrict__ cands,
-                                                           int64_t* __restrict__ leaf_cbase,
-                                                           int64_t* __restrict__ leaf_bbase,
-                                                           int32_t* __restrict__ leaf_ncand,
-                                                           int* err) {
-  __shared__ int64_t stacks[CAND_WARPS][STACK];
+__global__ void __launch_bounds__(CAND_WARPS * 32) k_lists_cand(
+    int64_t n, int64_t nwork, const uint64_t* __restrict__ order,
+    unsigned long long* __restrict__ next, TreeView tv, const double4* __restrict__ slo,
+    const double4* __restrict__ shi, const Box32* __restrict__ sq, const double* __restrict__ box6,
+    ListSlices ls, int32_t* __restrict__ cands, int32_t* __restrict__ wide,
+    unsigned long long* __restrict__ nwide) {
   __shared__ int32_t fronts[CAND_WARPS][2][CAND_SMEM];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
-  int64_t* stack = stacks[threadIdx.x >> 5];
   int32_t(*front)[CAND_SMEM] = fronts[threadIdx.x >> 5];
   const int64_t nsub = (n + SUB - 1) / SUB;
+  // records where the grid resolves anything, else (a bounding box that is not finite) the doubles
+  const bool records = box_scale(box6) > 0.0;
   while (true) {
     unsigned long long t = 0;
     if (lane == 0) t = atomicAdd(next, 1ull);
@@ -377,7 +457,7 @@ __global__ void __launch_bounds__(CAND_WARPS * 32) k_lists_cand(int64_t n, int64
     if (t >= (unsigned long long)nwork) break;  // warp-uniform
     const int64_t leaf = (int64_t)(order[t] & 0xffffffffull);
     const QueryLeaf q = query_leaf(tv, leaf);
-    const double qh = q.lo.w;
+    const Box32 qb = ld_box(tv.q + leaf);
     // level by level from the root; `cur` holds the frontier (ascending node indices)
     int cur = 0, fn = 1;
     bool over = false;
@@ -391,6 +471,7 @@ __global__ void __launch_bounds__(CAND_WARPS * 32) k_lists_cand(int64_t n, int64
       const int64_t coff = lvl > 0 ? tv.level_off[lvl - 1] : 0;
       const double4* clo = lvl > 0 ? tv.lo : slo;
       const double4* chi = lvl > 0 ? tv.hi : shi;
+      const Box32* cq = lvl > 0 ? tv.q : sq;
       const int total = fn * fan;
       int nn = 0;
       for (int c0 = 0; c0 < total; c0 += 32) {
@@ -399,11 +480,7 @@ __global__ void __launch_bounds__(CAND_WARPS * 32) k_lists_cand(int64_t n, int64
         int32_t child = 0;
         if (c < total) {
           child = front[cur][c / fan] * fan + c % fan;
-          if (child < csize) {
-            const double4 blo = clo[coff + child], bhi = chi[coff + child];
-            const double reach = 2.0 * fmax(qh, blo.w);
-            hit = box_gap2(q.lo, q.hi, blo, bhi) < reach * reach * (1.0 + 1e-12);
-          }
+          hit = child < csize && child_near(records, q, qb, clo, chi, cq, coff + child);
         }
         const unsigned mk = __ballot_sync(FULL, hit);
         if (nn + __popc(mk) > CAND_SMEM) {
@@ -417,78 +494,180 @@ __global__ void __launch_bounds__(CAND_WARPS * 32) k_lists_cand(int64_t n, int64
       cur ^= 1;
       fn = nn;
     }
-    int64_t count = fn;
     if (over) {
-      // a frontier outgrew its buffer: the depth-first walk counts instead
-      count = 0;
-      if (!walk_candidates(n, tv, q, slo, shi, stack, lane,
-                           [&](int64_t, unsigned mk) { count += __popc(mk); }))
-        set_error(err, ERR_TRAVERSAL_STACK);
+      if (lane == 0) wide[atomicAdd(nwide, 1ull)] = (int32_t)leaf;
+      continue;
     }
-    const int64_t nbat = (count + 3) / 4;
-    unsigned long long cb = 0, bb = 0;
-    if (lane == 0) {
-      cb = atomicAdd(cand_at, (unsigned long long)count);
-      bb = atomicAdd(batch_at, (unsigned long long)nbat);
-    }
+    int64_t cb = 0;
+    if (lane == 0) cb = take_slices(ls, leaf, fn);
     cb = __shfl_sync(FULL, cb, 0);
-    bb = __shfl_sync(FULL, bb, 0);
-    const bool fits = (int64_t)cb + count <= cap_cands && (int64_t)bb + nbat <= cap_batches;
-    if (fits) {
-      if (!over) {
-        for (int64_t c = lane; c < count; c += 32) cands[cb + c] = front[cur][c];
-      } else {
-        int64_t c2 = 0;
-        walk_candidates(n, tv, q, slo, shi, stack, lane, [&](int64_t s0, unsigned mk) {
-          const int pos = __popc(mk & below);
-          if (((mk >> lane) & 1u) && c2 + pos < count) cands[cb + c2 + pos] = (int32_t)(s0 + lane);
-          c2 += __popc(mk);
-        });
-      }
-    }
-    if (lane == 0) {
-      leaf_cbase[leaf] = (int64_t)cb;
-      leaf_bbase[leaf] = (int64_t)bb;
-      leaf_ncand[leaf] = (int32_t)count;
-    }
+    if (cb >= 0)
+      for (int c = lane; c < fn; c += 32) cands[cb + c] = front[cur][c];
     __syncwarp();
   }
 }
 
-// Pass 2: the tests, on each leaf's candidate list.  Each batch's final hit masks go to
-// masks[(batch base + b) * 32 + lane], the rows' entry counts to counts.
+// Pass 1 for the leaves with large frontiers: a block per leaf tests WIDE_THREADS children at a
+// time, with the leaf-level frontier (up to WIDE_CAP leaves) in shared memory; its sub-leaves are
+// counted and then written in two sweeps over it.  A frontier beyond that is left to a depth-first
+// walk by one warp.
+constexpr int WIDE_THREADS = 512;
+constexpr int WIDE_CAP = 12288;
+
+__global__ void __launch_bounds__(WIDE_THREADS) k_lists_wide(
+    int64_t n, const int32_t* __restrict__ wide, const unsigned long long* __restrict__ nwide,
+    TreeView tv, const double4* __restrict__ slo, const double4* __restrict__ shi,
+    const Box32* __restrict__ sq, const double* __restrict__ box6, ListSlices ls,
+    int32_t* __restrict__ cands, int* err) {
+  extern __shared__ int32_t wide_front[];  // two frontiers of WIDE_CAP
+  __shared__ int64_t stack[STACK];
+  __shared__ int hits_s[WIDE_THREADS / 32];
+  __shared__ int64_t base_s, count_s;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  const int64_t nsub = (n + SUB - 1) / SUB;
+  const bool records = box_scale(box6) > 0.0;
+  const int64_t all = (int64_t)*nwide;
+  for (int64_t w = blockIdx.x; w < all; w += gridDim.x) {
+    const int64_t leaf = wide[w];
+    const QueryLeaf q = query_leaf(tv, leaf);
+    const Box32 qb = ld_box(tv.q + leaf);
+    int32_t* cur = wide_front;
+    int32_t* nxt = wide_front + WIDE_CAP;
+    int fn = 1;
+    bool over = false;
+    __syncthreads();
+    if (threadIdx.x == 0) cur[0] = 0;
+    __syncthreads();
+    // children of the frontier's nodes, WIDE_THREADS at a time; f(child, its rank) for the near
+    // ones, ranks ascending.  Returns their number.
+    auto sweep = [&](int lvl, auto&& f) {
+      const int fan = lvl > 0 ? FAN : LEAF / SUB;
+      const int64_t csize = lvl > 0 ? tv.level_size[lvl - 1] : nsub;
+      const int64_t coff = lvl > 0 ? tv.level_off[lvl - 1] : 0;
+      const double4* clo = lvl > 0 ? tv.lo : slo;
+      const double4* chi = lvl > 0 ? tv.hi : shi;
+      const Box32* cq = lvl > 0 ? tv.q : sq;
+      const int total = fn * fan;
+      int64_t nn = 0;
+      for (int c0 = 0; c0 < total; c0 += WIDE_THREADS) {
+        const int c = c0 + (int)threadIdx.x;
+        bool hit = false;
+        int32_t child = 0;
+        if (c < total) {
+          child = cur[c / fan] * fan + c % fan;
+          hit = child < csize && child_near(records, q, qb, clo, chi, cq, coff + child);
+        }
+        const unsigned mk = __ballot_sync(FULL, hit);
+        if (lane == 0) hits_s[warp] = __popc(mk);
+        __syncthreads();
+        int before = 0, sum = 0;
+#pragma unroll
+        for (int v = 0; v < WIDE_THREADS / 32; ++v) {
+          before += v < warp ? hits_s[v] : 0;
+          sum += hits_s[v];
+        }
+        if (hit) f(child, nn + before + __popc(mk & below));
+        nn += sum;
+        __syncthreads();
+      }
+      return nn;
+    };
+    for (int lvl = tv.nlevels - 1; lvl > 0 && !over; --lvl) {
+      const int64_t nn = sweep(lvl, [&](int32_t child, int64_t at) {
+        if (at < WIDE_CAP) nxt[at] = child;
+      });
+      over = nn > WIDE_CAP;  // block-uniform
+      fn = (int)min(nn, (int64_t)WIDE_CAP);
+      int32_t* swap = cur;
+      cur = nxt;
+      nxt = swap;
+      __syncthreads();
+    }
+    if (!over) {
+      const int64_t count = sweep(0, [](int32_t, int64_t) {});
+      if (threadIdx.x == 0) base_s = take_slices(ls, leaf, count);
+      __syncthreads();
+      const int64_t cb = base_s;
+      if (cb >= 0) sweep(0, [&](int32_t child, int64_t at) { cands[cb + at] = child; });
+    } else if (warp == 0) {
+      int64_t count = 0;
+      if (!walk_candidates(n, tv, q, slo, shi, stack, lane,
+                           [&](int64_t, unsigned mk) { count += __popc(mk); }))
+        set_error(err, ERR_TRAVERSAL_STACK);
+      if (lane == 0) {
+        base_s = take_slices(ls, leaf, count);
+        count_s = count;
+      }
+      __syncwarp();
+      const int64_t cb = base_s;
+      if (cb >= 0) {
+        int64_t c2 = 0;
+        walk_candidates(n, tv, q, slo, shi, stack, lane, [&](int64_t s0, unsigned mk) {
+          const int pos = __popc(mk & below);
+          if (((mk >> lane) & 1u) && c2 + pos < count_s) cands[cb + c2 + pos] = (int32_t)(s0 + lane);
+          c2 += __popc(mk);
+        });
+      }
+    }
+  }
+}
+
+// Two floats in one register pair: the packed operations of sm_100 (each half rounds to nearest as
+// the scalar operation does).
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  return (uint64_t)__float_as_uint(a) | ((uint64_t)__float_as_uint(b) << 32);
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
+// Pass 2: the tests, on each work item's batches of candidates.  Each batch's final hit masks go
+// to masks[(batch base + b) * 32 + lane], the item's entries per row to part_count and, added up,
+// to counts (zeroed before).  Bound by issue (71 %) and by the broadcast loads of the staged
+// candidates (LSU 69 %): 0.98 ms on the 1M torus, 3.96 on the 4M torus.  Two candidates per packed
+// instruction, the whole batch unrolled, two blocks per SM (three spill); with scalar tests and a
+// warp alone on its leaf whatever the leaf's number of batches, 1.30 and 4.0 ms.
 #ifndef TEST_BLOCKS_PER_SM
-#define TEST_BLOCKS_PER_SM 3
+#define TEST_BLOCKS_PER_SM 2
 #endif
-__global__ void __launch_bounds__(NB_THREADS, TEST_BLOCKS_PER_SM) k_lists_test(int64_t n, int64_t nwork,
-                                                           const uint64_t* __restrict__ order,
-                                                           unsigned long long* __restrict__ next,
-                                                           TreeView tv,
-                                                           const double4* __restrict__ spos,
-                                                           const int32_t* __restrict__ cands,
-                                                           const int64_t* __restrict__ leaf_cbase,
-                                                           const int64_t* __restrict__ leaf_bbase,
-                                                           const int32_t* __restrict__ leaf_ncand,
-                                                           uint32_t* __restrict__ masks,
-                                                           int64_t* __restrict__ counts,
-                                                           unsigned long long* __restrict__ rowmax,
-                                                           int* err) {
-  __shared__ float4 cand_s[NB_THREADS / 32][32];
+__global__ void __launch_bounds__(NB_THREADS, TEST_BLOCKS_PER_SM) k_lists_test(
+    int64_t n, unsigned long long* __restrict__ next, TreeView tv,
+    const double4* __restrict__ spos, const int32_t* __restrict__ cands, ListSlices ls,
+    uint32_t* __restrict__ masks, uint32_t* __restrict__ part_count,
+    int64_t* __restrict__ counts) {
+  // the staged candidates' offsets and negated thresholds, four arrays of 32 per warp
+  __shared__ __align__(16) float cand_s[NB_THREADS / 32][4][32];
   __shared__ int32_t cidx_s[NB_THREADS / 32][32];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  float4* cand = cand_s[threadIdx.x >> 5];
+  float(*cand)[32] = cand_s[threadIdx.x >> 5];
   int32_t* cidx = cidx_s[threadIdx.x >> 5];
-  unsigned longest = 0;
+  const unsigned long long nitems = ls.cursor[2];
   while (true) {
     unsigned long long t = 0;
     if (lane == 0) t = atomicAdd(next, 1ull);
     t = __shfl_sync(FULL, t, 0);
-    if (t >= (unsigned long long)nwork) break;  // warp-uniform
-    const int64_t leaf = (int64_t)(order[t] & 0xffffffffull);
+    if (t >= nitems) break;  // warp-uniform
+    const uint64_t item = ls.items[t];
+    const int64_t leaf = (int64_t)(item & 0xffffffffull), part = (int64_t)(item >> 32);
     const QueryLeaf q = query_leaf(tv, leaf);
-    const int64_t cbase = leaf_cbase[leaf], bbase = leaf_bbase[leaf];
-    const int64_t ncand = leaf_ncand[leaf];
+    const int64_t cbase = ls.cbase[leaf], bbase = ls.bbase[leaf];
+    const int64_t ncand = ls.ncand[leaf], nbat = (ncand + 3) / 4;
+    const int64_t b_end = min(nbat, (part + 1) * ls.chunk);
     const int64_t k = leaf * LEAF + lane;
     const bool valid = k < n;
     const double4 me = valid ? spos[k] : make_double4(0, 0, 0, 0);
@@ -505,7 +684,7 @@ __global__ void __launch_bounds__(NB_THREADS, TEST_BLOCKS_PER_SM) k_lists_test(i
     // non-negative floats order like their bits
     const float Dq = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(Dl)));
     int64_t m = 0;
-    for (int64_t b = 0; 4 * b < ncand; ++b) {
+    for (int64_t b = part * ls.chunk; b < b_end; ++b) {
       // stage: slot = lane, candidate sub-leaf 4 b + lane / 8, particle lane % 8 of it
       const int64_t c = 4 * b + (lane >> 3);
       const int32_t sb = c < ncand ? cands[cbase + c] : -1;
@@ -527,23 +706,42 @@ __global__ void __launch_bounds__(NB_THREADS, TEST_BLOCKS_PER_SM) k_lists_test(i
       // offsets beyond float's comfortable range (never in code units): every pair exactly
       const bool wide = !(D < 1e15f);
       const float B = wide ? 0.0f : BAND_U * D * D;
-      cc.w -= B;
-      cand[lane] = cc;
+      cand[0][lane] = cc.x;
+      cand[1][lane] = cc.y;
+      cand[2][lane] = cc.z;
+      cand[3][lane] = -(cc.w - B);
       cidx[lane] = jj;
       __syncwarp();
-      const float ri_lo = r2i_f - B, twoB = 2.0f * B;
+      const float nri = -(r2i_f - B), twoB = 2.0f * B;
       // q = r^2 - (threshold - B) of each candidate: its sign bit is a certain hit, shifted into
       // the mask (candidate 31 first, so bit tt is candidate tt); the smallest non-negative q
       // (signed floats' bits sort above every non-negative float's) tells whether any lies in
-      // the band 0 <= q < 2B
+      // the band 0 <= q < 2B.  Two candidates per packed instruction, each lane of which rounds
+      // as the scalar one.
+      const uint64_t nmx = pack2(-mx, -mx), nmy = pack2(-my, -my), nmz = pack2(-mz, -mz);
       unsigned hit = 0u, closest = 0xffffffffu;
 #pragma unroll
-      for (int tt = 31; tt >= 0; --tt) {
-        const float4 e = cand[tt];
-        const float dx = e.x - mx, dy = e.y - my, dz = e.z - mz;
-        const float q = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) - fmaxf(e.w, ri_lo);
-        hit = __funnelshift_l(__float_as_uint(q), hit, 1);
-        closest = min(closest, __float_as_uint(q));
+      for (int t4 = 7; t4 >= 0; --t4) {
+        const ulonglong2 X = reinterpret_cast<const ulonglong2*>(cand[0])[t4];
+        const ulonglong2 Y = reinterpret_cast<const ulonglong2*>(cand[1])[t4];
+        const ulonglong2 Z = reinterpret_cast<const ulonglong2*>(cand[2])[t4];
+        const float4 W = reinterpret_cast<const float4*>(cand[3])[t4];
+        uint64_t q2[2];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const uint64_t dx = add2(p ? X.y : X.x, nmx), dy = add2(p ? Y.y : Y.x, nmy),
+                         dz = add2(p ? Z.y : Z.x, nmz);
+          const uint64_t r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+          q2[p] = add2(r2, pack2(fminf(p ? W.z : W.x, nri), fminf(p ? W.w : W.y, nri)));
+        }
+        const unsigned a = (unsigned)q2[0], b = (unsigned)(q2[0] >> 32), c = (unsigned)q2[1],
+                       d = (unsigned)(q2[1] >> 32);
+        hit = __funnelshift_l(d, hit, 1);
+        hit = __funnelshift_l(c, hit, 1);
+        hit = __funnelshift_l(b, hit, 1);
+        hit = __funnelshift_l(a, hit, 1);
+        closest = __vimin3_u32(closest, a, b);
+        closest = __vimin3_u32(closest, c, d);
       }
       unsigned amb = 0u;
       if (wide) {
@@ -551,9 +749,8 @@ __global__ void __launch_bounds__(NB_THREADS, TEST_BLOCKS_PER_SM) k_lists_test(i
         amb = __ballot_sync(FULL, jj >= 0);
       } else if (__any_sync(FULL, valid && closest < __float_as_uint(twoB))) {
         for (int tt = 0; tt < 32; ++tt) {
-          const float4 e = cand[tt];
-          const float dx = e.x - mx, dy = e.y - my, dz = e.z - mz;
-          const float q = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) - fmaxf(e.w, ri_lo);
+          const float dx = cand[0][tt] - mx, dy = cand[1][tt] - my, dz = cand[2][tt] - mz;
+          const float q = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) + fminf(cand[3][tt], nri);
           amb |= q >= 0.0f && q < twoB ? 1u << tt : 0u;
         }
       }
@@ -573,118 +770,116 @@ __global__ void __launch_bounds__(NB_THREADS, TEST_BLOCKS_PER_SM) k_lists_test(i
       m += __popc(hit);
       __syncwarp();  // the next batch overwrites the staged candidates
     }
-    if (valid) counts[k] = m;
-    longest = max(longest, valid ? (unsigned)m : 0u);
+    part_count[t * 32 + lane] = (uint32_t)m;
+    if (valid) {
+      if (nbat <= ls.chunk)
+        counts[k] = m;
+      else
+        atomicAdd(reinterpret_cast<unsigned long long*>(counts + k), (unsigned long long)m);
+    }
   }
-  const unsigned mx = __reduce_max_sync(FULL, longest);
-  if (lane == 0) atomicMax(rowmax, (unsigned long long)mx);
 }
 
-// Position of the k-th set bit (k from 0) of m, for k < popc(m): halving by population count.
-__device__ __forceinline__ int nth_set_bit(uint32_t m, int k) {
-  int p = 0;
-  int c = __popc(m & 0xffffu);
-  if (k >= c) { k -= c; p += 16; m >>= 16; }
-  c = __popc(m & 0xffu);
-  if (k >= c) { k -= c; p += 8; m >>= 8; }
-  c = __popc(m & 0xfu);
-  if (k >= c) { k -= c; p += 4; m >>= 4; }
-  c = __popc(m & 0x3u);
-  if (k >= c) { k -= c; p += 2; m >>= 2; }
-  if (k >= (int)(m & 1u)) p += 1;
-  return p;
-}
+// Pass 3: masks -> CSR entries.  One warp per work item, lane r on row r.  The batches come in order, four masks of
+// a row loaded at a time; each lane appends the entries of its mask's set bits (candidates
+// ascending) to a ring of its row in shared memory, whose slots are the entries' final positions
+// modulo 64, so the ring holds aligned stretches of 32 entries.  As soon as a row's stretch is
+// full the warp writes it with one store of 128 aligned bytes; an item's first and last stretches
+// of a row are written in part.  A lane appends at most 32 entries per batch to at most 31 pending
+// ones, so it never laps its ring.
+// Bound by issue (66 % active at 19 warps per SM, about 3 warp instructions per entry): 0.78 ms on
+// the 1M torus (160M entries), 22 us on a 4,096-particle cloud.  A scan over the batches' counts and
+// a binary search per entry, a warp per leaf, took 0.88 ms and 154 us; lanes that run ahead
+// through the masks of eight batches before the rings are emptied 0.92 ms.
+constexpr int EXPAND_WARPS = 4;
+constexpr int EXPAND_RING = 64;
+constexpr int EXPAND_STRIDE = EXPAND_RING + 1;  // lanes on the same slot of 32 rows: 32 banks
 
-// Pass 3: masks -> CSR entries.  One warp per query leaf.  The leaf's masks (all 32 rows) and
-// candidate sub-leaves are staged in shared memory a chunk of batches at a time; then the warp
-// takes the rows one after the other, 32 batches at a time with lane b on batch b: the batches'
-// entry counts are scanned across the lanes, and the row's entries of those batches are written
-// 32 at a time, lane s taking entry s: its batch is found by a binary search over the scanned
-// counts, its candidate as the set bit of that rank in the batch's mask.  Every store writes up
-// to 32 consecutive entries of one row, and each row's entries come out in ascending order
-// (batches ascending, a mask's bits from the lowest slot up), contiguous from the row's offset.
-//
-// Warps per block and batches staged at a time: measured on the 4M torus (list build ms per
-// build) 10.45 with 8 warps and 32 batches, 10.86 with 4 and 32, 11.35 with 4 and 64, 11.68
-// with 2 and 64 (37.9 KB of shared memory per block for 8 x 32 and 4 x 64)
-#ifndef EXPAND_WARPS
-#define EXPAND_WARPS 8
-#endif
-#ifndef EXPAND_CHUNK
-#define EXPAND_CHUNK 32
-#endif
-constexpr int EXPAND_STRIDE = 33;  // padded mask rows: lane b reading row r of batch b is conflict-free
-
-__global__ void __launch_bounds__(EXPAND_WARPS * 32) k_lists_expand(int64_t n, int64_t nleaf,
-                                                             const int32_t* __restrict__ cands,
-                                                             const int64_t* __restrict__ leaf_cbase,
-                                                             const int64_t* __restrict__ leaf_bbase,
-                                                             const int32_t* __restrict__ leaf_ncand,
-                                                             const uint32_t* __restrict__ masks,
-                                                             const int64_t* __restrict__ off,
-                                                             int32_t* __restrict__ idx, int* err) {
-  __shared__ uint32_t msk_s[EXPAND_WARPS][EXPAND_CHUNK * EXPAND_STRIDE];
-  __shared__ int32_t sub_s[EXPAND_WARPS][EXPAND_CHUNK * 4];
+__global__ void __launch_bounds__(EXPAND_WARPS * 32) k_lists_expand(
+    int64_t n, int64_t nitems, const int32_t* __restrict__ cands, ListSlices ls,
+    const uint32_t* __restrict__ masks, const uint32_t* __restrict__ part_count,
+    const int64_t* __restrict__ off, int32_t* __restrict__ idx, int* err) {
+  __shared__ int32_t ring_s[EXPAND_WARPS][32 * EXPAND_STRIDE];
+  __shared__ int32_t ids_s[EXPAND_WARPS][4][32];  // the candidates of four batches
   const unsigned FULL = 0xffffffffu;
-  const int64_t leaf = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (leaf >= nleaf) return;  // warp-uniform
-  uint32_t* msk = msk_s[threadIdx.x >> 5];
-  int32_t* sub = sub_s[threadIdx.x >> 5];
-  const int64_t cbase = leaf_cbase[leaf], bbase = leaf_bbase[leaf];
-  const int64_t ncand = leaf_ncand[leaf], nbat = (ncand + 3) / 4;
+  if (t >= nitems) return;  // warp-uniform
+  const int64_t leaf = (int64_t)(ls.items[t] & 0xffffffffull), part = (int64_t)(ls.items[t] >> 32);
+  int32_t* rings = ring_s[threadIdx.x >> 5];
+  int32_t* ring = rings + lane * EXPAND_STRIDE;
+  int32_t(*ids)[32] = ids_s[threadIdx.x >> 5];
+  const int32_t* cand = cands + ls.cbase[leaf];
+  const uint32_t* mask = masks + ls.bbase[leaf] * 32 + lane;
+  const int64_t ncand = ls.ncand[leaf], nbat = (ncand + 3) / 4;
+  const int64_t b_beg = part * ls.chunk, b_end = min(nbat, b_beg + ls.chunk);
   const int64_t k0 = leaf * LEAF;
   const int rows = (int)(n - k0 < LEAF ? n - k0 : LEAF);
-  // lane r keeps row r's running output position and its end
-  int64_t pos = lane < rows ? off[k0 + lane] : 0;
-  const int64_t stop = lane < rows ? off[k0 + lane + 1] : 0;
-  for (int64_t c0 = 0; c0 < nbat; c0 += EXPAND_CHUNK) {
-    const int nb = (int)(nbat - c0 < EXPAND_CHUNK ? nbat - c0 : EXPAND_CHUNK);
-    __syncwarp();
-    for (int e = lane; e < nb * 32; e += 32)
-      msk[(e >> 5) * EXPAND_STRIDE + (e & 31)] = masks[(bbase + c0) * 32 + e];
-    for (int e = lane; e < nb * 4; e += 32) {
-      const int64_t c = 4 * c0 + e;
-      sub[e] = c < ncand ? cands[cbase + c] : 0;
+  // positions relative to the leaf's first one, rounded down to a stretch
+  const int64_t base = off[k0] & ~(int64_t)31;
+  if (off[k0 + rows] - base > 0x7fffffc0ll) {  // beyond 32-bit positions within one leaf
+    if (lane == 0) set_error(err, ERR_LIST_OVERFLOW);
+    return;
+  }
+  int32_t* out = idx + base;
+  int first = lane < rows ? (int)(off[k0 + lane] - base) : 0;
+  for (int64_t p = part; p > 0; --p) first += (int)part_count[(t - p) * 32 + lane];  // earlier items
+  int w = first;           // next position of the row
+  int done = first & ~31;  // first position of the stretch being filled
+  for (int64_t b0 = b_beg; b0 < b_end; b0 += 4) {
+    uint32_t mm[4];
+    int32_t id[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool in = b0 + u < b_end;
+      const int64_t c = 4 * (b0 + u) + (lane >> 3);
+      mm[u] = in ? __ldcs(mask + (b0 + u) * 32) : 0u;
+      id[u] = in && c < ncand ? cand[c] * SUB + (lane & 7) : 0;
     }
     __syncwarp();
-    for (int r = 0; r < rows; ++r) {
-      int64_t at = __shfl_sync(FULL, pos, r);  // warp-uniform from here on
-      const int64_t end = __shfl_sync(FULL, stop, r);
-      for (int b0 = 0; b0 < nb; b0 += 32) {
-        const uint32_t m = b0 + lane < nb ? msk[(b0 + lane) * EXPAND_STRIDE + r] : 0u;
-        int incl = __popc(m);
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(FULL, incl, o);
-          if (lane >= o) incl += v;
-        }
-        const int total = __shfl_sync(FULL, incl, 31);
-        for (int base = 0; base < total; base += 32) {
-          const int s = base + lane;
-          // batch of entry s: the number of batches whose inclusive count is <= s (< 32 for
-          // s < total; the probes stay within lanes 0..30)
-          int j = 0;
+    for (int u = 0; u < 4; ++u) ids[u][lane] = id[u];
+    __syncwarp();
 #pragma unroll
-          for (int step = 16; step > 0; step >>= 1)
-            if (__shfl_sync(FULL, incl, j + step - 1) <= s) j += step;
-          const uint32_t mb = __shfl_sync(FULL, m, j);
-          const int first = __shfl_sync(FULL, incl, j) - __popc(mb);
-          if (s < total) {
-            const int t = nth_set_bit(mb, s - first);
-            const int64_t w = at + s;
-            if (w < end)
-              idx[w] = sub[4 * (b0 + j) + (t >> 3)] * SUB + (t & 7);
-            else
-              set_error(err, ERR_LIST_OVERFLOW);
-          }
-        }
-        at += total;
+    for (int u = 0; u < 4; ++u) {
+      uint32_t m = mm[u];
+      while (m) {
+        ring[w & (EXPAND_RING - 1)] = ids[u][__ffs(m) - 1];
+        m &= m - 1u;
+        w += 1;
       }
-      if (lane == r) pos = at;
+      __syncwarp();
+      for (unsigned full = __ballot_sync(FULL, w - done >= 32); full; full &= full - 1) {
+        const int r = __ffs(full) - 1;
+        const int p = __shfl_sync(FULL, done, r) + lane;
+        if (p >= __shfl_sync(FULL, first, r))
+          out[p] = rings[r * EXPAND_STRIDE + (p & (EXPAND_RING - 1))];
+        if (lane == r) done += 32;
+      }
+      __syncwarp();
     }
   }
-  if (lane < rows && pos != stop) set_error(err, ERR_LIST_OVERFLOW);
+  // the last stretches
+  for (unsigned some = __ballot_sync(FULL, w > done); some; some &= some - 1) {
+    const int r = __ffs(some) - 1;
+    const int p = __shfl_sync(FULL, done, r) + lane;
+    const bool mine = p >= __shfl_sync(FULL, first, r);
+    if (p < __shfl_sync(FULL, w, r) && mine)
+      out[p] = rings[r * EXPAND_STRIDE + (p & (EXPAND_RING - 1))];
+  }
+  if (b_end == nbat && lane < rows && w != (int)(off[k0 + lane + 1] - base))
+    set_error(err, ERR_LIST_OVERFLOW);
+}
+
+// The longest row.
+__global__ void __launch_bounds__(NB_THREADS) k_row_max(int64_t n, const int64_t* __restrict__ counts,
+                                                        unsigned long long* __restrict__ rowmax) {
+  unsigned m = 0;
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n;
+       k += (int64_t)gridDim.x * blockDim.x)
+    m = max(m, (unsigned)counts[k]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(rowmax, (unsigned long long)m);
 }
 
 // Order key of each query leaf: its cost class (the binary exponent of the linear size of the
@@ -845,7 +1040,10 @@ static int list_kernel_slots(Engine& E) {
   NB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_lists_test, NB_THREADS, 0));
   // resident warps of each pass over the whole device
   E.list_slots = (int64_t)sms * std::max(1, b1) * (NB_THREADS / 32);
+  E.wide_slots = sms;
   E.cand_slots = (int64_t)sms * std::max(1, b0) * CAND_WARPS;
+  NB_CUDA(cudaFuncSetAttribute(k_lists_wide, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               2 * WIDE_CAP * (int)sizeof(int32_t)));
   return 0;
 }
 int build_lists(Engine& E, int64_t n, const double* pos, const double* hs, cudaStream_t st) {
@@ -888,16 +1086,21 @@ int build_lists(Engine& E, int64_t n, const double* pos, const double* hs, cudaS
   tv.nlevels = nl;
   if (tv.level_size[nl - 1] != 1) return set_host_error(E, "tree deeper than MAX_LEVELS");
   NB_TRY(E.ensure_nodes(offs));
-  count_launch(), k_leaf_boxes<<<grid_for(nleaf), NB_THREADS, 0, st>>>(n, nleaf, L.spos, E.node_lo, E.node_hi);
+  Box32* node_q = static_cast<Box32*>(E.node_q);
+  count_launch(), k_leaf_boxes<<<grid_for(nleaf), NB_THREADS, 0, st>>>(
+      n, nleaf, L.spos, E.bbox, E.node_lo, E.node_hi, node_q);
   for (int l = 1; l < nl; ++l)
     count_launch(), k_level_up<<<grid_for(tv.level_size[l]), NB_THREADS, 0, st>>>(
         tv.level_size[l - 1], tv.level_size[l], E.node_lo + tv.level_off[l - 1],
-        E.node_hi + tv.level_off[l - 1], E.node_lo + tv.level_off[l], E.node_hi + tv.level_off[l]);
+        E.node_hi + tv.level_off[l - 1], E.bbox, E.node_lo + tv.level_off[l],
+        E.node_hi + tv.level_off[l], node_q + tv.level_off[l]);
   tv.lo = E.node_lo;
   tv.hi = E.node_hi;
+  tv.q = node_q;
   int64_t nsub = (n + SUB - 1) / SUB;
   NB_TRY(E.ensure_sub(nsub));
-  count_launch(), k_sub_boxes<<<grid_for(nsub), NB_THREADS, 0, st>>>(n, nsub, L.spos, E.sub_lo, E.sub_hi);
+  count_launch(), k_sub_boxes<<<grid_for(nsub), NB_THREADS, 0, st>>>(
+      n, nsub, L.spos, E.bbox, E.sub_lo, E.sub_hi, static_cast<Box32*>(E.sub_q));
   // query leaves by cost class, heaviest first, each class in curve order
   uint64_t* cost = E.keys_a;
   uint64_t* order = E.keys_b;
@@ -908,32 +1111,54 @@ int build_lists(Engine& E, int64_t n, const double* pos, const double* hs, cudaS
   tmp = E.cub_bytes;
   NB_CUDA(cub::DeviceRadixSort::SortKeys(E.cub_tmp, tmp, cost, order, (int)nleaf, 0, 40, st));
   NB_TRY(list_kernel_slots(E));
-  // persistent passes: at most one warp per query leaf, at most the resident warps
-  const unsigned grid = (unsigned)std::max<int64_t>(
-      1, std::min<int64_t>(nleaf, E.list_slots) / (NB_THREADS / 32));
   const unsigned cand_grid = (unsigned)std::max<int64_t>(
       1, std::min<int64_t>(nleaf, E.cand_slots) / CAND_WARPS);
   // candidate lists of the query leaves, each in its own slice of the buffers (sized from the
   // last build's totals; a pass that outgrows them is run again with buffers of its size)
   NB_TRY(E.ensure_leaves(nleaf));
-  NB_TRY(E.ensure_tiles(E.last_cands > 0 ? E.last_cands + E.last_cands / 4 : nleaf * 512,
-                        E.last_batches > 0 ? E.last_batches + E.last_batches / 4 : nleaf * 128));
+  // batches per work item: 64, less where the leaves are too few to fill the GPU with a warp each
+  ListSlices ls{};
+  ls.chunk = (int)std::max<int64_t>(4, std::min<int64_t>(64, 64 * nleaf / E.list_slots));
+  ls.cbase = E.leaf_cbase;
+  ls.bbase = E.leaf_bbase;
+  ls.ibase = E.leaf_ibase;
+  ls.ncand = E.leaf_ncand;
+  ls.cursor = E.d_rowmax + 4;
+  int64_t want_cands = E.last_cands > 0 ? E.last_cands + E.last_cands / 4 : nleaf * 512;
+  int64_t want_batches = E.last_batches > 0 ? E.last_batches + E.last_batches / 4 : nleaf * 128;
+  int64_t nitems = 0;
   for (int attempt = 0;; ++attempt) {
-    NB_CUDA(cudaMemsetAsync(E.d_rowmax, 0, 8 * sizeof(unsigned long long), st));
+    NB_TRY(E.ensure_tiles(want_cands, want_batches, want_batches / ls.chunk + nleaf));
+    ls.items = E.items;
+    ls.cap_cands = E.cap_cands;
+    ls.cap_batches = E.cap_masks / 32;
+    ls.cap_items = E.cap_items;
+    NB_CUDA(cudaMemsetAsync(E.d_rowmax, 0, 16 * sizeof(unsigned long long), st));
     count_launch(), k_lists_cand<<<cand_grid, CAND_WARPS * 32, 0, st>>>(
-        n, nleaf, order, E.d_rowmax + 2, tv, E.sub_lo, E.sub_hi, E.d_rowmax + 4, E.d_rowmax + 5,
-        E.cap_cands, E.cap_masks / 32, E.cands, E.leaf_cbase, E.leaf_bbase, E.leaf_ncand, E.d_err);
-    NB_CUDA(cudaMemcpyAsync(E.h_build, E.d_rowmax + 4, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        n, nleaf, order, E.d_rowmax + 2, tv, E.sub_lo, E.sub_hi,
+        static_cast<const Box32*>(E.sub_q), E.bbox, ls, E.cands, E.vals_a, E.d_rowmax + 8);
+    count_launch(), k_lists_wide<<<(unsigned)std::min<int64_t>(nleaf, E.wide_slots), WIDE_THREADS,
+                                   2 * WIDE_CAP * sizeof(int32_t), st>>>(
+        n, E.vals_a, E.d_rowmax + 8, tv, E.sub_lo, E.sub_hi, static_cast<const Box32*>(E.sub_q),
+        E.bbox, ls, E.cands, E.d_err);
+    NB_CUDA(cudaMemcpyAsync(E.h_build, E.d_rowmax + 4, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     NB_TRY(pending_check(E, st));
     const int64_t ncand = E.h_build[0], nbatch = E.h_build[1];
+    nitems = E.h_build[2];
     E.last_cands = ncand;
     E.last_batches = nbatch;
-    if (ncand <= E.cap_cands && nbatch <= E.cap_masks / 32) break;
+    if (ncand <= ls.cap_cands && nbatch <= ls.cap_batches && nitems <= ls.cap_items) break;
     if (attempt > 0) return set_host_error(E, "list build: candidate buffers outgrown twice");
-    NB_TRY(E.ensure_tiles(ncand + ncand / 4, nbatch + nbatch / 4));
+    want_cands = ncand + ncand / 4;
+    want_batches = nbatch + nbatch / 4;
   }
   // the tests, once: hit masks per batch and lane, entries per row
-  count_launch(), k_lists_test<<<grid, NB_THREADS, 0, st>>>(n, nleaf, order, E.d_rowmax + 3, tv, L.spos, E.cands, E.leaf_cbase, E.leaf_bbase, E.leaf_ncand, E.masks, E.counts, E.d_rowmax, E.d_err);
+  NB_CUDA(cudaMemsetAsync(E.counts, 0, sizeof(int64_t) * n, st));
+  const unsigned grid = (unsigned)std::max<int64_t>(
+      1, std::min<int64_t>(nitems, E.list_slots) / (NB_THREADS / 32));
+  count_launch(), k_lists_test<<<grid, NB_THREADS, 0, st>>>(
+      n, E.d_rowmax + 3, tv, L.spos, E.cands, ls, E.masks, E.part_count, E.counts);
+  count_launch(), k_row_max<<<std::min(grid_for(n), 592u), NB_THREADS, 0, st>>>(n, E.counts, E.d_rowmax);
   NB_CUDA(cudaMemsetAsync(L.off, 0, sizeof(int64_t), st));
   tmp = E.cub_bytes;
   NB_CUDA(cub::DeviceScan::InclusiveSum(E.cub_tmp, tmp, E.counts, L.off + 1, (int)n, st));
@@ -942,9 +1167,10 @@ int build_lists(Engine& E, int64_t n, const double* pos, const double* hs, cudaS
   NB_TRY(pending_check(E, st));
   const int64_t total = E.h_build[0], longest = E.h_build[1];
   NB_TRY(E.ensure_list_capacity(total));
-  // masks -> entries at the rows' offsets
-  count_launch(), k_lists_expand<<<grid_for(nleaf * 32, EXPAND_WARPS * 32), EXPAND_WARPS * 32, 0, st>>>(
-      n, nleaf, E.cands, E.leaf_cbase, E.leaf_bbase, E.leaf_ncand, E.masks, L.off, L.idx, E.d_err);
+  // masks -> entries at the rows' offsets (the store of a row's stretch stays inside the row: the
+  // counts are the masks' own)
+  count_launch(), k_lists_expand<<<grid_for(nitems * 32, EXPAND_WARPS * 32), EXPAND_WARPS * 32, 0, st>>>(
+      n, nitems, E.cands, ls, E.masks, E.part_count, L.off, L.idx, E.d_err);
   E.prof.end(PROF_LISTS, st, (double)n, (double)total);
   L.n = n;
   L.total = total;
@@ -971,7 +1197,7 @@ int export_lists(Engine& E, int64_t* off_out, int64_t* idx_out, cudaStream_t st)
   int64_t n = L.n;
   if (n == 0) return 0;
   const bool long_rows = L.longest > EXPORT_MAX;
-  unsigned long long* nseg = E.d_rowmax + 7;
+  unsigned long long* nseg = E.d_rowmax + 9;
   int64_t* seg_beg = E.counts;  // scratch of at least n entries each, free between builds
   int64_t* seg_end = reinterpret_cast<int64_t*>(E.keys_b);
   if (long_rows) {
