@@ -1,5 +1,7 @@
 // FP32 instantiations of the pair passes (fused multiply-add allowed: the FP32 path is judged
 // against the FP64 oracle by its stated tolerance, not bit for bit).
+#include <type_traits>
+
 #include "sph_impl.cuh"
 
 namespace nbk {
@@ -12,9 +14,15 @@ void launch_density32(int64_t nrows, const int64_t* rows, const float4* pos, con
                       int64_t* work, cudaStream_t st) {
   if (nrows <= 0) return;
   Pos32 geo{pos, 0.f, box6};
-  count_launch(), k_density<float, Pos32, I><<<grid_for((nrows + 3) / 4 * 32, DENSITY_THREADS), DENSITY_THREADS, 0, st>>>(
-      nrows, rows, geo, mass, h_start, h_search, off, idx, prm, out_map, h_out, rho, omega, iters,
-      flags, work);
+  auto run = [&](auto kid) {
+    count_launch(), k_density32<decltype(kid)::value, I><<<grid_for(nrows * 8, DENSITY_THREADS), DENSITY_THREADS, 0, st>>>(
+        nrows, rows, geo, mass, h_start, h_search, off, idx, prm, out_map, h_out, rho, omega, iters,
+        flags, work);
+  };
+  if (prm.kid == 0)
+    run(std::integral_constant<int, 0>{});
+  else
+    run(std::integral_constant<int, 1>{});
 }
 
 template <typename I>

@@ -53,7 +53,16 @@ struct Pos32 {
     }
   }
   __device__ __forceinline__ Own own(int64_t i) const { return Own{p[2 * i], p[2 * i + 1]}; }
-  __device__ __forceinline__ float mass(int64_t j) const { return p[2 * j].w; }
+  // the difference and particle j's mass, in one load
+  __device__ __forceinline__ void diff_m(const Own& o, int64_t j, float& dx, float& dy, float& dz,
+                                         float& m) const {
+    float4 b, cb;
+    ld_rec(p + 2 * j, b, cb);
+    dx = fmaf(cb.x - o.c.x, cell, b.x - o.a.x);
+    dy = fmaf(cb.y - o.c.y, cell, b.y - o.a.y);
+    dz = fmaf(cb.z - o.c.z, cell, b.z - o.a.z);
+    m = b.w;
+  }
   __device__ __forceinline__ void diff(const Own& o, int64_t j, float& dx, float& dy,
                                        float& dz) const {
     const float4 b = p[2 * j], cb = p[2 * j + 1];
@@ -135,166 +144,170 @@ __device__ __forceinline__ double group_total(const Acc<float>& a) {
   return (double)s + (double)k;
 }
 
-template <typename R>
-struct DensityEntry;
-#ifndef DENSITY_CAP
-#define DENSITY_CAP 128
-#endif
-template <>
-struct DensityEntry<float> {
-  using T = float2;
-  // entries inside r_in a row keeps in shared memory: 16 rows x 128 x 8 B = 16 KiB per block, so
-  // 8 resident blocks (the register limit) leave most of the SM's L1 to the gathered records
-  static constexpr int CAP = DENSITY_CAP;
-  static constexpr int BLOCKS = 8;
-};
 constexpr int DENSITY_THREADS = 128;  // 16 rows per block
-// rounds of 8 entries the list walk loads at once: 4 measured 3.55 ms per density launch on the
-// 4M torus against 3.88 with 2 and 3.75 with 8
-#ifndef DENSITY_UNROLL
-#define DENSITY_UNROLL 4
-#endif
+// FP32: entries inside r_in a row keeps in shared memory: 16 rows x 128 x 8 B = 16 KiB per block, so
+// 8 resident blocks (the register limit) leave most of the SM's L1 to the gathered records
+constexpr int DENSITY_CAP = 128;
+// rounds of 8 entries loaded at once by the first walk and by a walk within a sum, and resident
+// blocks.  Measured on the 4M torus (launches of the first evaluation, from a guess of h that is
+// far off, and of a step's 2.7M rows): 4, 2, 9: 35.8 and 4.05 ms; 4, 2, 8: 38.5 and 4.10; 4, 4, 8:
+// 34.7 and 4.59; 3, 3, 8: 40.2 and 4.31; 2, 2, 10: 35.1 and 4.39
+constexpr int DENSITY_UNROLL = 4, DENSITY_WALK = 2, DENSITY_BLOCKS = 9;
 
-// Eight lanes per row, four rows per warp.  The lanes of a row split its list (entry e to lane
-// e mod 8, coalesced index loads) and store the distance and mass of every entry inside r_in =
-// 2.1 h_start (the Newton iterates stay near the start h) in shared memory, in list order; each
-// Newton iteration then sums the kernel terms over that cache and reduces across the eight lanes,
-// so the lanes of a row take the same Newton steps.  A sum at an h whose support reaches past
-// r_in adds the entries beyond it from the list (the same distances, recomputed); rows with more
-// entries inside r_in than the cache holds re-walk their list in every sum.
-template <typename R, typename PosT, typename I>
-__global__ void __launch_bounds__(DENSITY_THREADS, DensityEntry<R>::BLOCKS)
-    k_density(int64_t nrows, const int64_t* __restrict__ rows, PosT geo_in,
+// FP32 form.  Eight lanes per row, four rows per warp.  The lanes of a row split its list (entry e to
+// lane e mod 8, coalesced index loads) and store the squared distance and mass of every entry
+// inside r_in = 2.1 h_start (the Newton iterates stay near the start h) in shared memory, in list
+// order; each Newton iteration then sums the kernel terms over that cache and reduces across the
+// eight lanes, so the lanes of a row take the same Newton steps.  The first sum turns the squares
+// into distances.  A sum at an h whose support reaches past r_in adds the entries beyond it from
+// the list (the same distances, recomputed); rows with more entries inside r_in than the cache
+// holds re-walk their list in every sum.  (The compensated float sums depend on the order of
+// their terms in the eighth digit: which lane adds which entry when is part of the result, and so
+// are the fused operations of a term, written out below where a rearrangement changed them.)
+// Bound by issue (65 % active, about 900 warp instructions per row) and by the gathers (LSU 68 %).
+// With a square root per list entry, three loads per record, divergent kernel branches and
+// conflicting cache rows the two launches above took 51.5 and 5.49 ms.
+template <int KID, typename I>
+__global__ void __launch_bounds__(DENSITY_THREADS, DENSITY_BLOCKS)
+    k_density32(int64_t nrows, const int64_t* __restrict__ rows, Pos32 geo,
               const double* __restrict__ mass, const double* __restrict__ h_start,
               const double* __restrict__ h_search, const int64_t* __restrict__ off,
               const I* __restrict__ idx, DensityParams prm, const int32_t* __restrict__ out_map,
               double* __restrict__ h_out, double* __restrict__ rho, double* __restrict__ omega,
               int64_t* __restrict__ iters, int64_t* __restrict__ flags, int64_t* __restrict__ work) {
-  PosT geo = geo_in;
   geo.ready();
-  using E2 = typename DensityEntry<R>::T;
-  constexpr int CAP = DensityEntry<R>::CAP;
-  __shared__ E2 cache_s[DENSITY_THREADS / 8][CAP];
+  // (rows half the banks apart: the four rows of a warp read in two wavefronts)
+  __shared__ float2 cache_s[DENSITY_THREADS / 8][DENSITY_CAP + 8];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, gl = lane & 7, g = lane >> 3;
   const int64_t q = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * 4 + g;
   const bool live = q < nrows;
   if (!__any_sync(FULL, live)) return;  // warp-uniform
-  E2* cache = cache_s[threadIdx.x >> 3];
-  int64_t i = 0, o = 0, e0 = 0, e1 = 0;
-  double m_i = 1.0, hs = 1.0;
+  float2* cache = cache_s[threadIdx.x >> 3];
+  int64_t i = 0, e0 = 0;
+  unsigned len = 0;
+  double m_i = 1.0, hs = 1.0, h = 1.0;
   if (live) {
     i = rows ? rows[q] : q;
-    o = out_map ? (int64_t)out_map[i] : q;
     m_i = mass[i];
     hs = fmin(h_search[i], prm.h_max);
+    h = fmin(h_start[i], hs);
     e0 = off[i];
-    e1 = off[i + 1];
+    len = (unsigned)(off[i + 1] - e0);
   }
-  const typename PosT::Own me_rec = geo.own(i);  // the row's own record, loaded once
-  auto mass_of = [&](int64_t j) -> R { return (R)geo.mass(j); };
-  const double r_max = 2.0 * hs;
-  const R r2max = (R)(r_max * r_max);
-  const int kid = prm.kid;
-  const R cn = (R)prm.cnorm;
-  // the Newton iterates stay near the start h0 (the previous step's h): entries inside
-  // r_in = 2.1 h0 are cached, and a sum at h adds the others only when r_in / h < 2 (else every
-  // one of them has q >= 2, a zero term)
-  const double h_first = live ? fmin(h_start[i], hs) : 1.0;
-  const R r_in = (R)(2.1 * h_first);
-  // distances and masses of the entries inside r_max (sim/sph.py:231-248), in list order
-  const unsigned len = (unsigned)(e1 - e0);
+  const I* list = idx + e0;
+  const Pos32::Own me_rec = geo.own(i);  // the row's own record, loaded once
+  const float r2max = (float)(2.0 * hs * (2.0 * hs));
+  const float cn = (float)prm.cnorm;
+  // entries inside r_in = 2.1 h are cached, and a sum at h adds the others only when r_in / h < 2
+  // (else every one of them has q >= 2, a zero term).  sqrt(d2) < r_in holds for the floats d2
+  // below the square of the midpoint of r_in and the float before it (exact in double)
+  const float r_in = (float)(2.1 * h);
+  const double mid = 0.5 * ((double)r_in + (double)__uint_as_float(__float_as_uint(r_in) - 1u));
+  const float d2_in = r_in > 0.0f ? fminf(__double2float_ru(mid * mid), r2max) : 0.0f;
   const unsigned maxlen = __reduce_max_sync(FULL, len);
   int cnt = 0;
-  // DENSITY_UNROLL rounds of 8 entries per pass: their index, position and mass loads are issued
-  // together (the walk is bound by the latency of those dependent gathers), then the rounds are
-  // appended to the cache one after the other, so the cache holds the entries in list order
+  // DENSITY_UNROLL rounds of 8 entries per pass: their index and record loads are issued together
+  // (the walk is bound by the latency of those dependent gathers), then the rounds are appended
+  // to the cache one after the other
   constexpr int U = DENSITY_UNROLL;
   for (unsigned b = 0; b < maxlen; b += 8 * U) {
-    int64_t jj[U];
-    bool inr[U];
-    R rr[U], mm[U];
+    int jj[U];
+    float d2[U], mm[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const unsigned e = b + 8 * u + gl;
-      jj[u] = e < len ? (int64_t)ld_stream(idx + e0 + e) : -1;
+      jj[u] = e < len ? (int)ld_stream(list + e) : -1;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      inr[u] = false;
-      rr[u] = R(0);
-      mm[u] = R(0);
+      d2[u] = INFINITY;
+      mm[u] = 0.0f;
       if (jj[u] >= 0) {
-        R dx, dy, dz;
-        geo.diff(me_rec, jj[u], dx, dy, dz);
-        R d2 = sqdist(dx, dy, dz);
-        if (d2 < r2max) {
-          inr[u] = true;
-          rr[u] = sqrt(d2);
-        }
+        float dx, dy, dz;
+        geo.diff_m(me_rec, jj[u], dx, dy, dz, mm[u]);
+        d2[u] = sqdist(dx, dy, dz);
       }
     }
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (inr[u]) mm[u] = mass_of(jj[u]);
-#pragma unroll
     for (int u = 0; u < U; ++u) {
-      const bool inner = inr[u] && rr[u] < r_in;
+      const bool inner = d2[u] < d2_in;
       const unsigned seg = (__ballot_sync(FULL, inner) >> (8 * g)) & 0xffu;
       const int pos = cnt + __popc(seg & ((1u << gl) - 1u));
-      if (inner && pos < CAP) {  // overflow: the walk below instead
-        E2 v;
-        v.x = rr[u];
-        v.y = mm[u];
-        cache[pos] = v;
-      }
+      if (inner && pos < DENSITY_CAP)  // overflow: the walk below instead
+        cache[pos] = make_float2(d2[u], mm[u]);
       cnt += __popc(seg);
     }
   }
   __syncwarp();
-  const bool cached = cnt <= CAP;
-  int64_t evals = 0;
+  const bool cached = cnt <= DENSITY_CAP;
+  bool squared = true;
+  int evals = 0;
   // kernel sums at h of the rows whose `active` is set; every lane takes part in the reductions
-  auto sums = [&](R h, bool active, double& rs_out, double& dws_out) {
-    Acc<R> rs, dws;
+  auto sums = [&](float h, bool active, double& rs_out, double& dws_out) {
+    Acc<float> rs, dws;
     if (active) {
-      R inv_h = R(1) / h;
-      R ih2 = inv_h * inv_h;
-      R ih3 = ih2 * inv_h;
-      R ih4 = ih2 * ih2;
-      auto term = [&](R rj, R mj) {
-        R qq = rj * inv_h;
-        if (qq < R(2)) {
+      float inv_h = 1.0f / h;
+      float ih2 = inv_h * inv_h;
+      float ih3 = ih2 * inv_h;
+      float ih4 = ih2 * ih2;
+      auto term = [&](float rj, float mj) {
+        float qq = rj * inv_h;
+        if (qq < 2.0f) {
           evals += 1;
-          R fq = kernel_f<R>(qq, kid);
+          float fq, df;
+          if (KID == 0) {
+            // both pieces of the spline, then the one that holds: no divergent branch
+            const float t = 2.0f - qq;
+            const float f1 = 1.0f - 1.5f * qq * qq + 0.75f * qq * qq * qq;
+            const float d1 = fmaf(2.25f * qq, qq, __fmul_rn(-3.0f, qq));
+            const float f2 = 0.25f * t * t * t, d2 = -0.75f * t * t;
+            fq = qq < 1.0f ? f1 : f2;
+            df = qq < 1.0f ? d1 : d2;
+          } else {
+            fq = kernel_f<float>(qq, 1);
+            df = kernel_df<float>(qq, 1);
+          }
           rs.add(mj * cn * ih3 * fq);
-          dws.add(mj * (-cn * ih4 * (R(3) * fq + qq * kernel_df<R>(qq, kid))));
+          dws.add(mj * (-cn * ih4 * fmaf(3.0f, fq, __fmul_rn(qq, df))));
         }
       };
+      const bool beyond = cached && !(r_in * inv_h >= 2.0f);
       if (cached) {
         for (int t = gl; t < cnt; t += 8) {
-          E2 v = cache[t];
+          float2 v = cache[t];
+          if (squared) {
+            v.x = sqrtf(v.x);
+            cache[t].x = v.x;  // only this lane reads it
+          }
           term(v.x, v.y);
         }
-        if (!(r_in * inv_h >= R(2)))
-          for (int64_t e = e0 + gl; e < e1; e += 8) {  // the entries beyond r_in
-            int64_t j = (int64_t)idx[e];
-            R dx, dy, dz;
-            geo.diff(me_rec, j, dx, dy, dz);
-            R d2 = sqdist(dx, dy, dz);
-            if (!(d2 < r2max)) continue;
-            const R rj = sqrt(d2);
-            if (rj < r_in) continue;
-            term(rj, mass_of(j));
+        squared = false;
+      }
+      if (!cached || beyond) {
+        // the list, or its entries beyond r_in, DENSITY_WALK rounds' loads in flight at once; an
+        // entry well outside 2 h (no term) costs no square root
+        constexpr int W = DENSITY_WALK;
+        const float d2_far = (2.001f * h) * (2.001f * h);
+        for (unsigned b = gl; b < len; b += 8 * W) {
+          int jj[W];
+          float d2[W], mm[W];
+#pragma unroll
+          for (int u = 0; u < W; ++u) jj[u] = b + 8 * u < len ? (int)list[b + 8 * u] : -1;
+#pragma unroll
+          for (int u = 0; u < W; ++u) {
+            d2[u] = INFINITY;
+            mm[u] = 0.0f;
+            if (jj[u] >= 0) {
+              float dx, dy, dz;
+              geo.diff_m(me_rec, jj[u], dx, dy, dz, mm[u]);
+              d2[u] = sqdist(dx, dy, dz);
+            }
           }
-      } else {
-        for (int64_t e = e0 + gl; e < e1; e += 8) {
-          int64_t j = (int64_t)idx[e];
-          R dx, dy, dz;
-          geo.diff(me_rec, j, dx, dy, dz);
-          R d2 = sqdist(dx, dy, dz);
-          if (!(d2 < r2max)) continue;
-          term(sqrt(d2), mass_of(j));
+#pragma unroll
+          for (int u = 0; u < W; ++u)
+            if (d2[u] < r2max && !(d2[u] > d2_far) && !(beyond && d2[u] < d2_in))
+              term(sqrtf(d2[u]), mm[u]);
         }
       }
     }
@@ -302,14 +315,13 @@ __global__ void __launch_bounds__(DENSITY_THREADS, DensityEntry<R>::BLOCKS)
     dws_out = group_total(dws);
   };
   double lo = 0.0, hi = hs;
-  double h = live ? fmin(h_start[i], hi) : 1.0;
-  double h0 = h;
+  const double h0 = h;
   int flag = 3, it = 0;
   bool done = !live;
   const double eta = prm.eta, e3 = eta * eta * eta;
   while (__any_sync(FULL, !done)) {
     double rs, dws;
-    sums((R)h, !done, rs, dws);
+    sums((float)h, !done, rs, dws);
     if (!done) {
       it += 1;
       double t = eta / h;
@@ -334,7 +346,7 @@ __global__ void __launch_bounds__(DENSITY_THREADS, DensityEntry<R>::BLOCKS)
   const bool cap_test = live && h >= hs * (1 - 1e-3);
   if (__any_sync(FULL, cap_test)) {
     double rs_lim, dummy;
-    sums((R)hs, cap_test, rs_lim, dummy);
+    sums((float)hs, cap_test, rs_lim, dummy);
     double t = eta / hs;
     if (cap_test && rs_lim - m_i * (t * t * t) < 0) {
       h = hs;
@@ -342,10 +354,13 @@ __global__ void __launch_bounds__(DENSITY_THREADS, DensityEntry<R>::BLOCKS)
     }
   }
   double rs, dws;
-  sums((R)h, live, rs, dws);
+  sums((float)h, live, rs, dws);
+  if (work) {
 #pragma unroll
-  for (int of = 4; of > 0; of >>= 1) evals += __shfl_xor_sync(FULL, evals, of);
+    for (int of = 4; of > 0; of >>= 1) evals += __shfl_xor_sync(FULL, evals, of);
+  }
   if (live && gl == 0) {
+    const int64_t o = out_map ? (int64_t)out_map[i] : q;
     h_out[o] = h;
     rho[o] = rs;
     omega[o] = flag == 1 ? 1.0 : 1.0 + h / (3.0 * rs) * dws;
