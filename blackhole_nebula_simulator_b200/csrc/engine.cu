@@ -518,9 +518,9 @@ __global__ void k_pack_density32(int64_t n, const int32_t* __restrict__ perm,
 }
 
 // The FP32 force pass's sorted inputs in one pass (the switch and the reconstruction off): the
-// position records (offset, m) (cell, h), the records (v, m), (h, rho, omega, P), (u, c_s, alpha)
-// and, when pk0 is given, the double (x, h) of the exact band test; with `only`, the records of
-// its particles alone.
+// position records (offset, m) (cell, h), the records (v, m) (1/h, rho, 1/(Omega rho^2), P) and (u,
+// c_s, alpha, Omega) and, when pk0 is given, the double (x, h) of the exact band test; with `only`,
+// the records of its particles alone.
 __global__ void k_pack_force32(int64_t n, const int32_t* __restrict__ perm,
                                const double* __restrict__ x, const double* __restrict__ m,
                                const double* __restrict__ h, const double* __restrict__ box6,
@@ -528,19 +528,18 @@ __global__ void k_pack_force32(int64_t n, const int32_t* __restrict__ perm,
                                const double* __restrict__ omega, const double* __restrict__ P,
                                const double* __restrict__ u, const double* __restrict__ cs,
                                const double* __restrict__ alpha, const uint8_t* __restrict__ only,
-                               float4* __restrict__ pk32, float4* __restrict__ pf1,
-                               float4* __restrict__ pf2, float4* __restrict__ pf3,
-                               double4* __restrict__ pk0) {
+                               float4* __restrict__ pk32, float4* __restrict__ pv,
+                               float4* __restrict__ aux, double4* __restrict__ pk0) {
   int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int64_t i = perm[k];
   if (only && !only[i]) return;  // a record the pass does not read
   const double hi = h[i];
-  const float mi = (float)m[i];
-  pos32_record(x, i, box6, mi, (float)hi, pk32 + 2 * k);
-  pf1[k] = make_float4((float)vel[3 * i], (float)vel[3 * i + 1], (float)vel[3 * i + 2], mi);
-  pf2[k] = make_float4((float)hi, (float)rho[i], (float)omega[i], (float)P[i]);
-  pf3[k] = make_float4((float)u[i], (float)cs[i], alpha ? (float)alpha[i] : 0.f, 0.f);
+  const float mi = (float)m[i], hf = (float)hi, rf = (float)rho[i], of = (float)omega[i];
+  pos32_record(x, i, box6, mi, hf, pk32 + 2 * k);
+  pv[2 * k] = make_float4((float)vel[3 * i], (float)vel[3 * i + 1], (float)vel[3 * i + 2], mi);
+  pv[2 * k + 1] = make_float4(1.0f / hf, rf, 1.0f / (of * rf * rf), (float)P[i]);
+  aux[k] = make_float4((float)u[i], (float)cs[i], alpha ? (float)alpha[i] : 0.f, of);
   if (pk0) pk0[k] = make_double4(x[3 * i], x[3 * i + 1], x[3 * i + 2], hi);
 }
 
@@ -723,7 +722,8 @@ int Workspace::ensure(Engine& E, int64_t n) {
   double4** d4[] = {&pk0, &pk1, &pk2, &pk3};
   for (double4** p : d4) NB_CUDA(cudaMalloc((void**)p, sizeof(double4) * c));
   NB_CUDA(cudaMalloc((void**)&pk32, sizeof(float4) * 2 * c));
-  float4** f4s[] = {&pf1, &pf2, &pf3};
+  NB_CUDA(cudaMalloc((void**)&pf1, sizeof(float4) * 2 * c));
+  float4** f4s[] = {&pf2, &pf3};
   for (float4** p : f4s) NB_CUDA(cudaMalloc((void**)p, sizeof(float4) * c));
   int64_t** i8[] = {&rows, &rows_s, &rows2, &iters, &flags, &need, &i_tmp, &pairs, &i_lvl, &i_tmp2};
   for (int64_t** p : i8) NB_CUDA(cudaMalloc((void**)p, sizeof(int64_t) * (c + 1)));
@@ -1173,9 +1173,9 @@ int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, in
   NB_TRY(rows_sorted(E, n, nrows, rows, &ns, st));
   const bool sw_on = prm->viscosity && prm->visc_switch && sk.switch_on;
   const bool recon = prm->viscosity && prm->recon;
-  // FP32 without the switch and the reconstruction: every sorted input in one pass below, for
+  // FP32 without the reconstruction: every sorted input in one pass below (after the switch), for
   // the touched particles only when they hold every list entry of the rows and are few
-  const bool fused_pack = prm->precision == 1 && !sw_on && !recon;
+  const bool fused_pack = prm->precision == 1 && !recon;
   const bool sparse_pack = fused_pack && touched && sk.touched_covers_lists && nrows * 8 < n;
   if (prm->precision == 1 && !fused_pack) {
     count_launch(), k_pack_sorted_f4<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, vel, s->mass, nullptr, nullptr, 1, W.pf1);
@@ -1272,7 +1272,7 @@ int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, in
     if (fused_pack)
       count_launch(), k_pack_force32<<<grid_for(n), NB_THREADS, 0, st>>>(
           n, L.perm, s->x, s->mass, s->h, E.bbox, vel, s->rho, s->omega, W.d_P, u, W.d_cs, s->alpha,
-          sparse_pack ? touched : nullptr, W.pk32, W.pf1, W.pf2, W.pf3, want_tight ? W.pk0 : nullptr);
+          sparse_pack ? touched : nullptr, W.pk32, W.pf1, W.pf3, want_tight ? W.pk0 : nullptr);
     else
       count_launch(), k_pack_sorted32<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, s->x, s->mass, s->h, E.bbox, W.pk32);
     E.prof.begin(st);

@@ -85,6 +85,10 @@ template <typename I>
 void launch_forces64(int64_t nrows, const int64_t* rows, const double4* pos, const double4* vm,
                      const double4* hydro, const double4* aux, const int64_t* off, const I* idx,
                      ForceParams prm, const int32_t* out_map, ForceOut out, cudaStream_t st);
+// FP32.  With the reconstruction vm, hydro and aux are arrays of one float4 per particle, (v, m),
+// (h, rho, Omega, P), (u, c_s, alpha, -).  Without it (prm.tidx and prm.tcnt given) vm holds two
+// per particle, (v, m) and (1/h, rho, 1/(Omega rho^2), P), aux is (u, c_s, alpha, Omega) and hydro
+// is not read.
 template <typename I>
 void launch_forces32(int64_t nrows, const int64_t* rows, const float4* pos, const double* box6,
                      const float4* vm, const float4* hydro, const float4* aux,

@@ -75,19 +75,14 @@ struct Pos32 {
     diff(own(i), j, dx, dy, dz);
   }
   // the difference and particle j's smoothing length, from the same record
-  template <typename V4>
-  __device__ __forceinline__ void diff_h(const Own& o, int64_t j, const V4* __restrict__,
-                                         float& dx, float& dy, float& dz, float& hj) const {
-    const float4 b = p[2 * j], cb = p[2 * j + 1];
+  __device__ __forceinline__ void diff_h(const Own& o, int64_t j, float& dx, float& dy, float& dz,
+                                         float& hj) const {
+    float4 b, cb;
+    ld_rec(p + 2 * j, b, cb);
     dx = fmaf(cb.x - o.c.x, cell, b.x - o.a.x);
     dy = fmaf(cb.y - o.c.y, cell, b.y - o.a.y);
     dz = fmaf(cb.z - o.c.z, cell, b.z - o.a.z);
     hj = cb.w;
-  }
-  template <typename V4>
-  __device__ __forceinline__ void diff_h(int64_t i, int64_t j, const V4* __restrict__ hydro,
-                                         float& dx, float& dy, float& dz, float& hj) const {
-    diff_h(own(i), j, hydro, dx, dy, dz, hj);
   }
 };
 
@@ -614,43 +609,222 @@ __device__ __forceinline__ R dwdr(R r, R h, int kid, R cnorm) {
 }
 
 constexpr int FORCE_QUEUE = 64;  // interacting entries a row queues before its lanes drain them
-#ifndef FORCE_UNROLL
-#define FORCE_UNROLL 4
-#endif
-// rounds of eight entries the walk launch (MODE 1) issues at once, and its resident blocks
-#ifndef WALK_UNROLL
-#define WALK_UNROLL 4
-#endif
-#ifndef WALK_BLOCKS
-#define WALK_BLOCKS 6
-#endif
-#ifndef WALK_OWN
-#define WALK_OWN 0  // 1: the walk launch keeps the row's own record in registers
-#endif
-// resident blocks per SM of the FP32 force pass (registers: 65536 / (256 * 4) = 64, a few spilled;
-// measured on the 4M torus 4.26 ms per launch against 4.59 with 3 blocks and 80 registers and
-// 5.63 with 2); the FP64 form keeps 2, its doubles would spill; the reconstruction forms, with
-// two 3x3 gradients per pair, 2 and 1
-#ifndef FORCE_BLOCKS_PER_SM_FP32
-#define FORCE_BLOCKS_PER_SM_FP32 4
-#endif
+constexpr int FORCE_UNROLL = 4;  // rounds of eight entries a walk issues at once
 
-// Fused pressure + artificial viscosity (+ conductivity) + P dV (+ disc viscosity) pass.  Eight
-// lanes per row (lanes 8g .. 8g+7 of a warp), each taking every eighth list entry; the pair terms
-// are summed per lane and then over the row's lanes.
-// MODE 0: the walk queues the interacting entries and drains them into the pair terms as it
-// goes.  The same pass can run as two launches: MODE 1 only walks, writing every row's
-// interacting entries (self included, list order) to prm.tidx / prm.tcnt, with few registers
-// and so many resident warps to hide the walk's dependent loads; MODE 2 then reads those
-// entries, every lane busy on pair terms, with no walk state alive beside the accumulators.
-template <int MODE, bool RECON>
-struct ForceBlocks {
-  static constexpr int value = MODE == 1 ? WALK_BLOCKS : RECON ? 2 : FORCE_BLOCKS_PER_SM_FP32;
-};
+// The FP32 pass without the reconstruction runs as two launches: k_walk32 tests the rows' lists and
+// writes their interacting entries, with few registers and so many resident warps to hide the
+// dependent loads; k_pairs32 then reads those entries, every lane busy on pair terms, with no walk
+// state alive beside the accumulators.
+//
+// k_walk32: every row's interacting entries (r < 2 max(h_a, h_b), self included, list order) to
+// prm.tidx (the lists' layout) and their number to prm.tcnt.  With prm.pos64 the level limiter reads
+// them too: entries within 1e-5 of the boundary are decided by the reference's FP64 test.
+// Bound by the gathers; 2.35M rows of the 4M torus: 2.33 ms (3.01 with the record in two loads and
+// the row's own read again per entry; 8 blocks per SM 2.28 for these rows but 3.86 against 3.80
+// for all, 5 blocks 2.58).
+template <typename I>
+__global__ void __launch_bounds__(NB_THREADS, 6)
+    k_walk32(int64_t nrows, const int64_t* __restrict__ rows, Pos32 geo,
+             const int64_t* __restrict__ off, const I* __restrict__ idx, ForceParams prm) {
+  geo.ready();
+  const unsigned FULL = 0xffffffffu;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t q = t >> 3;
+  const int gl = (int)(t & 7), g = (threadIdx.x & 31) >> 3;
+  const bool live = q < nrows;
+  if (!__any_sync(FULL, live)) return;  // warp-uniform
+  const int a = live ? (int)(rows ? rows[q] : q) : 0;
+  const Pos32::Own me = geo.own(a);
+  const float h_a = me.c.w;
+  const int64_t e_beg = live ? off[a] : 0;
+  const unsigned len = live ? (unsigned)(off[a + 1] - e_beg) : 0u;
+  const unsigned maxlen = __reduce_max_sync(FULL, len);
+  const I* list = idx + e_beg;
+  int32_t* out = prm.tidx + e_beg;
+  int m_tot = 0;
+  constexpr int U = FORCE_UNROLL;
+  for (unsigned base = 0; base < maxlen; base += 8 * U) {
+    int bb[U];
+    bool tight[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned e = base + 8 * u + gl;
+      bb[u] = e < len ? (int)ld_stream(list + e) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      tight[u] = bb[u] == a;  // self: listed for the limiter, not a pair
+      if (bb[u] >= 0 && bb[u] != a) {
+        float dx, dy, dz, h_b;
+        geo.diff_h(me, bb[u], dx, dy, dz, h_b);
+        const float rr = 2.0f * (h_a > h_b ? h_a : h_b);
+        const float d2 = sqdist(dx, dy, dz), r2 = rr * rr;
+        bool tk = d2 < r2;
+        if (prm.pos64 && d2 > r2 * (float)(1.0 - 1e-5) && d2 < r2 * (float)(1.0 + 1e-5)) {
+          const double4 pa = prm.pos64[a], pb = prm.pos64[bb[u]];
+          const double e2 = d2_exact(pb.x - pa.x, pb.y - pa.y, pb.z - pa.z);
+          const double er = 2.0 * fmax(pa.w, pb.w);
+          tk = e2 < er * er;
+        }
+        tight[u] = tk;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned seg = (__ballot_sync(FULL, tight[u]) >> (8 * g)) & 0xffu;
+      if (tight[u]) out[m_tot + __popc(seg & ((1u << gl) - 1u))] = bb[u];
+      m_tot += __popc(seg);
+    }
+  }
+  if (live && gl == 0) prm.tcnt[q] = m_tot;
+}
 
-template <typename R, typename PosT, typename I, typename V4, bool RECON, int MODE = 0>
-__global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, RECON>::value))
-    k_forces_g(int64_t nrows, const int64_t* __restrict__ rows, PosT geo_in,
+// k_pairs32: the pair terms of the rows' interacting entries.  One reciprocal square root per pair,
+// and reciprocals of the per-particle denominators that come with the records: pk (offset, m)
+// (cell, h); pv (v, m) (1/h, rho, 1/(Omega rho^2), P); aux (u, c_s, alpha, Omega).
+// Bound by issue and the gathers' latency; the same rows, 58 pairs each: 3.71 ms (4.55 with two
+// reciprocals per pair and five loads; 3 blocks per SM 3.85, 5 blocks 4.76).  The flags are looked
+// at per pair on purpose: a variant compiled for one of them fuses other operations, which changes
+// the float sums in their eighth digit.
+static __global__ void __launch_bounds__(NB_THREADS, 4)
+    k_pairs32(int64_t nrows, const int64_t* __restrict__ rows, Pos32 geo,
+              const float4* __restrict__ pv, const float4* __restrict__ aux,
+              const int64_t* __restrict__ off, ForceParams prm,
+              const int32_t* __restrict__ out_map, ForceOut out) {
+  geo.ready();
+  using R = float;
+  const unsigned FULL = 0xffffffffu;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t q = t >> 3;
+  const int gl = (int)(t & 7);
+  const bool live = q < nrows;
+  if (!__any_sync(FULL, live)) return;  // warp-uniform
+  const int a = live ? (int)(rows ? rows[q] : q) : 0;
+  const Pos32::Own me = geo.own(a);
+  const float4 va = pv[2 * (int64_t)a], ha = pv[2 * (int64_t)a + 1], xa = aux[a];
+  const R h_a = me.c.w, rho_a = ha.y, P_a = ha.w;
+  const R inv_or_a = R(1) / (xa.w * rho_a), inv_orr_a = ha.z;
+  const R cs_a = xa.y, al_a = xa.z, u_a = xa.x;
+  const R beta = (R)prm.beta, alpha_u = (R)prm.alpha_u, aav = (R)prm.disc_alpha_av;
+  const R cn = (R)prm.cnorm;
+  const int kid = prm.kid;
+  const R ih_a = ha.x;
+  const R cn4_a = cn * (ih_a * ih_a) * (ih_a * ih_a);
+  Acc<R> ax, ay, az, work, heat, vheat, cheat, dax, day, daz, dheat;
+  R vmax = prm.use_visc ? cs_a : R(0);
+  int npairs = 0;
+  auto pair = [&](int b) {
+    R ddx, ddy, ddz, h_b;
+    geo.diff_h(me, b, ddx, ddy, ddz, h_b);  // x_b - x_a
+    float4 vb, hb4;
+    ld_rec(pv + 2 * (int64_t)b, vb, hb4);
+    const float4 xb = aux[b];
+    const R d2 = sqdist(ddx, ddy, ddz);
+    npairs += 1;
+    const R rho_b = hb4.y, P_b = hb4.w;
+    const R m_b = vb.w;
+    const R inv_r = rsqrtf(d2);
+    const R r = d2 * inv_r;
+    const R rx = -ddx * inv_r, ry = -ddy * inv_r, rz = -ddz * inv_r;  // r_hat of x_a - x_b
+    const R ih_b = hb4.x;
+    const R fa = cn4_a * kernel_df<R>(r * ih_a, kid);
+    const R fb = cn * (ih_b * ih_b) * (ih_b * ih_b) * kernel_df<R>(r * ih_b, kid);
+    const R dvx = va.x - vb.x, dvy = va.y - vb.y, dvz = va.z - vb.z;
+    const R vdotr = dvx * rx + dvy * ry + dvz * rz;
+    R num_a = P_a, num_b = P_b;
+    const R inv_orr_b = hb4.z;
+    if (prm.use_visc) {
+      R vsig_a = al_a * cs_a + beta * fabs(vdotr);
+      R vsig_b = xb.z * xb.y + beta * fabs(vdotr);
+      if (vsig_a > vmax) vmax = vsig_a;
+      if (vdotr < R(0)) {
+        num_a += R(-0.5) * rho_a * vsig_a * vdotr;
+        num_b += R(-0.5) * rho_b * vsig_b * vdotr;
+        R dh = m_b * vsig_a * R(0.5) * vdotr * vdotr * fa * inv_or_a;
+        heat.add(-dh);
+        vheat.add(-dh);
+      }
+      if (prm.use_cond) {
+        R vu;
+        if (prm.cond_signal == 0)
+          vu = sqrt(fabs(P_a - P_b) * __frcp_rn(R(0.5) * (rho_a + rho_b)));
+        else
+          vu = fabs(vdotr);
+        R dc = m_b * alpha_u * vu * (u_a - xb.x) * R(0.5) *
+               (fa * inv_or_a + fb * inv_orr_b * rho_b);
+        heat.add(dc);
+        cheat.add(dc);
+      }
+    }
+    R f = m_b * (num_a * inv_orr_a * fa + num_b * inv_orr_b * fb);
+    ax.add(-f * rx);
+    ay.add(-f * ry);
+    az.add(-f * rz);
+    work.add(m_b * vdotr * fa);
+    if (prm.use_disc) {
+      const R vdr = vdotr;  // v_ab . (x_a - x_b) / r
+      R qa = -rho_a * h_a * R(0.5) * inv_r * aav * cs_a * vdr * inv_orr_a;
+      R qb = -rho_b * h_b * R(0.5) * inv_r * aav * xb.y * vdr * inv_orr_b;
+      R f = m_b * (qa * fa + qb * fb);
+      dax.add(-(f * rx));
+      day.add(-(f * ry));
+      daz.add(-(f * rz));
+      dheat.add(m_b * qa * vdr * fa);
+    }
+  };
+  const int cnt = live ? prm.tcnt[q] : 0;
+  const int32_t* list = prm.tidx + (live ? off[a] : 0);
+  int next = gl < cnt ? ld_stream(list + gl) : a;
+  for (int k = gl; k < cnt; k += 8) {
+    const int b = next;
+    next = k + 8 < cnt ? ld_stream(list + k + 8) : a;
+    if (b != a) pair(b);
+  }
+  double s_ax = group_total(ax), s_ay = group_total(ay), s_az = group_total(az);
+  double s_work = group_total(work), s_heat = group_total(heat);
+  double s_vheat = group_total(vheat), s_cheat = group_total(cheat);
+  double s_dax = 0, s_day = 0, s_daz = 0, s_dheat = 0;
+  if (prm.use_disc) {
+    s_dax = group_total(dax);
+    s_day = group_total(day);
+    s_daz = group_total(daz);
+    s_dheat = group_total(dheat);
+  }
+#pragma unroll
+  for (int of = 4; of > 0; of >>= 1) {
+    R vo = __shfl_xor_sync(FULL, vmax, of);
+    vmax = vo > vmax ? vo : vmax;
+    npairs += __shfl_xor_sync(FULL, npairs, of);
+  }
+  if (!live || gl != 0) return;
+  const int64_t o = out_map ? (int64_t)out_map[a] : q;
+  if (out.acc) {
+    out.acc[3 * o + 0] = s_ax;
+    out.acc[3 * o + 1] = s_ay;
+    out.acc[3 * o + 2] = s_az;
+  }
+  if (out.dudt) out.dudt[o] = (double)P_a * (double)inv_or_a / (double)rho_a * s_work + s_heat;
+  if (out.vsig) out.vsig[o] = (double)vmax;
+  if (out.vheat) out.vheat[o] = s_vheat;
+  if (out.cheat) out.cheat[o] = s_cheat;
+  if (prm.use_disc) {
+    if (out.dacc) {
+      out.dacc[3 * o + 0] = s_dax;
+      out.dacc[3 * o + 1] = s_day;
+      out.dacc[3 * o + 2] = s_daz;
+    }
+    if (out.ddudt) out.ddudt[o] = s_dheat;
+  }
+  if (out.pairs) out.pairs[o] = npairs;
+}
+
+// FP32 with the reconstruction: pressure + artificial viscosity (+ conductivity) + P dV (+ disc
+// viscosity) in one launch, eight lanes per row (lanes 8g .. 8g+7 of a warp); the walk queues the
+// interacting entries in shared memory and drains them into the pair terms as it goes.  Two
+// blocks per SM: with two 3x3 gradients per pair more would spill.
+template <typename R, typename PosT, typename I, typename V4>
+__global__ void __launch_bounds__(NB_THREADS, 2)
+    k_forces_recon32(int64_t nrows, const int64_t* __restrict__ rows, PosT geo_in,
              const V4* __restrict__ vm,    // (vx, vy, vz, mass)
              const V4* __restrict__ hydro, // (h, rho, omega, P)
              const V4* __restrict__ aux,   // (u, c_s, alpha, unused)
@@ -697,10 +871,7 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, RECON>::value))
   R Ga[9];
 #pragma unroll
   for (int e = 0; e < 9; ++e) {
-    if constexpr (!RECON)
-      Ga[e] = R(0);
-    else
-      Ga[e] = prm.gv32[9 * a + e];
+    Ga[e] = prm.gv32[9 * a + e];
   }
   const R eta_crit = (R)prm.eta_crit, eta_fold = (R)prm.eta_fold;
   auto recon_visc = [&](int64_t b, R dx0, R dx1, R dx2, R r, R rx, R ry, R rz, R h_b, R vdotr,
@@ -781,21 +952,8 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, RECON>::value))
     if (prm.use_sph) {
       if (prm.use_visc) {
         const V4 xb = aux[b];
-        if constexpr (RECON) {
-          recon_visc(b, -ddx, -ddy, -ddz, r, rx, ry, rz, h_b, vdotr, vb, xb, rho_b, m_b, fa,
-                     num_a, num_b);
-        } else {
-          R vsig_a = al_a * cs_a + beta * fabs(vdotr);
-          R vsig_b = (R)xb.z * (R)xb.y + beta * fabs(vdotr);
-          if (vsig_a > vmax) vmax = vsig_a;
-          if (vdotr < R(0)) {
-            num_a += R(-0.5) * rho_a * vsig_a * vdotr;
-            num_b += R(-0.5) * rho_b * vsig_b * vdotr;
-            R dh = m_b * vsig_a * R(0.5) * vdotr * vdotr * fa * inv_or_a;
-            heat.add(-dh);
-            vheat.add(-dh);
-          }
-        }
+        recon_visc(b, -ddx, -ddy, -ddz, r, rx, ry, rz, h_b, vdotr, vb, xb, rho_b, m_b, fa, num_a,
+                   num_b);
         if (prm.use_cond) {
           R vu;
           if (prm.cond_signal == 0)
@@ -837,20 +995,10 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, RECON>::value))
   // written out for the level limiter: exactly the reference's FP64 test, which the FP32 form
   // takes from prm.pos64 where its float test falls within 1e-5 of the boundary
   int m_tot = 0;
-  if constexpr (MODE == 2) {
-    // the interacting entries the walk launch wrote (self included: skipped here)
-    const int cnt = live ? prm.tcnt[q] : 0;
-    for (int k2 = gl; k2 < cnt; k2 += 8) {
-      const int64_t b = (int64_t)ld_stream(prm.tidx + e_beg + k2);
-      if (b == a) continue;
-      pair_fast(b);
-    }
-  }
   // FORCE_UNROLL rounds of eight entries at a time: their index and position loads are issued
   // together, then the rounds are queued one after the other in list order
-  constexpr int FU = MODE == 1 ? WALK_UNROLL : FORCE_UNROLL;
-  const typename PosT::Own me_walk = geo.own(a);
-  for (unsigned base = 0; MODE != 2 && base < maxlen; base += 8 * FU) {
+  constexpr int FU = FORCE_UNROLL;
+  for (unsigned base = 0; base < maxlen; base += 8 * FU) {
     int64_t bb[FU];
     bool take[FU], tight[FU];
 #pragma unroll
@@ -868,10 +1016,7 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, RECON>::value))
           bool tk = true;
           if (prm.tighten) {
             R ddx, ddy, ddz, h_b;
-            if constexpr (MODE == 1 && WALK_OWN)
-              geo.diff_h(me_walk, b, hydro, ddx, ddy, ddz, h_b);
-            else
-              geo.diff_h(a, b, hydro, ddx, ddy, ddz, h_b);
+            geo.diff_h(geo.own(a), b, ddx, ddy, ddz, h_b);
             R rr = R(2) * (h_a > h_b ? h_a : h_b);
             const R d2 = sqdist(ddx, ddy, ddz), r2 = rr * rr;
             tk = d2 < r2;
@@ -891,11 +1036,9 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, RECON>::value))
     }
 #pragma unroll
     for (int u = 0; u < FU; ++u) {
-      if constexpr (MODE == 0) {
-        unsigned seg = (__ballot_sync(FULL, take[u]) >> (8 * g)) & 0xffu;
-        if (take[u]) pq[pc + __popc(seg & ((1u << gl) - 1u))] = (int32_t)bb[u];
-        pc += __popc(seg);
-      }
+      unsigned seg = (__ballot_sync(FULL, take[u]) >> (8 * g)) & 0xffu;
+      if (take[u]) pq[pc + __popc(seg & ((1u << gl) - 1u))] = (int32_t)bb[u];
+      pc += __popc(seg);
       if (prm.tidx) {
         const unsigned tseg = (__ballot_sync(FULL, tight[u]) >> (8 * g)) & 0xffu;
         if (tight[u])
@@ -903,11 +1046,10 @@ __global__ void __launch_bounds__(NB_THREADS, (ForceBlocks<MODE, RECON>::value))
         m_tot += __popc(tseg);
       }
     }
-    if (MODE == 0 && __any_sync(FULL, pc > FORCE_QUEUE - 8)) drain();
+    if (__any_sync(FULL, pc > FORCE_QUEUE - 8)) drain();
   }
-  if constexpr (MODE == 0) drain();
-  if (MODE != 2 && prm.tcnt && live && gl == 0) prm.tcnt[q] = m_tot;
-  if constexpr (MODE == 1) return;  // the walk launch writes only the entries and counts
+  drain();
+  if (prm.tcnt && live && gl == 0) prm.tcnt[q] = m_tot;
   // sums over the row's eight lanes (uniform flags: every lane takes part in every reduction)
   double s_ax = 0, s_ay = 0, s_az = 0, s_work = 0, s_heat = 0, s_vheat = 0, s_cheat = 0;
   double s_dax = 0, s_day = 0, s_daz = 0, s_dheat = 0;
