@@ -101,6 +101,10 @@ _SIGS = {
                                      _vp, _vp]),
     "nb_deposit_log": (_int, [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _dbl, _dbl, _dbl, _dbl, _int,
                               _int, _int, _int, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "nb_log_tables": (_int, [_vp, _dbl, _dbl, _dbl, _dbl, _int, _int, _int, _vp, _vp]),
+    "nb_deposit_log_split": (_int, [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _dbl, _dbl, _dbl, _dbl,
+                                    _int, _int, _int, _dbl, _dbl, _dbl, _int, _int, _int, _dbl,
+                                    _int, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "nb_deposit_box": (_int, [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _dbl, _dbl, _dbl, _dbl, _int,
                               _int, _vp, _vp, _vp, _vp]),
     "nb_grid_finish": (_int, [_vp, _i64, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp]),

@@ -500,39 +500,74 @@ int nb_eos(nb_ctx* ctx, int64_t n, const double* rho, const double* u, const nb_
 }
 
 // ---------------------------------------------------------------- grid deposition
-// On the log grid large inputs are deposited in the spatial order of their centres' cells (sorted keys, gathered
-// copies of the particle data): neighbouring threads then add to neighbouring cells.
-constexpr int64_t DEPOSIT_SORT_MIN = 1 << 16;
-
-static int deposit_order(Engine& E, int64_t n, const nbk::LogGeom& g, const double*& x,
-                         const double*& h, const double*& m, const double*& t, const double*& v,
-                         cudaStream_t st) {
-  if (n < DEPOSIT_SORT_MIN) return 0;
-  NB_TRY(E.ensure_deposit(n));
-  nbk::launch_deposit_keys(n, x, g, E.dep_k0, E.dep_i0, st);
-  const unsigned long long max_key = (unsigned long long)(g.nr + 2) * g.nth * g.nph;
-  int bits = 1;
-  while (bits < 64 && (1ull << bits) <= max_key) ++bits;
-  cub::DoubleBuffer<unsigned long long> kb(E.dep_k0, E.dep_k1);
-  cub::DoubleBuffer<int32_t> vb(E.dep_i0, E.dep_i1);
-  size_t tmp = E.cub_bytes;
-  NB_CUDA(cub::DeviceRadixSort::SortPairs(E.cub_tmp, tmp, kb, vb, (int)n, 0, bits, st));
-  nbk::launch_deposit_gather(n, vb.Current(), x, h, m, t, v, E.dep_buf, st);
-  x = E.dep_buf;
-  h = E.dep_buf + 3 * n;
-  m = h + n;
-  t = m + n;
-  v = t + n;
+// `count` grids' mass outside and trilinear counts back to the host (and the wide particles)
+static int deposit_finish_host(nbk::Engine& E, int count, double* outside, int64_t* n_trilinear,
+                               int64_t* n_wide, cudaStream_t st) {
+  NB_CUDA(cudaGetLastError());
+  nbk::Workspace& W = E.ws;
+  NB_CUDA(cudaMemcpyAsync(W.h_dbl, W.d_scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+  NB_CUDA(cudaMemcpyAsync(W.h_i64, W.d_i64, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  NB_CUDA(nbk::host_sync(st));
+  for (int g = 0; g < count; ++g) {
+    outside[g] = W.h_dbl[g];
+    n_trilinear[g] = W.h_i64[g];
+  }
+  if (n_wide) *n_wide = W.h_i64[2];
   return 0;
 }
 
-static int deposit_finish_host(nbk::Engine& E, double* outside, int64_t* n_trilinear,
-                               cudaStream_t st) {
-  NB_CUDA(cudaGetLastError());
-  NB_CUDA(cudaMemcpyAsync(outside, E.ws.d_scal, sizeof(double), cudaMemcpyDeviceToHost, st));
-  NB_CUDA(cudaMemcpyAsync(n_trilinear, E.ws.d_i64, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  NB_CUDA(nbk::host_sync(st));
+static int deposit_zero(nbk::Engine& E, double* acc, int64_t ncell, cudaStream_t st) {
+  NB_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * nbk::DEP_FIELDS * ncell, st));
+  NB_CUDA(cudaMemsetAsync(E.ws.d_scal, 0, 2 * sizeof(double), st));
+  NB_CUDA(cudaMemsetAsync(E.ws.d_i64, 0, 4 * sizeof(int64_t), st));
   return 0;
+}
+
+static bool log_grid_ok(double r_min, double dlnr, int nr, int nth, int nph) {
+  return nr >= 1 && nth >= 2 && nph >= 1 && r_min > 0.0 && dlnr > 0.0;
+}
+
+static nbk::LogGeom log_geom(double r_min, double dlnr, double dth, double dph, int nr, int nth,
+                             int nph, const double* tables) {
+  return nbk::LogGeom{r_min, dlnr, dth, dph, nr, nth, nph, tables, tables + nth, tables + 2 * nth,
+                      tables + 3 * nth, tables + 3 * nth + nph};
+}
+
+int nb_log_tables(nb_ctx* ctx, double r_min, double dlnr, double dth, double dph, int nr, int nth,
+                  int nph, double* tables, void* stream) {
+  NB_TRY(begin(ctx));
+  Engine& E = ctx->E;
+  if (!log_grid_ok(r_min, dlnr, nr, nth, nph))
+    return nbk::set_host_error(E, "bad log-spherical grid"), NB_ERR_INPUT;
+  nbk::launch_log_tables(log_geom(r_min, dlnr, dth, dph, nr, nth, nph, tables), tables, S(stream));
+  NB_CUDA(cudaGetLastError());
+  return 0;
+}
+
+int nb_deposit_log_split(nb_ctx* ctx, int64_t n, const double* x, const double* h, const double* m,
+                         const double* t, const double* v, double r_min, double dlnr, double dth,
+                         double dph, int nr, int nth, int nph, double dlnr_c, double dth_c,
+                         double dph_c, int nr_c, int nth_c, int nph_c, double wide_cells,
+                         int kernel_id, const double* tables, const double* tables_c, double* acc,
+                         double* acc_c, double* outside, int64_t* n_trilinear, int64_t* n_wide,
+                         void* stream) {
+  NB_TRY(begin(ctx));
+  Engine& E = ctx->E;
+  if (kernel_id != 0 && kernel_id != 1) return nbk::set_host_error(E, "bad kernel_id"), NB_ERR_INPUT;
+  if (!log_grid_ok(r_min, dlnr, nr, nth, nph) || !log_grid_ok(r_min, dlnr_c, nr_c, nth_c, nph_c) ||
+      !(wide_cells > 0.0))
+    return nbk::set_host_error(E, "bad log-spherical grid"), NB_ERR_INPUT;
+  if (!outside || !n_trilinear || !n_wide)
+    return nbk::set_host_error(E, "outputs missing"), NB_ERR_INPUT;
+  cudaStream_t st = S(stream);
+  NB_TRY(E.ws.ensure(E, std::max<int64_t>(E.ws.cap, 1024)));
+  NB_TRY(deposit_zero(E, acc, (int64_t)nr * nth * nph, st));
+  NB_CUDA(cudaMemsetAsync(acc_c, 0, sizeof(double) * nbk::DEP_FIELDS * nr_c * nth_c * nph_c, st));
+  const nbk::LogGeom g = log_geom(r_min, dlnr, dth, dph, nr, nth, nph, tables);
+  const nbk::LogGeom gc = log_geom(r_min, dlnr_c, dth_c, dph_c, nr_c, nth_c, nph_c, tables_c);
+  NB_TRY(nbk::deposit_log(E, n, x, h, m, t, v, g, &gc, wide_cells, kernel_id, acc, acc_c,
+                          E.ws.d_scal, (unsigned long long*)E.ws.d_i64, st));
+  return deposit_finish_host(E, 2, outside, n_trilinear, n_wide, st);
 }
 
 int nb_deposit_log(nb_ctx* ctx, int64_t n, const double* x, const double* h, const double* m,
@@ -543,20 +578,16 @@ int nb_deposit_log(nb_ctx* ctx, int64_t n, const double* x, const double* h, con
   NB_TRY(begin(ctx));
   Engine& E = ctx->E;
   if (kernel_id != 0 && kernel_id != 1) return nbk::set_host_error(E, "bad kernel_id"), NB_ERR_INPUT;
-  if (nr < 1 || nth < 2 || nph < 1 || !(r_min > 0.0) || !(dlnr > 0.0))
+  if (!log_grid_ok(r_min, dlnr, nr, nth, nph))
     return nbk::set_host_error(E, "bad log-spherical grid"), NB_ERR_INPUT;
   if (!outside || !n_trilinear) return nbk::set_host_error(E, "outputs missing"), NB_ERR_INPUT;
   cudaStream_t st = S(stream);
   NB_TRY(E.ws.ensure(E, std::max<int64_t>(E.ws.cap, 1024)));
-  const int64_t ncell = (int64_t)nr * nth * nph;
-  NB_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * nbk::DEP_FIELDS * ncell, st));
-  NB_CUDA(cudaMemsetAsync(E.ws.d_scal, 0, sizeof(double), st));
-  NB_CUDA(cudaMemsetAsync(E.ws.d_i64, 0, sizeof(int64_t), st));
+  NB_TRY(deposit_zero(E, acc, (int64_t)nr * nth * nph, st));
   nbk::LogGeom g{r_min, dlnr, dth, dph, nr, nth, nph, sth, cth, dcth, cph, sph};
-  NB_TRY(deposit_order(E, n, g, x, h, m, t, v, st));
-  nbk::launch_deposit_log(n, x, h, m, t, v, g, kernel_id, acc, E.ws.d_scal,
-                          (unsigned long long*)E.ws.d_i64, st);
-  return deposit_finish_host(E, outside, n_trilinear, st);
+  NB_TRY(nbk::deposit_log(E, n, x, h, m, t, v, g, nullptr, 0.0, kernel_id, acc, nullptr, E.ws.d_scal,
+                          (unsigned long long*)E.ws.d_i64, st));
+  return deposit_finish_host(E, 1, outside, n_trilinear, nullptr, st);
 }
 
 int nb_deposit_box(nb_ctx* ctx, int64_t n, const double* x, const double* h, const double* m,
@@ -570,13 +601,10 @@ int nb_deposit_box(nb_ctx* ctx, int64_t n, const double* x, const double* h, con
   if (!outside || !n_trilinear) return nbk::set_host_error(E, "outputs missing"), NB_ERR_INPUT;
   cudaStream_t st = S(stream);
   NB_TRY(E.ws.ensure(E, std::max<int64_t>(E.ws.cap, 1024)));
-  const int64_t ncell = (int64_t)nb * nb * nb;
-  NB_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * nbk::DEP_FIELDS * ncell, st));
-  NB_CUDA(cudaMemsetAsync(E.ws.d_scal, 0, sizeof(double), st));
-  NB_CUDA(cudaMemsetAsync(E.ws.d_i64, 0, sizeof(int64_t), st));
+  NB_TRY(deposit_zero(E, acc, (int64_t)nb * nb * nb, st));
   NB_TRY(nbk::deposit_box(E, n, x, h, m, t, v, x0, y0, z0, dx, nb, kernel_id, acc, E.ws.d_scal,
                           (unsigned long long*)E.ws.d_i64, st));
-  return deposit_finish_host(E, outside, n_trilinear, st);
+  return deposit_finish_host(E, 1, outside, n_trilinear, nullptr, st);
 }
 
 int nb_grid_finish(nb_ctx* ctx, int64_t ncell, const double* acc, const double* vol,

@@ -2,8 +2,9 @@
 // each particle's fields (m, m T, m T^4, m v) go to the cells whose centres lie inside its
 // support (q < 2), weighted by f(q) V_c and normalised; fewer than 8 such centres: trilinear
 // weights in index space over the 8 nearest centres.  Weight beyond the grid goes to the
-// `outside` total.  On the log grid one thread per particle walks its candidate centres twice (sum
-// of weights, then the atomic adds); the box is gathered brick by brick; the cell sums are FP64.  Compiled without fused multiply-add, so a
+// `outside` total.  On the log grid a thread (a warp for wide supports) walks a particle's candidate
+// centres twice (sum of weights, then the atomic adds); the box is gathered brick by brick; the
+// cell sums are FP64.  Compiled without fused multiply-add, so a
 // particle's weights round like the reference's (the order of the atomic adds does not).
 #include <cub/cub.cuh>
 
@@ -16,10 +17,10 @@ namespace nbk {
 constexpr int DEP_MIN_CELLS = 8;
 constexpr int DEP_INNER_VIRTUAL = 64;  // virtual log shells below r_min (render/gasgrid.py:49)
 
-__device__ __forceinline__ double py_mod(double a, double b) {  // Python's a % b, b > 0
-  double r = fmod(a, b);
-  if (r < 0.0) r += b;
-  return r;
+// the azimuth in [0, 2 pi): Python's atan2(y, x) % (2 pi)
+__device__ __forceinline__ double azimuth(double y, double x) {
+  const double a = atan2(y, x);
+  return a < 0.0 ? a + 2.0 * 3.141592653589793 : a;
 }
 __device__ __forceinline__ int py_imod(int a, int b) { return ((a % b) + b) % b; }
 
@@ -41,119 +42,154 @@ __device__ __forceinline__ void add_cell(double* acc, int64_t cell, double w, co
   for (int f = 0; f < DEP_FIELDS; ++f) atomicAdd(c + f, w * vals[f]);
 }
 
-// render/gasgrid.py:316-412 (_nb_log_kernel_pass): MODE 0 sums f V and counts the centres
-// inside the support, MODE 1 adds the normalised weights and returns the mass beyond the grid
-template <int MODE>
-__device__ void log_pass(const LogGeom& g, double xp, double yp, double zp, double rr,
-                         double th, double ph, double hp, int i_lo, int i_hi, int kid,
-                         double inv, const double* vals, double* acc, double& wsum, int& n_in,
-                         double& outside) {
-  const double big = 2.0 * hp;
-  const double ct0 = cos(th), st0 = sin(th);
-  // q < 2 decided on d^2 against (2h)^2 with a relative margin of 1e-12 (sqrt(d^2) / h only
-  // inside the margin); the weights take q = sqrt(d^2) (1 / h), within an ulp of the
-  // reference's quotient
-  const double big2 = big * big;
-  const double in2 = big2 * (1.0 - 1e-12), out2 = big2 * (1.0 + 1e-12);
-  const double ih = 1.0 / hp;
-  for (int i = i_lo; i <= i_hi; ++i) {
-    const double rc = g.r_min * exp((i + 0.5) * g.dlnr);
-    const double cos_a = (rc * rc + rr * rr - big * big) / (2.0 * rc * rr);
-    if (cos_a > 1.0) continue;
-    int j0, j1;
-    if (cos_a <= -1.0) {
-      j0 = 0;
-      j1 = g.nth - 1;
-    } else {
-      const double a = acos(cos_a);
-      j0 = max(0, (int)floor((th - a) / g.dth) - 1);
-      j1 = min(g.nth - 1, (int)floor((th + a) / g.dth) + 1);
+// ---------------------------------------------------------------- log-spherical grid
+// Shell i of a log grid, from -DEP_INNER_VIRTUAL: radius of its centres and (r2^3 - r1^3) / 3.
+__device__ __forceinline__ double2 log_shell(const LogGeom& g, int i) {
+  const double rc = g.r_min * exp((i + 0.5) * g.dlnr);
+  const double r1 = g.r_min * exp(i * g.dlnr);
+  const double r2 = r1 * exp(g.dlnr);
+  return make_double2(rc, (r2 * r2 * r2 - r1 * r1 * r1) / 3.0);
+}
+
+__global__ void k_log_shells(LogGeom g, double2* __restrict__ shells) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < g.nr + DEP_INNER_VIRTUAL) shells[i] = log_shell(g, i - DEP_INNER_VIRTUAL);
+}
+
+// The tables of a grid in the order sth, cth, dcth (nth each), cph, sph (nph each), cell volumes
+// (nr, nth) (render/gasgrid.py:125-129, 688-692).
+__global__ void k_log_tables(LogGeom g, double* __restrict__ out) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  double* vol = out + 3 * g.nth + 2 * g.nph;
+  if (e < g.nth) {
+    const double th = (e + 0.5) * g.dth;
+    out[e] = sin(th);
+    out[g.nth + e] = cos(th);
+    out[2 * g.nth + e] = cos(e * g.dth) - cos((e + 1) * g.dth);
+  }
+  if (e < g.nph) {
+    const double ph = (e + 0.5) * g.dph;
+    out[3 * g.nth + e] = cos(ph);
+    out[3 * g.nth + g.nph + e] = sin(ph);
+  }
+  if (e < g.nr * g.nth) {
+    const int i = e / g.nth, j = e % g.nth;
+    const double r1 = g.r_min * exp(i * g.dlnr), r2 = r1 * exp(g.dlnr);
+    vol[e] = (r2 * r2 * r2 - r1 * r1 * r1) / 3.0 *
+             (cos(j * g.dth) - cos((j + 1) * g.dth)) * g.dph;
+  }
+}
+
+// One particle's candidate centres: a block of shells, theta rows and phi columns that holds every
+// centre inside its support, from the support's angular radius asin(2h / r) and the widest
+// azimuth asin(2h / (r sin theta)) of that cap, both a hair wide.
+struct LogParticle {
+  double x, y, z, h, rr, th, ph;
+  int i_lo, i_hi, j0, nj, k0, nk;
+};
+
+__device__ __forceinline__ LogParticle log_particle(const LogGeom& g, int64_t p,
+                                                    const double* __restrict__ x,
+                                                    const double* __restrict__ h) {
+  LogParticle q;
+  q.x = x[3 * p];
+  q.y = x[3 * p + 1];
+  q.z = x[3 * p + 2];
+  q.h = h[p];
+  const double big = 2.0 * q.h;
+  q.rr = sqrt(q.x * q.x + q.y * q.y + q.z * q.z);
+  q.th = acos(fmin(1.0, fmax(-1.0, q.z / q.rr)));
+  q.ph = azimuth(q.y, q.x);
+  const double s = big / q.rr;
+  const int i_max = (int)fmin(720.0 / g.dlnr, 1e9);  // beyond, radii overflow
+  q.j0 = q.k0 = 0;
+  q.nj = g.nth;
+  q.nk = g.nph;
+  if (s < 1.0) {
+    // log(1 + s) <= s, log(1 - s) >= -s / (1 - s)
+    const double fr = log(q.rr / g.r_min) / g.dlnr;
+    q.i_hi = (int)floor(fmin(fr + s / g.dlnr + 1e-6, (double)i_max));
+    q.i_lo = (int)floor(fmax(fr - s / ((1.0 - s) * g.dlnr) - 1e-6, -(double)DEP_INNER_VIRTUAL)) - 1;
+    const double a = asin(s) + 1e-9, st = sqrt(q.x * q.x + q.y * q.y) / q.rr;
+    q.j0 = max(0, (int)floor((q.th - a) / g.dth - 0.5));
+    q.nj = min(g.nth - 1, (int)ceil((q.th + a) / g.dth - 0.5)) - q.j0 + 1;
+    if (s < st * (1.0 - 1e-6)) {
+      const double d = asin(s / st) + 1e-9;
+      const int k0 = (int)floor((q.ph - d) / g.dph - 0.5), k1 = (int)ceil((q.ph + d) / g.dph - 0.5);
+      if (k1 - k0 + 1 < g.nph) {
+        q.k0 = k0;
+        q.nk = k1 - k0 + 1;
+      }
     }
-    const double r1 = g.r_min * exp(i * g.dlnr);
-    const double r2 = r1 * exp(g.dlnr);
-    const double vr = (r2 * r2 * r2 - r1 * r1 * r1) / 3.0;
-    const bool ing = 0 <= i && i < g.nr;
-    for (int j = j0; j <= j1; ++j) {
-      const double ss = st0 * g.sth[j];
-      bool full = true;
-      int k0 = 0, k1 = g.nph - 1;
-      if (ss > 1e-300 && cos_a > -1.0) {
-        const double cd = (cos_a - ct0 * g.cth[j]) / ss;
-        if (cd > 1.0 + 1e-12) continue;
-        if (cd > -1.0) {
-          const double dp = acos(fmin(cd, 1.0));
-          k0 = (int)ceil((ph - dp) / g.dph - 0.5) - 1;
-          k1 = (int)floor((ph + dp) / g.dph - 0.5) + 1;
-          if (k1 - k0 + 1 < g.nph) full = false;
-        }
-      }
-      if (full) {
-        k0 = 0;
-        k1 = g.nph - 1;
-      }
-      const double rst = rc * g.sth[j];
-      const double dzc = rc * g.cth[j] - zp;
-      const double vrt = vr * g.dcth[j] * g.dph;
-      for (int kk = k0; kk <= k1; ++kk) {
-        const int k = py_imod(kk, g.nph);
-        const double dxc = rst * g.cph[k] - xp;
-        const double dyc = rst * g.sph[k] - yp;
-        const double dd = dxc * dxc + dyc * dyc + dzc * dzc;
+  } else {
+    q.i_hi = (int)fmin(floor((log(q.rr + big) - log(g.r_min)) / g.dlnr), (double)i_max);
+    q.i_lo = -DEP_INNER_VIRTUAL;
+  }
+  q.i_lo = max(q.i_lo, -DEP_INNER_VIRTUAL);
+  if (!(big > 0.0) || isnan(s) || isinf(q.rr)) q.nj = 0;  // no centre is inside
+  return q;
+}
+
+// render/gasgrid.py:316-412 (_nb_log_kernel_pass) over those candidates, dealt to `size` threads:
+// MODE 0 sums f V and counts the centres inside the support, MODE 1 adds the normalised weights
+// and the mass beyond the grid.  q < 2 is decided on d^2 against (2h)^2 with a relative margin of
+// 1e-12 (sqrt(d^2) / h only inside the margin); the weights take q = sqrt(d^2) (1 / h), within an ulp
+// of the reference's quotient.
+template <int MODE>
+__device__ __forceinline__ void log_pass(const LogGeom& g, const double2* __restrict__ shells,
+                                         const LogParticle& q, int rank, int size, int kid,
+                                         double inv, const double* vals, double* acc,
+                                         double& wsum, int& n_in, double& outside) {
+  const double big = 2.0 * q.h, big2 = big * big;
+  const double in2 = big2 * (1.0 - 1e-12), out2 = big2 * (1.0 + 1e-12);
+  const double ih = 1.0 / q.h;
+  const int dj = size / q.nk, dk = size % q.nk;
+  int j = q.j0 + rank / q.nk, c = rank % q.nk;
+  for (int e = rank; e < q.nj * q.nk; e += size) {
+    int k = q.k0 + c;
+    if (k < 0 || k >= g.nph) k = py_imod(k, g.nph);
+    const double sth = g.sth[j], cth = g.cth[j], cph = g.cph[k], sph = g.sph[k];
+    const double ux = sth * cph, uy = sth * sph;
+    // the nearest point of the ray through this column's centres
+    const double along = q.x * ux + q.y * uy + q.z * cth;
+    const double off2 = along > 0.0 ? q.rr * q.rr - along * along : q.rr * q.rr;
+    if (off2 < out2 + 1e-9 * q.rr * q.rr) {
+      const double dvol = g.dcth[j] * g.dph;
+      for (int i = q.i_lo; i <= q.i_hi; ++i) {
+        const double2 sh = i < g.nr ? shells[i + DEP_INNER_VIRTUAL] : log_shell(g, i);
+        const double dxc = fma(sh.x, ux, -q.x), dyc = fma(sh.x, uy, -q.y), dzc = fma(sh.x, cth, -q.z);
+        const double dd = fma(dzc, dzc, fma(dyc, dyc, dxc * dxc));
         if (dd >= out2) continue;
         const double r = sqrt(dd);
-        if (dd >= in2 && !(r / hp < 2.0)) continue;
-        const double q = r * ih;
-        {
-          if (MODE == 0) {
-            n_in += 1;
-            wsum += kernel_f<double>(q, kid) * vrt;
-          } else {
-            const double w = kernel_f<double>(q, kid) * vrt * inv;
-            if (ing)
-              add_cell(acc, ((int64_t)i * g.nth + j) * g.nph + k, w, vals);
-            else
-              outside += w * vals[0];
-          }
+        if (dd >= in2 && !(r / q.h < 2.0)) continue;
+        const double f = kernel_f<double>(r * ih, kid) * (sh.y * dvol);
+        if (MODE == 0) {
+          n_in += 1;
+          wsum += f;
+        } else {
+          const double w = f * inv;
+          if (0 <= i && i < g.nr)
+            add_cell(acc, ((int64_t)i * g.nth + j) * g.nph + k, w, vals);
+          else
+            outside += w * vals[0];
         }
       }
+    }
+    j += dj;
+    c += dk;
+    if (c >= q.nk) {
+      c -= q.nk;
+      j += 1;
     }
   }
 }
 
-// render/gasgrid.py:415-531 (_nb_log_deposit_chunk)
-__global__ void k_deposit_log(int64_t n, const double* __restrict__ x,
-                              const double* __restrict__ h, const double* __restrict__ m,
-                              const double* __restrict__ t, const double* __restrict__ v,
-                              LogGeom g, int kid, double* __restrict__ acc, double* outside_sum,
-                              unsigned long long* n_tri) {
-  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  double vals[DEP_FIELDS];
-  particle_vals(p, m, t, v, vals);
-  const double xp = x[3 * p], yp = x[3 * p + 1], zp = x[3 * p + 2];
-  const double rr = sqrt(xp * xp + yp * yp + zp * zp);
-  const double hp = h[p];
-  const double big = 2.0 * hp;
-  const double lnr0 = log(g.r_min);
-  const int i_hi = (int)floor((log(rr + big) - lnr0) / g.dlnr);
-  int i_lo = -DEP_INNER_VIRTUAL;
-  if (!(big >= rr)) i_lo = max((int)floor((log(rr - big) - lnr0) / g.dlnr), -DEP_INNER_VIRTUAL);
-  const double th = acos(fmin(1.0, fmax(-1.0, zp / rr)));
-  const double ph = py_mod(atan2(yp, xp), 2.0 * 3.141592653589793);
-  double wsum = 0.0, out = 0.0;
-  int n_in = 0;
-  log_pass<0>(g, xp, yp, zp, rr, th, ph, hp, i_lo, i_hi, kid, 0.0, vals, acc, wsum, n_in, out);
-  if (n_in >= DEP_MIN_CELLS) {
-    log_pass<1>(g, xp, yp, zp, rr, th, ph, hp, i_lo, i_hi, kid, 1.0 / wsum, vals, acc, wsum,
-                n_in, out);
-    if (out != 0.0) atomicAdd(outside_sum, out);
-    return;
-  }
-  // trilinear fallback (render/gasgrid.py:217-237)
-  atomicAdd(n_tri, 1ull);
-  const double fr = log(rr / g.r_min) / g.dlnr - 0.5;
-  const double fth = th / g.dth - 0.5;
-  const double fph = ph / g.dph - 0.5;
+// render/gasgrid.py:217-237: trilinear weights in index space over the eight nearest centres
+__device__ __forceinline__ void log_trilinear(const LogGeom& g, const LogParticle& q,
+                                              const double* vals, double* acc, double& out) {
+  const double fr = log(q.rr / g.r_min) / g.dlnr - 0.5;
+  const double fth = q.th / g.dth - 0.5;
+  const double fph = q.ph / g.dph - 0.5;
   const int i0 = (int)floor(fr);
   int j0 = (int)floor(fth);
   const int k0 = (int)floor(fph);
@@ -174,15 +210,112 @@ __global__ void k_deposit_log(int64_t n, const double* __restrict__ x,
       for (int dk = 0; dk < 2; ++dk) {
         const double wk = dk == 1 ? tk : 1.0 - tk;
         const double w = wi * wj * wk;
-        const int i = i0 + di;
+        const int64_t i = (int64_t)i0 + di;
         if (0 <= i && i < g.nr)
-          add_cell(acc, ((int64_t)i * g.nth + j0 + dj) * g.nph + py_imod(k0 + dk, g.nph), w, vals);
+          add_cell(acc, (i * g.nth + j0 + dj) * g.nph + py_imod(k0 + dk, g.nph), w, vals);
         else
           out += w * vals[0];
       }
     }
   }
-  if (out != 0.0) atomicAdd(outside_sum, out);
+}
+
+struct LogTarget {
+  LogGeom g;
+  const double2* shells;
+  double* acc;
+  double* outside;
+  unsigned long long* n_tri;
+};
+
+// render/gasgrid.py:415-531 (_nb_log_deposit_chunk) for one particle, by one thread or by a warp;
+// returns (a part of) the mass beyond the grid
+template <int SIZE>
+__device__ __forceinline__ double log_one(const LogTarget& T, const LogParticle& q, int64_t p,
+                                          int rank, const double* __restrict__ m,
+                                          const double* __restrict__ t,
+                                          const double* __restrict__ v, int kid) {
+  double vals[DEP_FIELDS];
+  particle_vals(p, m, t, v, vals);
+  double wsum = 0.0, out = 0.0;
+  int n_in = 0;
+  log_pass<0>(T.g, T.shells, q, rank, SIZE, kid, 0.0, vals, T.acc, wsum, n_in, out);
+  if (SIZE > 1) {
+    n_in = __reduce_add_sync(0xffffffffu, n_in);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, d);
+  }
+  if (n_in >= DEP_MIN_CELLS) {
+    log_pass<1>(T.g, T.shells, q, rank, SIZE, kid, 1.0 / wsum, vals, T.acc, wsum, n_in, out);
+  } else if (rank == 0) {
+    atomicAdd(T.n_tri, 1ull);
+    log_trilinear(T.g, q, vals, T.acc, out);
+  }
+  return out;
+}
+
+// A thread per particle, those with more than LOG_WIDE candidates listed for a warp each in a second
+// launch: a serial walk of thousands of centres would be a tail of its own, and a small input with
+// wide supports would leave the chip idle.  Bound by L2's FP64 adds (eight a centre) and the walk's
+// FP64 arithmetic.  The whole call for the disc sampled by 1,000,003 particles (cubic) 1.49 ms, of
+// which 0.87 + 0.45 ms these two launches; 2.08 with a thread for every particle over the reference's
+// wider windows, one grid after the other.  25,000 / 150,000 / 700,000 particles 3.1 / 0.94 / 1.64 ms
+// (16.2 / 3.87 / 3.26).  LOG_WIDE 64 / 96 / 192 / 256 / 384 / 600: 1.79 / 1.69 / 1.51 / 1.50 / 1.49 /
+// 1.46 ms at 1,000,003 and 2.70 / 2.74 / 2.63 / 3.07 / 3.22 / 3.23 at 25,000.  LOG_B blocks an SM, 3 / 4 /
+// 5: 1.77 / 1.69 / 1.70 ms (at 96); the registers cap the rest.
+// Particles from n_narrow on are the second grid's (the coarser one of very wide particles).
+constexpr int LOG_WIDE = 256;
+constexpr int LOG_B = 4;
+__global__ void __launch_bounds__(128, LOG_B) k_deposit_log(
+    int64_t n, const unsigned long long* __restrict__ n_wide, const double* __restrict__ x,
+    const double* __restrict__ h, const double* __restrict__ m, const double* __restrict__ t,
+    const double* __restrict__ v, LogTarget fine, LogTarget coarse, int kid,
+    int32_t* __restrict__ list, unsigned long long* __restrict__ nlist) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t n_narrow = n_wide ? n - (int64_t)*n_wide : n;
+  double out = 0.0;
+  bool heavy = false;
+  if (p < n) {
+    const LogTarget& T = p < n_narrow ? fine : coarse;
+    const LogParticle q = log_particle(T.g, p, x, h);
+    heavy = (int64_t)(q.i_hi - q.i_lo + 1) * q.nj * q.nk > LOG_WIDE;
+    if (!heavy) {
+      const double o = log_one<1>(T, q, p, 0, m, t, v, kid);
+      if (p < n_narrow)
+        out = o;
+      else if (o != 0.0)
+        atomicAdd(coarse.outside, o);
+    }
+  }
+  const unsigned hm = __ballot_sync(FULL, heavy);
+  if (hm) {
+    unsigned long long at = 0;
+    if (lane == 0) at = atomicAdd(nlist, (unsigned long long)__popc(hm));
+    at = __shfl_sync(FULL, at, 0);
+    if (heavy) list[at + __popc(hm & ((1u << lane) - 1u))] = (int32_t)p;
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) out += __shfl_xor_sync(FULL, out, d);
+  if (lane == 0 && out != 0.0) atomicAdd(fine.outside, out);
+}
+
+__global__ void __launch_bounds__(128, LOG_B) k_deposit_log_heavy(
+    int64_t n, const unsigned long long* __restrict__ n_wide, const double* __restrict__ x,
+    const double* __restrict__ h, const double* __restrict__ m, const double* __restrict__ t,
+    const double* __restrict__ v, LogTarget fine, LogTarget coarse, int kid,
+    const int32_t* __restrict__ list, const unsigned long long* __restrict__ nlist) {
+  const int lane = threadIdx.x & 31;
+  const int64_t n_narrow = n_wide ? n - (int64_t)*n_wide : n;
+  const int64_t all = (int64_t)*nlist;
+  for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < all;
+       w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const int64_t p = list[w];
+    const LogTarget& T = p < n_narrow ? fine : coarse;
+    const double o = log_one<32>(T, log_particle(T.g, p, x, h), p, lane, m, t, v, kid);
+    if (o != 0.0) atomicAdd(T.outside, o);
+  }
 }
 
 // ---------------------------------------------------------------- Cartesian box
@@ -618,8 +751,7 @@ __global__ void k_grid_finish(int64_t ncell, const double* __restrict__ acc,
 }
 
 // render/gasgrid.py:757-788 (refine_sums): fine sums from the coarse sums' densities,
-// trilinear in index space (theta and r clamped, phi periodic), times the fine volume; the
-// fine mass is summed into msum for the rescaling
+// trilinear in index space (theta and r clamped, phi periodic), times the fine volume
 __device__ __forceinline__ void refine_axis(int i, int c, int nc, bool periodic, int& i0,
                                             int& i1, double& w) {
   double f = (i + 0.5) / c - 0.5;
@@ -640,8 +772,7 @@ __device__ __forceinline__ void refine_axis(int i, int c, int nc, bool periodic,
 
 __global__ void k_refine(const double* __restrict__ acc_c, const double* __restrict__ vc,
                          int nrc, int nthc, int nphc, const double* __restrict__ vf, int nr,
-                         int nth, int nph, int cr, int ct, int cp, double* __restrict__ out,
-                         double* msum) {
+                         int nth, int nph, int cr, int ct, int cp, double* __restrict__ out) {
   const int64_t cell = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (cell >= (int64_t)nr * nth * nph) return;
   const int k = (int)(cell % nph);
@@ -666,12 +797,17 @@ __global__ void k_refine(const double* __restrict__ acc_c, const double* __restr
   const double vfc = vf[(int64_t)i * nth + j];
 #pragma unroll
   for (int f = 0; f < DEP_FIELDS; ++f) out[cell * DEP_FIELDS + f] = s[f] * vfc;
-  atomicAdd(msum, s[0] * vfc);
 }
 
+// the sum of the first field (mass), one add per warp of a grid-stride pass
 __global__ void k_field_sum(int64_t ncell, const double* __restrict__ acc, double* sum) {
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c < ncell) atomicAdd(sum, acc[c * DEP_FIELDS]);
+  double v = 0.0;
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncell;
+       c += (int64_t)gridDim.x * blockDim.x)
+    v += acc[c * DEP_FIELDS];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(sum, v);
 }
 
 __global__ void k_refine_scale(int64_t nval, const double* __restrict__ sums, double* out) {
@@ -686,18 +822,27 @@ __global__ void k_refine_scale(int64_t nval, const double* __restrict__ sums, do
 // centre, so neighbouring threads add to neighbouring cells while those lines sit in L2 (in the
 // caller's order each atomic add of a large grid travels to DRAM).  Keys: the grid's own linear
 // cell index, with the out-of-grid cells clamped to one layer beyond each face.
-__global__ void k_dep_keys_log(int64_t n, const double* __restrict__ x, double r_min, double dlnr,
-                               double dth, double dph, int nr, int nth, int nph,
-                               unsigned long long* keys, int32_t* idx) {
+// With wide_cells > 0 the particles whose support spans that many fine angular cells or more
+// (render/gasgrid.py:751-754) come last, and are counted.
+__global__ void k_dep_keys_log(int64_t n, const double* __restrict__ x,
+                               const double* __restrict__ h, LogGeom g, double wide_cells,
+                               unsigned long long* keys, int32_t* idx,
+                               unsigned long long* __restrict__ n_wide) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const double xp = x[3 * p], yp = x[3 * p + 1], zp = x[3 * p + 2];
-  const double rr = sqrt(xp * xp + yp * yp + zp * zp);
-  const int i = min(max((int)floor(log(rr / r_min) / dlnr), -1), nr) + 1;
-  const int j = min(max((int)floor(acos(fmin(1.0, fmax(-1.0, zp / rr))) / dth), 0), nth - 1);
-  const int k = min(max((int)floor(py_mod(atan2(yp, xp), 2.0 * 3.141592653589793) / dph), 0), nph - 1);
-  keys[p] = ((unsigned long long)i * nth + j) * nph + k;
-  idx[p] = (int32_t)p;
+  bool wide = false;
+  if (p < n) {
+    const double xp = x[3 * p], yp = x[3 * p + 1], zp = x[3 * p + 2];
+    const double rr = sqrt(xp * xp + yp * yp + zp * zp);
+    const int i = min(max((int)floor(log(rr / g.r_min) / g.dlnr), -1), g.nr) + 1;
+    const int j = min(max((int)floor(acos(fmin(1.0, fmax(-1.0, zp / rr))) / g.dth), 0), g.nth - 1);
+    const int k = min(max((int)floor(azimuth(yp, xp) / g.dph), 0), g.nph - 1);
+    wide = wide_cells > 0.0 && 2.0 * h[p] >= wide_cells * fmax(rr, g.r_min) * g.dth;
+    const unsigned long long cells = (unsigned long long)(g.nr + 2) * g.nth * g.nph;
+    keys[p] = wide ? cells : ((unsigned long long)i * g.nth + j) * g.nph + k;
+    idx[p] = (int32_t)p;
+  }
+  const unsigned w = __ballot_sync(0xffffffffu, wide);
+  if (w && (threadIdx.x & 31) == 0) atomicAdd(n_wide, (unsigned long long)__popc(w));
 }
 
 __global__ void k_dep_gather(int64_t n, const int32_t* __restrict__ idx,
@@ -721,30 +866,61 @@ __global__ void k_dep_gather(int64_t n, const int32_t* __restrict__ idx,
   ts[q] = t[p];
 }
 
-void launch_deposit_keys(int64_t n, const double* x, const LogGeom& g, unsigned long long* keys,
-                         int32_t* idx, cudaStream_t st) {
-  if (n > 0)
-    count_launch(), k_dep_keys_log<<<grid_for(n), NB_THREADS, 0, st>>>(
-        n, x, g.r_min, g.dlnr, g.dth, g.dph, g.nr, g.nth, g.nph, keys, idx);
+// Inputs of this size on, and those split over two grids, are deposited in the spatial order of
+// their centres' cells (sorted keys, gathered copies of the particle data).
+constexpr int64_t DEPOSIT_SORT_MIN = 1 << 16;
+
+void launch_log_tables(const LogGeom& g, double* out, cudaStream_t st) {
+  const int64_t most = std::max<int64_t>(std::max<int64_t>(g.nph, g.nth), (int64_t)g.nr * g.nth);
+  count_launch(), k_log_tables<<<grid_for(most), NB_THREADS, 0, st>>>(g, out);
 }
 
-void launch_deposit_gather(int64_t n, const int32_t* idx, const double* x, const double* h,
-                           const double* m, const double* t, const double* v, double* out,
-                           cudaStream_t st) {
-  if (n > 0)
-    count_launch(), k_dep_gather<<<grid_for(n), NB_THREADS, 0, st>>>(n, idx, x, h, m, t, v, out);
+// scal: device doubles, the mass outside of each grid; ints: device words, the trilinear counts of
+// each grid, the number of wide particles and one for the walk; all and the sums zeroed by the caller
+int deposit_log(Engine& E, int64_t n, const double* x, const double* h, const double* m,
+                const double* t, const double* v, const LogGeom& fine, const LogGeom* coarse,
+                double wide_cells, int kid, double* acc, double* acc_c, double* scal,
+                unsigned long long* ints, cudaStream_t st) {
+  if (n <= 0) return 0;
+  NB_TRY(E.ensure_deposit(n));
+  const int nsh = fine.nr + DEP_INNER_VIRTUAL, nsh_c = coarse ? coarse->nr + DEP_INNER_VIRTUAL : 0;
+  NB_TRY(E.ensure_shells(nsh + nsh_c));
+  double2* shells = static_cast<double2*>(E.dep_shells);
+  count_launch(), k_log_shells<<<grid_for(nsh), NB_THREADS, 0, st>>>(fine, shells);
+  if (coarse) count_launch(), k_log_shells<<<grid_for(nsh_c), NB_THREADS, 0, st>>>(*coarse, shells + nsh);
+  if (coarse || n >= DEPOSIT_SORT_MIN) {
+    count_launch(), k_dep_keys_log<<<grid_for(n), NB_THREADS, 0, st>>>(
+        n, x, h, fine, coarse ? wide_cells : 0.0, E.dep_k0, E.dep_i0, ints + 2);
+    const unsigned long long max_key = (unsigned long long)(fine.nr + 2) * fine.nth * fine.nph;
+    int bits = 1;
+    while (bits < 64 && (1ull << bits) <= max_key) ++bits;
+    cub::DoubleBuffer<unsigned long long> kb(E.dep_k0, E.dep_k1);
+    cub::DoubleBuffer<int32_t> vb(E.dep_i0, E.dep_i1);
+    size_t tmp = E.cub_bytes;
+    NB_CUDA(cub::DeviceRadixSort::SortPairs(E.cub_tmp, tmp, kb, vb, (int)n, 0, bits, st));
+    count_launch(), k_dep_gather<<<grid_for(n), NB_THREADS, 0, st>>>(n, vb.Current(), x, h, m, t, v, E.dep_buf);
+    x = E.dep_buf;
+    h = E.dep_buf + 3 * n;
+    m = h + n;
+    t = m + n;
+    v = t + n;
+  }
+  const LogTarget a{fine, shells, acc, scal, ints};
+  const LogTarget b = coarse ? LogTarget{*coarse, shells + nsh, acc_c, scal + 1, ints + 1} : a;
+  int sms = 0;
+  NB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E.device));
+  const unsigned long long* n_wide = coarse ? ints + 2 : nullptr;
+  unsigned long long* nlist = ints + 3;
+  int32_t* list = reinterpret_cast<int32_t*>(E.dep_k0);  // the sort's keys are done with
+  count_launch(), k_deposit_log<<<grid_for(n, 128), 128, 0, st>>>(n, n_wide, x, h, m, t, v, a, b,
+                                                                    kid, list, nlist);
+  const unsigned gb = (unsigned)std::min<int64_t>(grid_for(n * 32, 128), (int64_t)sms * LOG_B);
+  count_launch(), k_deposit_log_heavy<<<gb, 128, 0, st>>>(n, n_wide, x, h, m, t, v, a, b, kid, list,
+                                                          nlist);
+  return 0;
 }
 
 // ---------------------------------------------------------------- launchers
-void launch_deposit_log(int64_t n, const double* x, const double* h, const double* m,
-                        const double* t, const double* v, const LogGeom& g, int kid,
-                        double* acc, double* outside, unsigned long long* n_tri,
-                        cudaStream_t st) {
-  if (n > 0)
-    count_launch(), k_deposit_log<<<grid_for(n, 128), 128, 0, st>>>(n, x, h, m, t, v, g, kid,
-                                                                      acc, outside, n_tri);
-}
-
 void launch_grid_finish(int64_t ncell, const double* acc, const double* vol, int64_t per,
                         double* mass, float* rho, float* t_mass, float* t_em, float* vel,
                         cudaStream_t st) {
@@ -758,8 +934,9 @@ void launch_refine_sums(const double* acc_c, const double* vol_c, int nrc, int n
                         double* out, double* sums2, cudaStream_t st) {
   const int64_t nf = (int64_t)nr * nth * nph, nc = (int64_t)nrc * nthc * nphc;
   count_launch(), k_refine<<<grid_for(nf), NB_THREADS, 0, st>>>(
-      acc_c, vol_c, nrc, nthc, nphc, vol_f, nr, nth, nph, cr, ct, cp, out, sums2);
-  count_launch(), k_field_sum<<<grid_for(nc), NB_THREADS, 0, st>>>(nc, acc_c, sums2 + 1);
+      acc_c, vol_c, nrc, nthc, nphc, vol_f, nr, nth, nph, cr, ct, cp, out);
+  count_launch(), k_field_sum<<<std::min(grid_for(nf), 1184u), NB_THREADS, 0, st>>>(nf, out, sums2);
+  count_launch(), k_field_sum<<<std::min(grid_for(nc), 1184u), NB_THREADS, 0, st>>>(nc, acc_c, sums2 + 1);
   count_launch(), k_refine_scale<<<grid_for(nf * DEP_FIELDS), NB_THREADS, 0, st>>>(
       nf * DEP_FIELDS, sums2, out);
 }

@@ -15,10 +15,15 @@ struct LogGeom {
   const double *sth, *cth, *dcth, *cph, *sph;  // theta / phi cell-centre tables
 };
 
-void launch_deposit_log(int64_t n, const double* x, const double* h, const double* m,
-                        const double* t, const double* v, const LogGeom& g, int kid,
-                        double* acc, double* outside, unsigned long long* n_tri,
-                        cudaStream_t st);
+void launch_log_tables(const LogGeom& g, double* out, cudaStream_t st);
+// the log grid's sums; with `coarse` the particles whose support spans wide_cells fine angular
+// cells or more go to acc_c instead.  scal[0, 1]: the mass outside of each grid, ints[0, 1]: the
+// trilinear counts, ints[2]: the wide particles, ints[3]: scratch (device words, zeroed with the
+// sums by the caller)
+int deposit_log(Engine& E, int64_t n, const double* x, const double* h, const double* m,
+                const double* t, const double* v, const LogGeom& fine, const LogGeom* coarse,
+                double wide_cells, int kid, double* acc, double* acc_c, double* scal,
+                unsigned long long* ints, cudaStream_t st);
 // the box' sums (acc, *outside and *n_tri zeroed by the caller); waits for the stream once
 int deposit_box(Engine& E, int64_t n, const double* x, const double* h, const double* m,
                 const double* t, const double* v, double x0, double y0, double z0, double dx,
@@ -31,13 +36,5 @@ void launch_grid_finish(int64_t ncell, const double* acc, const double* vol, int
 void launch_refine_sums(const double* acc_c, const double* vol_c, int nrc, int nthc, int nphc,
                         const double* vol_f, int nr, int nth, int nph, int cr, int ct, int cp,
                         double* out, double* sums2, cudaStream_t st);
-
-// spatial order of the particles on the log grid: keys and identity indices
-void launch_deposit_keys(int64_t n, const double* x, const LogGeom& g, unsigned long long* keys,
-                         int32_t* idx, cudaStream_t st);
-// out (9 n doubles): x (3n), h, m, t, v (3n) gathered in idx order
-void launch_deposit_gather(int64_t n, const int32_t* idx, const double* x, const double* h,
-                           const double* m, const double* t, const double* v, double* out,
-                           cudaStream_t st);
 
 }  // namespace nbk

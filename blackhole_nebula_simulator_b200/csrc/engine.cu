@@ -182,6 +182,16 @@ int Engine::ensure_deposit(int64_t n) {
   return ensure_cub(b);
 }
 
+int Engine::ensure_shells(int64_t m) {
+  Engine& E = *this;
+  if (m <= cap_shells && dep_shells) return 0;
+  if (dep_shells) cudaFree(dep_shells);
+  dep_shells = nullptr;
+  NB_CUDA(cudaMalloc(&dep_shells, 2 * sizeof(double) * m));
+  cap_shells = m;
+  return 0;
+}
+
 int Engine::ensure_bricks(int64_t nbricks) {
   Engine& E = *this;
   if (!dep_count) NB_CUDA(cudaMalloc((void**)&dep_count, 4 * sizeof(int64_t)));
@@ -212,7 +222,7 @@ void Engine::release() {
   void* ps[] = {dep_k0, dep_k1, dep_i0, dep_i1, dep_buf, d_err, bbox, bbox_part, keys_a, keys_b, vals_a, counts, node_lo, node_hi, sub_lo, sub_hi, node_q, sub_q,
                 cub_tmp, sort_keys, red, lists.perm, lists.inv_perm, lists.spos, lists.off,
                 lists.idx, d_rowmax, tidx, leaf_cbase, leaf_bbase, leaf_ibase, leaf_ncand, cands, masks, items, part_count,
-                dep_count, brick_count, brick_cursor, brick_off, brick_pairs, brick_tasks};
+                dep_shells, dep_count, brick_count, brick_cursor, brick_off, brick_pairs, brick_tasks};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (h_err) cudaFreeHost(h_err);

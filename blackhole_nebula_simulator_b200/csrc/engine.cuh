@@ -178,6 +178,9 @@ struct Engine {
   double* dep_buf = nullptr;
   int64_t dep_cap = 0;
   int ensure_deposit(int64_t n);
+  void* dep_shells = nullptr;  // the log grids' shells (radius of the centres, volume factor)
+  int64_t cap_shells = 0;
+  int ensure_shells(int64_t m);
   // the box' bricks of cells: counters, particles per brick, lists, tasks
   int64_t* dep_count = nullptr;
   unsigned long long* brick_count = nullptr;

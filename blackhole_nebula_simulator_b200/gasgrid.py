@@ -8,9 +8,9 @@ over the 8 nearest centres.  Weight beyond the grid goes to ``outside``, so grid
 = sum m for every particle.  ``deposit_log_split`` sends very wide particles to a coarser grid
 whose sums are interpolated back (render/gasgrid.py:741-808).
 
-The deposition is one warp per particle on the device (FP64 sums by atomic addition: the cell
-sums are the reference's to rounding, but their last bits depend on the order the warps
-arrive in); the cell fields are finished on the device too.  Inputs may be NumPy arrays or
+The deposition runs on the device (FP64 sums, in part by atomic addition: the cell sums are the
+reference's to rounding, but their last bits depend on the order the threads arrive in); the
+grids' tables are made and the cell fields finished on the device too.  Inputs may be NumPy arrays or
 CUDA tensors; the GasGrid fields are CUDA tensors.
 """
 
@@ -26,7 +26,7 @@ import torch
 
 from . import _lib
 from .config import KERNEL_IDS
-from .device import ctx, dev_f64, ptr, stream
+from .device import ctx, dev_f64, ptr, require_cuda, stream
 
 R_SUPPORT = 2.0
 MIN_KERNEL_CELLS = 8
@@ -139,36 +139,48 @@ def _check_kernel(kernel):
     return KERNEL_IDS[kernel]
 
 
-def _log_accumulate(x, h, m, t, v, g: LogSphericalGrid, kernel: str):
+def _geometry(g: LogSphericalGrid):
+    return (float(g.dlnr), float(g.dth), float(g.dph), int(g.nr), int(g.nth), int(g.nph))
+
+
+def _device_tables(g: LogSphericalGrid, device) -> torch.Tensor:
+    """``g.tables()`` (sth, cth, dcth, cph, sph) and then ``g.volumes()``, made on the device."""
+    size = 3 * g.nth + 2 * g.nph + g.nr * g.nth
+    tab = torch.empty(size, dtype=torch.float64, device=device)
+    _call("nb_log_tables", float(g.r_min), *_geometry(g), ptr(tab), stream())
+    return tab
+
+
+def _volumes(g: LogSphericalGrid, tab: torch.Tensor) -> torch.Tensor:
+    return tab[3 * g.nth + 2 * g.nph :]
+
+
+def _log_accumulate(x, h, m, t, v, g: LogSphericalGrid, kernel: str, tab: torch.Tensor):
     """Accumulated sums (nr, nth, nph, N_FIELDS), outside mass, trilinear count."""
     kid = _check_kernel(kernel)
     n, x, h, m, t, v = _inputs(x, h, m, t, v)
-    d = x.device
-    acc = torch.empty((*g.shape, N_FIELDS), dtype=torch.float64, device=d)
-    tab = {k: torch.as_tensor(a, dtype=torch.float64, device=d) for k, a in g.tables().items()}
+    acc = torch.empty((*g.shape, N_FIELDS), dtype=torch.float64, device=x.device)
+    at = [0, g.nth, 2 * g.nth, 3 * g.nth, 3 * g.nth + g.nph]  # sth, cth, dcth, cph, sph
     out = (ctypes.c_double * 1)()
     ntri = (ctypes.c_int64 * 1)()
     _call("nb_deposit_log", n, ptr(x), ptr(h), ptr(m), ptr(t), ptr(v), float(g.r_min),
-          float(g.dlnr), float(g.dth), float(g.dph), int(g.nr), int(g.nth), int(g.nph), kid,
-          ptr(tab["sth"]), ptr(tab["cth"]), ptr(tab["dcth"]), ptr(tab["cph"]), ptr(tab["sph"]),
-          ptr(acc), out, ntri, stream())  # fmt: skip
+          *_geometry(g), kid, *[ptr(tab[k:]) for k in at], ptr(acc), out, ntri,
+          stream())  # fmt: skip
     return acc, float(out[0]), int(ntri[0])
 
 
 def _finish(g, acc, vol, outside, n_tri) -> GasGrid:
-    """render/gasgrid.py:293-313 on the device; vol: (nr, nth) for the log grid (one volume per
-    theta row of a shell) or a scalar for a box."""
+    """render/gasgrid.py:293-313 on the device; vol: a device tensor (nr, nth) for the log grid (one
+    volume per theta row of a shell) or a scalar for a box."""
     d = acc.device
     ncell = acc.numel() // N_FIELDS
     mass = torch.empty(acc.shape[:-1], dtype=torch.float64, device=d)
     rho, t_mass, t_em = (torch.empty(acc.shape[:-1], dtype=torch.float32, device=d) for _ in range(3))
     vel = torch.empty((*acc.shape[:-1], 3), dtype=torch.float32, device=d)
-    if np.ndim(vol) == 0:
-        volt = torch.full((1,), float(vol), dtype=torch.float64, device=d)
-        per = ncell
+    if isinstance(vol, torch.Tensor):
+        volt, per = vol, acc.shape[2]  # cells of one (i, j) row share its volume
     else:
-        volt = torch.as_tensor(np.ascontiguousarray(vol), dtype=torch.float64, device=d)
-        per = acc.shape[2]  # cells of one (i, j) row share its volume
+        volt, per = torch.full((1,), float(vol), dtype=torch.float64, device=d), ncell
     _call("nb_grid_finish", ncell, ptr(acc), ptr(volt), int(per), ptr(mass), ptr(rho),
           ptr(t_mass), ptr(t_em), ptr(vel), stream())
     return GasGrid(g, mass, rho, t_mass, t_em, vel, float(outside), int(n_tri))
@@ -177,8 +189,10 @@ def _finish(g, acc, vol, outside, n_tri) -> GasGrid:
 def deposit_log(x, h, m, t, v, g: LogSphericalGrid, kernel: str = "wendland_c4") -> GasGrid:
     """render/gasgrid.py:722-738: deposition onto a log-spherical grid.  x (N, 3) positions; h
     (N,) smoothing lengths; m mass(es); t (N,) temperatures [K]; v (N, 3) velocities."""
-    acc, outside, n_tri = _log_accumulate(x, h, m, t, v, g, kernel)
-    return _finish(g, acc, g.volumes(), outside, n_tri)
+    _check_kernel(kernel)
+    tab = _device_tables(g, require_cuda())
+    acc, outside, n_tri = _log_accumulate(x, h, m, t, v, g, kernel, tab)
+    return _finish(g, acc, _volumes(g, tab), outside, n_tri)
 
 
 def deposit_box(x, h, m, t, v, b: CartesianBox, kernel: str = "wendland_c4") -> GasGrid:
@@ -217,8 +231,7 @@ def refine_sums(acc_c, gc: LogSphericalGrid, g: LogSphericalGrid, coarsen=COARSE
     interpolated trilinearly in index space at the fine centres, theta and r clamped, phi
     periodic, times the fine volume, scaled to the coarse grid's mass)."""
     out = torch.empty((*g.shape, N_FIELDS), dtype=torch.float64, device=acc_c.device)
-    vc = torch.as_tensor(gc.volumes(), dtype=torch.float64, device=acc_c.device)
-    vf = torch.as_tensor(g.volumes(), dtype=torch.float64, device=acc_c.device)
+    vc, vf = (_volumes(a, _device_tables(a, acc_c.device)) for a in (gc, g))
     cr, ct, cp = coarsen
     _call("nb_refine_sums", ptr(acc_c.contiguous()), ptr(vc), int(gc.nr), int(gc.nth), int(gc.nph),
           ptr(vf), int(g.nr), int(g.nth), int(g.nph), int(cr), int(ct), int(cp), ptr(out),
@@ -229,17 +242,36 @@ def refine_sums(acc_c, gc: LogSphericalGrid, g: LogSphericalGrid, coarsen=COARSE
 def deposit_log_split(x, h, m, t, v, g: LogSphericalGrid, kernel: str = "wendland_c4",
                       wide_cells: float = WIDE_CELLS, coarsen=COARSEN) -> GasGrid:  # fmt: skip
     """render/gasgrid.py:791-808: very wide particles on a coarser grid, interpolated back."""
+    kid = _check_kernel(kernel)
     n, x, h, m, t, v = _inputs(x, h, m, t, v)
-    wide = wide_particles(x, h, g, wide_cells)
-    nar = ~wide
-    total, outside, n_tri = _log_accumulate(x[nar], h[nar], m[nar], t[nar], v[nar], g, kernel)
-    n_wide = int(wide.sum())
-    if n_wide:
+    cr, ct, cp = coarsen
+    d = x.device
+    tab = _device_tables(g, d)
+    if min(coarsen) < 1 or g.nr % cr or g.nth % ct or g.nph % cp or g.nth // ct < 2 or not wide_cells > 0:
+        # no coarse grid to deposit on alongside: an error if a particle needs one
+        wide = wide_particles(x, h, g, wide_cells)
+        nar = ~wide
+        total, outside, n_tri = _log_accumulate(x[nar], h[nar], m[nar], t[nar], v[nar], g, kernel,
+                                                tab)  # fmt: skip
+        n_wide = int(wide.sum())
+        if n_wide:
+            gc = coarse_log_grid(g, coarsen)
+            acc_c, out_c, tri_c = _log_accumulate(x[wide], h[wide], m[wide], t[wide], v[wide], gc,
+                                                  kernel, _device_tables(gc, d))  # fmt: skip
+    else:
         gc = coarse_log_grid(g, coarsen)
-        acc_c, out_c, tri_c = _log_accumulate(x[wide], h[wide], m[wide], t[wide], v[wide], gc,
-                                              kernel)  # fmt: skip
+        tab_c = _device_tables(gc, d)
+        total = torch.empty((*g.shape, N_FIELDS), dtype=torch.float64, device=d)
+        acc_c = torch.empty((*gc.shape, N_FIELDS), dtype=torch.float64, device=d)
+        out, ntri, nw = (ctypes.c_double * 2)(), (ctypes.c_int64 * 2)(), (ctypes.c_int64 * 1)()
+        _call("nb_deposit_log_split", n, ptr(x), ptr(h), ptr(m), ptr(t), ptr(v), float(g.r_min),
+              *_geometry(g), *_geometry(gc), float(wide_cells), kid, ptr(tab), ptr(tab_c),
+              ptr(total), ptr(acc_c), out, ntri, nw, stream())  # fmt: skip
+        n_wide = int(nw[0])
+        (outside, out_c), (n_tri, tri_c) = out, ntri
+    if n_wide:
         total = total + refine_sums(acc_c, gc, g, coarsen)
         outside, n_tri = outside + out_c, n_tri + tri_c
-    grid = _finish(g, total, g.volumes(), outside, n_tri)
+    grid = _finish(g, total, _volumes(g, tab), outside, n_tri)
     grid.extra["n_wide"] = n_wide
     return grid

@@ -334,6 +334,21 @@ NB_API int nb_deposit_log(nb_ctx* ctx, int64_t n, const double* x, const double*
                    const double* sth, const double* cth, const double* dcth, const double* cph,
                    const double* sph, double* acc, double* outside, int64_t* n_trilinear,
                    void* stream);
+/* nb_log_tables: a grid's tables in device memory, in the order sin th_j, cos th_j, cos th_j1 -
+ * cos th_j2 (nth each), cos ph_k, sin ph_k (nph each), cell volumes (nr x nth)
+ * (render/gasgrid.py:125-129, 688-692): 3 nth + 2 nph + nr nth doubles. */
+NB_API int nb_log_tables(nb_ctx* ctx, double r_min, double dlnr, double dth, double dph, int nr,
+                   int nth, int nph, double* tables, void* stream);
+/* nb_deposit_log_split (render/gasgrid.py:751-754, 791-808): particles whose support 2 h spans
+ * wide_cells cells r dth of the fine grid or more go to the coarse grid's sums acc_c, the others to
+ * acc; tables and tables_c as nb_log_tables makes them; outside[2], n_trilinear[2]: fine, coarse;
+ * *n_wide the particles on the coarse grid. */
+NB_API int nb_deposit_log_split(nb_ctx* ctx, int64_t n, const double* x, const double* h,
+                   const double* m, const double* t, const double* v, double r_min, double dlnr,
+                   double dth, double dph, int nr, int nth, int nph, double dlnr_c, double dth_c,
+                   double dph_c, int nr_c, int nth_c, int nph_c, double wide_cells, int kernel_id,
+                   const double* tables, const double* tables_c, double* acc, double* acc_c,
+                   double* outside, int64_t* n_trilinear, int64_t* n_wide, void* stream);
 /* nb_deposit_box: a Cartesian box of nb^3 cells of edge dx from the corner (x0, y0, z0)
  * (render/gasgrid.py:534-597, 811-825). */
 NB_API int nb_deposit_box(nb_ctx* ctx, int64_t n, const double* x, const double* h,
