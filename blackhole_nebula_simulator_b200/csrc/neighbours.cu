@@ -427,9 +427,11 @@ __device__ __forceinline__ bool child_near(bool records, const QueryLeaf& q, con
 // one level (a frontier in shared memory, ascending) give the next level's nodes to test, 32 at
 // a time, one per lane; the leaves within reach give the sub-leaves to test the same way, and the
 // sub-leaves within reach are the leaf's candidate list (ascending, since every frontier is).  A
-// leaf whose frontier outgrows its buffer goes to the list `wide`, for k_lists_wide.
-// Latency bound (a dependent chain of box loads per level): 0.14 ms on the 1M torus, 0.54 on the
-// 4M torus, 0.04 on the 262,144-particle cloud.  With 64-byte boxes in double, and the few leaves
+// leaf whose frontier outgrows its buffer goes to the list `wide`, for k_lists_wide.  A sub-leaf is
+// within reach if one of the leaf's own sub-leaves is: 32 particles along the curve rarely fill
+// their box, so this costs 0.04 ms here and saves 0.16 + 0.06 ms of passes 2 and 3 (1M torus).
+// Latency bound (a dependent chain of box loads per level): 0.18 ms on the 1M torus,
+// 0.04 on the 262,144-particle cloud.  With 64-byte boxes in double, and the few leaves
 // with large frontiers walked node by node by their warps, twice, 1.34, 2.3 and 0.04 ms.
 constexpr int CAND_WARPS = 4;
 #ifndef CAND_SMEM
@@ -458,6 +460,10 @@ __global__ void __launch_bounds__(CAND_WARPS * 32) k_lists_cand(
     const int64_t leaf = (int64_t)(order[t] & 0xffffffffull);
     const QueryLeaf q = query_leaf(tv, leaf);
     const Box32 qb = ld_box(tv.q + leaf);
+    Box32 own[LEAF / SUB];
+#pragma unroll
+    for (int i = 0; i < LEAF / SUB; ++i)
+      own[i] = ld_box(sq + min(leaf * (LEAF / SUB) + i, nsub - 1));
     // level by level from the root; `cur` holds the frontier (ascending node indices)
     int cur = 0, fn = 1;
     bool over = false;
@@ -480,7 +486,17 @@ __global__ void __launch_bounds__(CAND_WARPS * 32) k_lists_cand(
         int32_t child = 0;
         if (c < total) {
           child = front[cur][c / fan] * fan + c % fan;
-          hit = child < csize && child_near(records, q, qb, clo, chi, cq, coff + child);
+          if (lvl == 0 && records) {
+            // the leaf's box holds more than its own sub-leaves do
+            hit = false;
+            if (child < csize) {
+              const Box32 cb = ld_box(sq + child);
+#pragma unroll
+              for (int i = 0; i < LEAF / SUB; ++i) hit = hit || box_near(own[i], cb);
+            }
+          } else {
+            hit = child < csize && child_near(records, q, qb, clo, chi, cq, coff + child);
+          }
         }
         const unsigned mk = __ballot_sync(FULL, hit);
         if (nn + __popc(mk) > CAND_SMEM) {
@@ -638,9 +654,10 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 // Pass 2: the tests, on each work item's batches of candidates.  Each batch's final hit masks go
 // to masks[(batch base + b) * 32 + lane], the item's entries per row to part_count and, added up,
 // to counts (zeroed before).  Bound by issue (71 %) and by the broadcast loads of the staged
-// candidates (LSU 69 %): 0.98 ms on the 1M torus, 3.96 on the 4M torus.  Two candidates per packed
-// instruction, the whole batch unrolled, two blocks per SM (three spill); with scalar tests and a
-// warp alone on its leaf whatever the leaf's number of batches, 1.30 and 4.0 ms.
+// candidates (LSU 69 %, but four rows by eight candidates a lane, with a quarter of those loads,
+// gain 1 %): 0.83 ms on the 1M torus.  Two candidates per packed instruction, the whole batch
+// unrolled, two blocks per SM (three spill); with scalar tests, a warp alone on its leaf whatever the
+// leaf's number of batches and candidates by the leaf's box alone, 1.30 ms.
 #ifndef TEST_BLOCKS_PER_SM
 #define TEST_BLOCKS_PER_SM 2
 #endif
@@ -780,92 +797,69 @@ __global__ void __launch_bounds__(NB_THREADS, TEST_BLOCKS_PER_SM) k_lists_test(
   }
 }
 
-// Pass 3: masks -> CSR entries.  One warp per work item, lane r on row r.  The batches come in order, four masks of
-// a row loaded at a time; each lane appends the entries of its mask's set bits (candidates
-// ascending) to a ring of its row in shared memory, whose slots are the entries' final positions
-// modulo 64, so the ring holds aligned stretches of 32 entries.  As soon as a row's stretch is
-// full the warp writes it with one store of 128 aligned bytes; an item's first and last stretches
-// of a row are written in part.  A lane appends at most 32 entries per batch to at most 31 pending
-// ones, so it never laps its ring.
-// Bound by issue (66 % active at 19 warps per SM, about 3 warp instructions per entry): 0.78 ms on
-// the 1M torus (160M entries), 22 us on a 4,096-particle cloud.  A scan over the batches' counts and
-// a binary search per entry, a warp per leaf, took 0.88 ms and 154 us; lanes that run ahead
-// through the masks of eight batches before the rings are emptied 0.92 ms.
+// Pass 3: masks -> CSR entries.  One warp per work item, EXPAND_BATCHES batches at a time, in order:
+// lane c holds candidate c of each batch, and for every row with a hit in them the lanes whose bit
+// is set in the row's mask store their candidates at the row's next positions (a bit's rank in
+// the mask), so a row's entries come ascending.
+// Bound by issue, about ten instructions per row and batch: 0.65 ms on the 1M torus (160M entries),
+// 0.52 on a 400,000-particle Wendland torus, 12 us on a 4,096-particle cloud.  Each lane appending a
+// row's entries to a ring in shared memory that the warp empties in aligned stretches of 32 took
+// 0.78, 0.75 ms and 22 us (fewer stores, but a loop over the longest of 32 masks).  Batches at a
+// time 2 / 4 / 8: 0.65 / 0.65 / 0.68 ms.  The candidates culled by sub-leaf (pass 1) leave 0.59, 0.51 ms, 12 us.
 constexpr int EXPAND_WARPS = 4;
-constexpr int EXPAND_RING = 64;
-constexpr int EXPAND_STRIDE = EXPAND_RING + 1;  // lanes on the same slot of 32 rows: 32 banks
+constexpr int EXPAND_BATCHES = 4;
 
 __global__ void __launch_bounds__(EXPAND_WARPS * 32) k_lists_expand(
     int64_t n, int64_t nitems, const int32_t* __restrict__ cands, ListSlices ls,
     const uint32_t* __restrict__ masks, const uint32_t* __restrict__ part_count,
     const int64_t* __restrict__ off, int32_t* __restrict__ idx, int* err) {
-  __shared__ int32_t ring_s[EXPAND_WARPS][32 * EXPAND_STRIDE];
-  __shared__ int32_t ids_s[EXPAND_WARPS][4][32];  // the candidates of four batches
+  __shared__ __align__(16) uint32_t mask_s[EXPAND_WARPS][EXPAND_BATCHES * 32];
   const unsigned FULL = 0xffffffffu;
   const int64_t t = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= nitems) return;  // warp-uniform
   const int64_t leaf = (int64_t)(ls.items[t] & 0xffffffffull), part = (int64_t)(ls.items[t] >> 32);
-  int32_t* rings = ring_s[threadIdx.x >> 5];
-  int32_t* ring = rings + lane * EXPAND_STRIDE;
-  int32_t(*ids)[32] = ids_s[threadIdx.x >> 5];
+  uint32_t* ms = mask_s[threadIdx.x >> 5];
   const int32_t* cand = cands + ls.cbase[leaf];
   const uint32_t* mask = masks + ls.bbase[leaf] * 32 + lane;
   const int64_t ncand = ls.ncand[leaf], nbat = (ncand + 3) / 4;
   const int64_t b_beg = part * ls.chunk, b_end = min(nbat, b_beg + ls.chunk);
   const int64_t k0 = leaf * LEAF;
   const int rows = (int)(n - k0 < LEAF ? n - k0 : LEAF);
-  // positions relative to the leaf's first one, rounded down to a stretch
-  const int64_t base = off[k0] & ~(int64_t)31;
+  const int64_t base = off[k0];  // positions are relative to the leaf's first one
   if (off[k0 + rows] - base > 0x7fffffc0ll) {  // beyond 32-bit positions within one leaf
     if (lane == 0) set_error(err, ERR_LIST_OVERFLOW);
     return;
   }
   int32_t* out = idx + base;
-  int first = lane < rows ? (int)(off[k0 + lane] - base) : 0;
-  for (int64_t p = part; p > 0; --p) first += (int)part_count[(t - p) * 32 + lane];  // earlier items
-  int w = first;           // next position of the row
-  int done = first & ~31;  // first position of the stretch being filled
-  for (int64_t b0 = b_beg; b0 < b_end; b0 += 4) {
-    uint32_t mm[4];
-    int32_t id[4];
+  int w = lane < rows ? (int)(off[k0 + lane] - base) : 0;  // next position of the row
+  for (int64_t p = part; p > 0; --p) w += (int)part_count[(t - p) * 32 + lane];  // earlier items
+  const unsigned below = (1u << lane) - 1u;
+  for (int64_t b0 = b_beg; b0 < b_end; b0 += EXPAND_BATCHES) {
+    uint32_t some = 0u;
+    int32_t id[EXPAND_BATCHES];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < EXPAND_BATCHES; ++u) {
       const bool in = b0 + u < b_end;
       const int64_t c = 4 * (b0 + u) + (lane >> 3);
-      mm[u] = in ? __ldcs(mask + (b0 + u) * 32) : 0u;
+      const uint32_t m = in ? __ldcs(mask + (b0 + u) * 32) : 0u;
       id[u] = in && c < ncand ? cand[c] * SUB + (lane & 7) : 0;
+      ms[lane * EXPAND_BATCHES + u] = m;
+      some |= m;
     }
     __syncwarp();
+    for (unsigned left = __ballot_sync(FULL, some != 0u); left; left &= left - 1) {
+      const int r = __ffs(left) - 1;
+      int at = __shfl_sync(FULL, w, r);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) ids[u][lane] = id[u];
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      uint32_t m = mm[u];
-      while (m) {
-        ring[w & (EXPAND_RING - 1)] = ids[u][__ffs(m) - 1];
-        m &= m - 1u;
-        w += 1;
+      for (int u = 0; u < EXPAND_BATCHES; ++u) {
+        const uint32_t m = ms[r * EXPAND_BATCHES + u];
+        if (m >> lane & 1u) out[at + __popc(m & below)] = id[u];
+        at += __popc(m);
       }
-      __syncwarp();
-      for (unsigned full = __ballot_sync(FULL, w - done >= 32); full; full &= full - 1) {
-        const int r = __ffs(full) - 1;
-        const int p = __shfl_sync(FULL, done, r) + lane;
-        if (p >= __shfl_sync(FULL, first, r))
-          out[p] = rings[r * EXPAND_STRIDE + (p & (EXPAND_RING - 1))];
-        if (lane == r) done += 32;
-      }
-      __syncwarp();
+      if (lane == r) w = at;
     }
-  }
-  // the last stretches
-  for (unsigned some = __ballot_sync(FULL, w > done); some; some &= some - 1) {
-    const int r = __ffs(some) - 1;
-    const int p = __shfl_sync(FULL, done, r) + lane;
-    const bool mine = p >= __shfl_sync(FULL, first, r);
-    if (p < __shfl_sync(FULL, w, r) && mine)
-      out[p] = rings[r * EXPAND_STRIDE + (p & (EXPAND_RING - 1))];
+    __syncwarp();
   }
   if (b_end == nbat && lane < rows && w != (int)(off[k0 + lane + 1] - base))
     set_error(err, ERR_LIST_OVERFLOW);
