@@ -854,6 +854,16 @@ static int rows_sorted(Engine& E, int64_t n, int64_t nrows, const int64_t* rows,
     *count = W.rs_count;  // the active rows, sorted already on these lists
     return 0;
   }
+  if (W.all_rows(n, nrows, rows)) {  // every position, on any lists
+    launch_iota(n, W.rows_s, st);
+    NB_CUDA(cudaMemsetAsync(W.m_sorted, 1, n, st));
+    *count = nrows;
+    W.rs_ver = W.rows_ver;
+    W.rs_gen = E.lists.gen;
+    W.rs_n = nrows;
+    W.rs_count = nrows;
+    return 0;
+  }
   NB_CUDA(cudaMemsetAsync(W.m_x, 0, n, st));
   count_launch(), k_mask_rows<<<grid_for(nrows), NB_THREADS, 0, st>>>(nrows, rows, n, W.m_x, E.d_err);
   count_launch(), k_sorted_mask<<<grid_for(n), NB_THREADS, 0, st>>>(n, E.lists.perm, W.m_x, W.m_sorted);
@@ -925,6 +935,14 @@ static int read_int(Engine& E, int* d, int* out, cudaStream_t st) {
   NB_TRY(pending_enqueue(E, st));
   NB_CUDA(host_sync(st));
   *out = E.ws.h_int[0];
+  return pending_finish(E, st);
+}
+
+int read_word(Engine& E, const int64_t* d, int64_t* out, cudaStream_t st) {
+  NB_CUDA(cudaMemcpyAsync(E.ws.h_i64, d, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  NB_TRY(pending_enqueue(E, st));
+  NB_CUDA(host_sync(st));
+  *out = E.ws.h_i64[0];
   return pending_finish(E, st);
 }
 
@@ -1045,7 +1063,7 @@ static int reuse_limits(Engine& E, int64_t n, const double* x, const uint8_t* ma
   return 0;
 }
 
-// sim/sph.py:329-387 (compute_density) for `rows` (caller order, W.rows is NOT used here): reuse
+// sim/sph.py:329-387 (compute_density) for `rows` (caller order; W.rows if every particle is active): reuse
 // the cached lists while provably complete, else rebuild with search h_guess * skin and double
 // the search of rows whose root lies beyond it, up to 12 rounds.  h (in/out, caller order) is the
 // guess for every particle; rows get their solved h, and rho / omega.

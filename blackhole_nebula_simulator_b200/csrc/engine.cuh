@@ -71,6 +71,11 @@ struct Workspace {
   // W.rows (the active rows of the current step) changes version whenever it is rewritten; the
   // sorted copy in rows_s is kept while the rows and the lists stay the same
   int64_t rows_ver = 0, rs_ver = -1, rs_gen = -1, rs_n = -1, rs_count = 0;
+  // the version of W.rows that holds every particle, ascending
+  int64_t all_ver = -1;
+  bool all_rows(int64_t n, int64_t nrows, const int64_t* r) const {
+    return r == rows && nrows == n && all_ver == rows_ver;
+  }
   // the rows' interacting entries in E.tidx / i32a, written by the force pass of these rows
   // (rows version, lists generation, row count), for the level choice that follows
   int64_t tight_ver = -1, tight_gen = -1, tight_n = -1;
