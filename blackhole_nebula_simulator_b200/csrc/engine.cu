@@ -946,17 +946,29 @@ int read_word(Engine& E, const int64_t* d, int64_t* out, cudaStream_t st) {
   return pending_finish(E, st);
 }
 
-// Density pass of `rows` on the current lists with the given search radii; results into the
-// caller-order arrays h_out, rho, omega and the scratch flags/iters.
+// Density pass of `rows` (`mask`, caller order) on the current lists with the given search radii;
+// results into the caller-order arrays h_out, rho, omega and the scratch flags/iters.
 static int density_on_lists(Engine& E, int64_t n, const double* x, const double* mass,
                             const double* h_start, const double* h_search, int64_t nrows,
-                            const int64_t* rows, const nb_params* prm, double* h_out,
-                            double* rho, double* omega, cudaStream_t st) {
+                            const int64_t* rows, const uint8_t* mask, const nb_params* prm,
+                            double* h_out, double* rho, double* omega, cudaStream_t st) {
   Workspace& W = E.ws;
   Lists& L = E.lists;
   if (nrows == 0) return 0;
-  int64_t ns = 0;
-  NB_TRY(rows_sorted(E, n, nrows, rows, &ns, st));
+  const int64_t* rows_d = W.rows_s;
+  if (W.all_rows(n, nrows, rows)) {
+    int64_t ns = 0;
+    NB_TRY(rows_sorted(E, n, nrows, rows, &ns, st));
+  } else {
+    // the rows are the mask's (their number is known), sorted beside the active rows' copy, which
+    // the force pass then finds still valid: nine launches less per block step on reused lists (20
+    // steps of 300,000 particles 15.6 -> 14.9 ms)
+    count_launch(), k_sorted_mask<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, mask, W.m_smark);
+    size_t tmp = E.cub_bytes;
+    NB_CUDA(cub::DeviceSelect::Flagged(E.cub_tmp, tmp, thrust::counting_iterator<int64_t>(0), W.m_smark,
+                                       W.i_tmp, W.d_i64 + 4, (int)n, st));
+    rows_d = W.i_tmp;
+  }
   DensityParams dp{prm->kernel_id, prm->cnorm, prm->eta, prm->tol, prm->h_max};
   if (prm->precision == 1) {
     // grid over the box of the last list build (cells clamp to it; the edge is derived on the
@@ -964,7 +976,7 @@ static int density_on_lists(Engine& E, int64_t n, const double* x, const double*
     count_launch(), k_pack_density32<<<grid_for(n), NB_THREADS, 0, st>>>(
         n, L.perm, x, mass, h_start, h_search, E.bbox, W.d_a, W.d_b, W.d_c, W.pk32);
     E.prof.begin(st);
-    launch_density32<int32_t>(nrows, W.rows_s, W.pk32, E.bbox, W.d_a, W.d_b, W.d_c, L.off,
+    launch_density32<int32_t>(nrows, rows_d, W.pk32, E.bbox, W.d_a, W.d_b, W.d_c, L.off,
                               L.idx, dp, L.perm, h_out, rho, omega, W.iters, W.flags,
                               E.prof.on ? W.pairs : nullptr, st);
   } else {
@@ -972,7 +984,7 @@ static int density_on_lists(Engine& E, int64_t n, const double* x, const double*
         n, L.perm, mass, h_start, h_search, W.d_a, W.d_b, W.d_c);
     count_launch(), k_pack_sorted<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, x, mass, W.pk0);
     E.prof.begin(st);
-    launch_density64<int32_t>(nrows, W.rows_s, W.pk0, W.d_a, W.d_b, W.d_c, L.off, L.idx, dp,
+    launch_density64<int32_t>(nrows, rows_d, W.pk0, W.d_a, W.d_b, W.d_c, L.off, L.idx, dp,
                               L.perm, h_out, rho, omega, W.iters, W.flags,
                               E.prof.on ? W.pairs : nullptr, st);
   }
@@ -1085,7 +1097,7 @@ int compute_density(Engine& E, int64_t n, const double* x, const double* mass, d
     int ok = 0;
     NB_TRY(reuse_limits(E, n, x, mask, first_fail, &ok, st));
     if (ok) {
-      NB_TRY(density_on_lists(E, n, x, mass, W.d_hg, W.d_heff, nrows, rows, prm, h, rho, omega, st));
+      NB_TRY(density_on_lists(E, n, x, mass, W.d_hg, W.d_heff, nrows, rows, mask, prm, h, rho, omega, st));
       NB_CUDA(cudaMemsetAsync(W.d_int, 0, sizeof(int), st));
       count_launch(), k_count_flag2<<<grid_for(nrows), NB_THREADS, 0, st>>>(nrows, rows, W.flags, W.d_int);
       int grow_n = 0;
@@ -1102,7 +1114,7 @@ int compute_density(Engine& E, int64_t n, const double* x, const double* mass, d
   for (int round = 0; round < 12; ++round) {
     NB_TRY(build_lists(E, n, x, W.d_hs, st));
     *builds += 1;
-    NB_TRY(density_on_lists(E, n, x, mass, W.d_hg, W.d_hs, nrows, rows, prm, h, rho, omega, st));
+    NB_TRY(density_on_lists(E, n, x, mass, W.d_hg, W.d_hs, nrows, rows, mask, prm, h, rho, omega, st));
     NB_CUDA(cudaMemsetAsync(W.d_int, 0, sizeof(int), st));
     count_launch(), k_grow<<<grid_for(nrows), NB_THREADS, 0, st>>>(nrows, rows, W.flags, h, W.d_hs, W.d_hg, W.d_int);
     int grow_n = 0;
