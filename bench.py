@@ -39,23 +39,23 @@ FP64_NOMINAL_TFLOPS = FP32_NOMINAL_TFLOPS / 2.0
 FLOP_PER_DENSITY_EVAL = 25.0  # distance + kernel + two sums per pair evaluation
 FLOP_PER_FORCE_PAIR = 75.0  # pressure + viscosity + P dV (+20 with disc viscosity)
 # DRAM bytes (read + write) per row of one launch, from ncu captures (cold caches) of the FP32
-# kernels on the 1,048,576-particle torus, scaled to a launch by its rows: density 199.9 MB over
-# 195,200 rows; forces (walk + pair launches) 1,347 + 1,007 MB over 1,045,504 rows; a list build
-# (candidate, test and expansion passes of a build after the start, 163 entries per row)
-# 1,273 MB over 1,048,576 particles
-DRAM_BYTES_PER_ROW = {"forces": 2251.0, "density": 1024.0, "lists": 1214.0}
+# kernels on the 1,048,576-particle torus, scaled to a launch by its rows: density 209.5 MB over
+# 214,784 rows; forces (walk + pair launches) 2,106 + 994 MB over 1,048,576 rows; a list build
+# (candidate, test and expansion passes of a build after the start) 1,483 MB over 1,048,576
+# particles
+DRAM_BYTES_PER_ROW = {"forces": 2956.0, "density": 975.0, "lists": 1415.0}
 # What the ncu counters of the same captures show limits each kernel (the roofline's ceiling
 # stays the HBM copy bandwidth; none of these kernels is a contraction)
 LIMITER = {
-    "lists": "issue: the test pass at 80 % issue active (FMA 45 %, ALU 42 %), the expansion at "
-             "64 %; the candidate pass latency bound (long-scoreboard 3.2 per issue at 24 % warp "
-             "occupancy); DRAM 0.1-9 % of peak",
+    "lists": "issue: the test pass at 60 % issue active (24 % warp occupancy, 120 registers; ALU 44 %, "
+             "FMA 23 %), the expansion at 73 %; the candidate pass latency bound (52 % issue active at "
+             "30 % warp occupancy); DRAM 0.5-23 % of peak",
     "cooling": "issue and shared-memory latency: 39 % issue active at 24 % warp occupancy (128 "
                "registers), tensor pipe 19.5 %, FP64 pipe 6.4 % (the check)",
-    "density": "latency: long-scoreboard stalls 4.2 per issue on the gathered records, 66 % "
-               "issue active at 43 % warp occupancy, DRAM 8 % of peak",
-    "forces": "latency: the walk launch stalls 11.5 per issue on the gathered records (DRAM 21 %); "
-              "the pair launch runs the FMA pipe at 36 % with 43 % warp occupancy",
+    "density": "issue: 74-77 % issue active at 50 % warp occupancy, ALU 44 %, FMA 32 %, DRAM 11 % of "
+               "peak",
+    "forces": "issue and the gathers' latency: the walk launch 61 % issue active (DRAM 26 %); the "
+              "pair launch 72 % issue active, FMA pipe 41 %, with 43 % warp occupancy",
     "flow": "FP64 pipe 69-71 % (the double-precision flow update), DRAM 25-29 %",
 }
 
