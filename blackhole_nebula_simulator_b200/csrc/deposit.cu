@@ -82,7 +82,7 @@ __global__ void k_log_tables(LogGeom g, double* __restrict__ out) {
 
 // One particle's candidate centres: a block of shells, theta rows and phi columns that holds every
 // centre inside its support, from the support's angular radius asin(2h / r) and the widest
-// azimuth asin(2h / (r sin theta)) of that cap, both a hair wide.
+// azimuth asin(2h / (r sin theta)) of that cap, both wider than acos and asin round (1.5e-8 at worst).
 struct LogParticle {
   double x, y, z, h, rr, th, ph;
   int i_lo, i_hi, j0, nj, k0, nk;
@@ -108,15 +108,17 @@ __device__ __forceinline__ LogParticle log_particle(const LogGeom& g, int64_t p,
   if (s < 1.0) {
     // log(1 + s) <= s, log(1 - s) >= -s / (1 - s)
     const double fr = log(q.rr / g.r_min) / g.dlnr;
-    q.i_hi = (int)floor(fmin(fr + s / g.dlnr + 1e-6, (double)i_max));
-    q.i_lo = (int)floor(fmax(fr - s / ((1.0 - s) * g.dlnr) - 1e-6, -(double)DEP_INNER_VIRTUAL)) - 1;
-    const double a = asin(s) + 1e-9, st = sqrt(q.x * q.x + q.y * q.y) / q.rr;
-    q.j0 = max(0, (int)floor((q.th - a) / g.dth - 0.5));
-    q.nj = min(g.nth - 1, (int)ceil((q.th + a) / g.dth - 0.5)) - q.j0 + 1;
+    q.i_hi = (int)floor(fmin(fr + s / g.dlnr - 0.5 + 1e-6, (double)i_max));
+    q.i_lo = (int)ceil(fmax(fr - s / ((1.0 - s) * g.dlnr) - 0.5 - 1e-6, -(double)DEP_INNER_VIRTUAL));
+    const double a = asin(s) + 1e-7, st = sqrt(q.x * q.x + q.y * q.y) / q.rr;
+    q.j0 = max(0, (int)ceil((q.th - a) / g.dth - 0.5));
+    q.nj = max(0, min(g.nth - 1, (int)floor((q.th + a) / g.dth - 0.5)) - q.j0 + 1);
     if (s < st * (1.0 - 1e-6)) {
-      const double d = asin(s / st) + 1e-9;
-      const int k0 = (int)floor((q.ph - d) / g.dph - 0.5), k1 = (int)ceil((q.ph + d) / g.dph - 0.5);
-      if (k1 - k0 + 1 < g.nph) {
+      const double d = asin(s / st) + 1e-7;
+      const int k0 = (int)ceil((q.ph - d) / g.dph - 0.5), k1 = (int)floor((q.ph + d) / g.dph - 0.5);
+      if (k1 < k0) {
+        q.nj = 0;
+      } else if (k1 - k0 + 1 < g.nph) {
         q.k0 = k0;
         q.nk = k1 - k0 + 1;
       }
@@ -234,7 +236,7 @@ template <int SIZE>
 __device__ __forceinline__ double log_one(const LogTarget& T, const LogParticle& q, int64_t p,
                                           int rank, const double* __restrict__ m,
                                           const double* __restrict__ t,
-                                          const double* __restrict__ v, int kid) {
+                                          const double* __restrict__ v, int kid, bool& tri) {
   double vals[DEP_FIELDS];
   particle_vals(p, m, t, v, vals);
   double wsum = 0.0, out = 0.0;
@@ -248,7 +250,7 @@ __device__ __forceinline__ double log_one(const LogTarget& T, const LogParticle&
   if (n_in >= DEP_MIN_CELLS) {
     log_pass<1>(T.g, T.shells, q, rank, SIZE, kid, 1.0 / wsum, vals, T.acc, wsum, n_in, out);
   } else if (rank == 0) {
-    atomicAdd(T.n_tri, 1ull);
+    tri = true;
     log_trilinear(T.g, q, vals, T.acc, out);
   }
   return out;
@@ -257,16 +259,16 @@ __device__ __forceinline__ double log_one(const LogTarget& T, const LogParticle&
 // A thread per particle, those with more than LOG_WIDE candidates listed for a warp each in a second
 // launch: a serial walk of thousands of centres would be a tail of its own, and a small input with
 // wide supports would leave the chip idle.  Bound by L2's FP64 adds (eight a centre) and the walk's
-// FP64 arithmetic.  The whole call for the disc sampled by 1,000,003 particles (cubic) 1.49 ms, of
-// which 0.87 + 0.45 ms these two launches; 2.08 with a thread for every particle over the reference's
-// wider windows, one grid after the other.  25,000 / 150,000 / 700,000 particles 3.1 / 0.94 / 1.64 ms
-// (16.2 / 3.87 / 3.26).  LOG_WIDE 64 / 96 / 192 / 256 / 384 / 600: 1.79 / 1.69 / 1.51 / 1.50 / 1.49 /
-// 1.46 ms at 1,000,003 and 2.70 / 2.74 / 2.63 / 3.07 / 3.22 / 3.23 at 25,000.  LOG_B blocks an SM, 3 / 4 /
-// 5: 1.77 / 1.69 / 1.70 ms (at 96); the registers cap the rest.
+// FP64 arithmetic.  The whole call for the disc sampled by 1,000,003 particles (cubic) 0.90 ms; 2.08
+// with a thread for every particle over the reference's wider windows, one grid after the other, and
+// 1.51 with an atomic count per particle beyond the kernel's reach and candidate boxes a centre wider
+// on each side.  20,000 / 150,000 / 2,000,000 particles 1.1 / 0.73 / 1.35 ms (8.1 / 3.87 / 2.38).
+// LOG_WIDE 64 / 128 / 256 differ by 2 % but for 50,000 Wendland particles: 1.56 / 1.60 / 1.71 ms.  Blocks
+// an SM of the first launch, 4 / 5 / 6: 0.905 / 0.894 / 0.926 ms at 1,000,003.
 // Particles from n_narrow on are the second grid's (the coarser one of very wide particles).
-constexpr int LOG_WIDE = 256;
-constexpr int LOG_B = 4;
-__global__ void __launch_bounds__(128, LOG_B) k_deposit_log(
+constexpr int LOG_WIDE = 128;
+constexpr int LOG_B = 4;  // blocks an SM of the second launch
+__global__ void __launch_bounds__(128, 5) k_deposit_log(
     int64_t n, const unsigned long long* __restrict__ n_wide, const double* __restrict__ x,
     const double* __restrict__ h, const double* __restrict__ m, const double* __restrict__ t,
     const double* __restrict__ v, LogTarget fine, LogTarget coarse, int kid,
@@ -276,13 +278,13 @@ __global__ void __launch_bounds__(128, LOG_B) k_deposit_log(
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t n_narrow = n_wide ? n - (int64_t)*n_wide : n;
   double out = 0.0;
-  bool heavy = false;
+  bool heavy = false, tri = false;
   if (p < n) {
     const LogTarget& T = p < n_narrow ? fine : coarse;
     const LogParticle q = log_particle(T.g, p, x, h);
     heavy = (int64_t)(q.i_hi - q.i_lo + 1) * q.nj * q.nk > LOG_WIDE;
     if (!heavy) {
-      const double o = log_one<1>(T, q, p, 0, m, t, v, kid);
+      const double o = log_one<1>(T, q, p, 0, m, t, v, kid, tri);
       if (p < n_narrow)
         out = o;
       else if (o != 0.0)
@@ -296,9 +298,15 @@ __global__ void __launch_bounds__(128, LOG_B) k_deposit_log(
     at = __shfl_sync(FULL, at, 0);
     if (heavy) list[at + __popc(hm & ((1u << lane) - 1u))] = (int32_t)p;
   }
+  // one count per warp and grid: an atomic per particle on one address would bound the small supports
+  const unsigned tf = __ballot_sync(FULL, tri && p < n_narrow), tc = __ballot_sync(FULL, tri && p >= n_narrow);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) out += __shfl_xor_sync(FULL, out, d);
-  if (lane == 0 && out != 0.0) atomicAdd(fine.outside, out);
+  if (lane == 0) {
+    if (out != 0.0) atomicAdd(fine.outside, out);
+    if (tf) atomicAdd(fine.n_tri, (unsigned long long)__popc(tf));
+    if (tc) atomicAdd(coarse.n_tri, (unsigned long long)__popc(tc));
+  }
 }
 
 __global__ void __launch_bounds__(128, LOG_B) k_deposit_log_heavy(
@@ -313,7 +321,9 @@ __global__ void __launch_bounds__(128, LOG_B) k_deposit_log_heavy(
        w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     const int64_t p = list[w];
     const LogTarget& T = p < n_narrow ? fine : coarse;
-    const double o = log_one<32>(T, log_particle(T.g, p, x, h), p, lane, m, t, v, kid);
+    bool tri = false;
+    const double o = log_one<32>(T, log_particle(T.g, p, x, h), p, lane, m, t, v, kid, tri);
+    if (tri) atomicAdd(T.n_tri, 1ull);
     if (o != 0.0) atomicAdd(T.outside, o);
   }
 }

@@ -1,6 +1,6 @@
 """The log-spherical deposition's walks of the candidate centres against the CPU oracle.
 
-A particle with up to LOG_WIDE (256) candidates is one thread's, the others a warp's; supports here
+A particle with up to LOG_WIDE (128) candidates is one thread's, the others a warp's; supports here
 run from less than a cell (trilinear) to past the origin, on both sides of that line, on the poles,
 across phi = 0 and beyond both ends of the radii.  Split grids put the wide particles on a second
 grid in the same launches.
