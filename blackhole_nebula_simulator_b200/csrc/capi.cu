@@ -537,7 +537,8 @@ int nb_log_tables(nb_ctx* ctx, double r_min, double dlnr, double dth, double dph
                   int nph, double* tables, void* stream) {
   NB_TRY(begin(ctx));
   Engine& E = ctx->E;
-  if (!log_grid_ok(r_min, dlnr, nr, nth, nph))
+  // any grid that has cells: one theta row is enough for volumes (a refined grid's), not for a deposit
+  if (nr < 1 || nth < 1 || nph < 1)
     return nbk::set_host_error(E, "bad log-spherical grid"), NB_ERR_INPUT;
   nbk::launch_log_tables(log_geom(r_min, dlnr, dth, dph, nr, nth, nph, tables), tables, S(stream));
   NB_CUDA(cudaGetLastError());
