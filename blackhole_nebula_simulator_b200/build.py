@@ -27,6 +27,7 @@ SOURCES = {
     "sph32.cu": True,
     "gravity.cu": False,
     "engine.cu": False,
+    "scratch.cu": False,
     "steps.cu": False,
     "capi.cu": False,
     "noalloc.cu": False,

@@ -880,6 +880,14 @@ __global__ void k_dep_gather(int64_t n, const int32_t* __restrict__ idx,
 // their centres' cells (sorted keys, gathered copies of the particle data).
 constexpr int64_t DEPOSIT_SORT_MIN = 1 << 16;
 
+size_t deposit_cub_bytes(int64_t n) {
+  size_t b = 0;
+  cub::DeviceRadixSort::SortPairs((void*)nullptr, b, (unsigned long long*)nullptr,
+                                  (unsigned long long*)nullptr, (int32_t*)nullptr,
+                                  (int32_t*)nullptr, (int)n);
+  return b;
+}
+
 void launch_log_tables(const LogGeom& g, double* out, cudaStream_t st) {
   const int64_t most = std::max<int64_t>(std::max<int64_t>(g.nph, g.nth), (int64_t)g.nr * g.nth);
   count_launch(), k_log_tables<<<grid_for(most), NB_THREADS, 0, st>>>(g, out);

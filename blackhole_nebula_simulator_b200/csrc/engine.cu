@@ -21,217 +21,6 @@
 
 namespace nbk {
 
-// the reuse test looks at the TOPK = 65 largest displacements (its fast sets hold at most 64)
-constexpr int TOPK = 65;
-constexpr int TOPK_CHUNK = 2048;
-
-// ---------------------------------------------------------------- workspace
-template <typename T>
-static int grow(Engine& E, T*& p, int64_t& cap, int64_t want) {
-  if (want <= cap && p) return 0;
-  int64_t c = std::max<int64_t>(want + want / 4, 1024);
-  if (p) cudaFree(p);
-  p = nullptr;
-  NB_CUDA(cudaMalloc((void**)&p, sizeof(T) * (size_t)c));
-  cap = c;
-  return 0;
-}
-
-int Engine::ensure_cub(size_t bytes) {
-  Engine& E = *this;
-  if (bytes <= cub_bytes && cub_tmp) return 0;
-  if (cub_tmp) cudaFree(cub_tmp);
-  cub_tmp = nullptr;
-  size_t b = bytes + bytes / 4 + 4096;
-  NB_CUDA(cudaMalloc(&cub_tmp, b));
-  cub_bytes = b;
-  return 0;
-}
-
-int Engine::ensure_n(int64_t n) {
-  Engine& E = *this;
-  if (!d_err) {
-    NB_CUDA(cudaMalloc((void**)&d_err, sizeof(int) * 4));
-    NB_CUDA(cudaMemset(d_err, 0, sizeof(int) * 4));
-    NB_CUDA(cudaMallocHost((void**)&h_err, sizeof(int) * 4));
-    NB_CUDA(cudaMalloc((void**)&bbox, sizeof(double) * 8));
-    NB_CUDA(cudaMallocHost((void**)&h_red, sizeof(double) * 64));
-    NB_CUDA(cudaMalloc((void**)&d_rowmax, 16 * sizeof(unsigned long long)));
-    NB_CUDA(cudaMallocHost((void**)&h_build, sizeof(int64_t) * 4));
-  }
-  if (n <= cap_n && keys_a) return 0;
-  int64_t c = std::max<int64_t>(n + n / 4, 1024);
-  auto fr = [](void* p) {
-    if (p) cudaFree(p);
-  };
-  fr(bbox_part); fr(keys_a); fr(keys_b); fr(vals_a); fr(counts); fr(red);
-  fr(lists.perm); fr(lists.inv_perm); fr(lists.spos); fr(lists.off);
-  NB_CUDA(cudaMalloc((void**)&bbox_part, sizeof(double) * 6 * 1184));
-  NB_CUDA(cudaMalloc((void**)&keys_a, sizeof(uint64_t) * c));
-  NB_CUDA(cudaMalloc((void**)&keys_b, sizeof(uint64_t) * c));
-  NB_CUDA(cudaMalloc((void**)&vals_a, sizeof(int32_t) * c));
-  NB_CUDA(cudaMalloc((void**)&counts, sizeof(int64_t) * (c + 1)));
-  NB_CUDA(cudaMalloc((void**)&red, sizeof(double) * 16 * 1184));
-  NB_CUDA(cudaMalloc((void**)&lists.perm, sizeof(int32_t) * c));
-  NB_CUDA(cudaMalloc((void**)&lists.inv_perm, sizeof(int32_t) * c));
-  NB_CUDA(cudaMalloc((void**)&lists.spos, sizeof(double4) * c));
-  NB_CUDA(cudaMalloc((void**)&lists.off, sizeof(int64_t) * (c + 1)));
-  cap_n = c;
-  lists.n = 0;
-  return ensure_cub(cub_bytes_needed(c, 0));
-}
-
-int Prof::ensure() {
-  if (ev[0]) return 0;
-  for (int k = 0; k < 2 * POOL; ++k)
-    if (cudaEventCreate(&ev[k]) != cudaSuccess) return -2;
-  if (cudaMalloc((void**)&d_pairs, sizeof(unsigned long long) * PROF_NCAT) != cudaSuccess) return -2;
-  if (cudaMemset(d_pairs, 0, sizeof(unsigned long long) * PROF_NCAT) != cudaSuccess) return -2;
-  return 0;
-}
-
-int Engine::ensure_nodes(int64_t m) { return grow2(m); }
-
-int Engine::grow2(int64_t m) {
-  Engine& E = *this;
-  if (m <= cap_nodes && node_lo) return 0;
-  int64_t c = std::max<int64_t>(m + m / 4, 256);
-  if (node_lo) cudaFree(node_lo);
-  if (node_hi) cudaFree(node_hi);
-  if (node_q) cudaFree(node_q);
-  NB_CUDA(cudaMalloc(&node_q, 32 * c));
-  NB_CUDA(cudaMalloc((void**)&node_lo, sizeof(double4) * c));
-  NB_CUDA(cudaMalloc((void**)&node_hi, sizeof(double4) * c));
-  cap_nodes = c;
-  return 0;
-}
-
-int Engine::ensure_sub(int64_t m) {
-  Engine& E = *this;
-  if (m <= cap_sub && sub_lo) return 0;
-  int64_t c = std::max<int64_t>(m + m / 4, 256);
-  if (sub_lo) cudaFree(sub_lo);
-  if (sub_hi) cudaFree(sub_hi);
-  if (sub_q) cudaFree(sub_q);
-  NB_CUDA(cudaMalloc(&sub_q, 32 * c));
-  NB_CUDA(cudaMalloc((void**)&sub_lo, sizeof(double4) * c));
-  NB_CUDA(cudaMalloc((void**)&sub_hi, sizeof(double4) * c));
-  cap_sub = c;
-  return 0;
-}
-
-int Engine::ensure_list_capacity(int64_t m) {
-  Engine& E = *this;
-  NB_TRY(grow(E, lists.idx, cap_list, std::max<int64_t>(m, 1)));
-  return 0;
-}
-
-int Engine::ensure_tight(int64_t m) {
-  Engine& E = *this;
-  return grow(E, tidx, cap_tidx, std::max<int64_t>(m, 1));
-}
-
-int Engine::ensure_leaves(int64_t m) {
-  Engine& E = *this;
-  if (m <= cap_leaf && leaf_cbase) return 0;
-  int64_t c = 0;
-  NB_TRY(grow(E, leaf_cbase, c, m));
-  c = 0;
-  NB_TRY(grow(E, leaf_bbase, c, m));
-  c = 0;
-  NB_TRY(grow(E, leaf_ibase, c, m));
-  c = 0;
-  NB_TRY(grow(E, leaf_ncand, c, m));
-  cap_leaf = c;
-  return 0;
-}
-
-int Engine::ensure_tiles(int64_t ncand, int64_t nbatch, int64_t nitem) {
-  Engine& E = *this;
-  NB_TRY(grow(E, cands, cap_cands, std::max<int64_t>(ncand, 1)));
-  NB_TRY(grow(E, masks, cap_masks, std::max<int64_t>(nbatch * 32, 32)));
-  if (nitem <= cap_items && items) return 0;
-  int64_t c = 0;
-  NB_TRY(grow(E, items, c, nitem));
-  cap_items = c;
-  c = 0;
-  return grow(E, part_count, c, cap_items * 32);
-}
-
-int Engine::ensure_deposit(int64_t n) {
-  Engine& E = *this;
-  if (n > dep_cap || !dep_buf) {
-    void* ps[] = {dep_k0, dep_k1, dep_i0, dep_i1, dep_buf};
-    for (void* p : ps)
-      if (p) cudaFree(p);
-    dep_k0 = dep_k1 = nullptr;
-    dep_i0 = dep_i1 = nullptr;
-    dep_buf = nullptr;
-    const int64_t c = std::max<int64_t>(n + n / 4, 1024);
-    NB_CUDA(cudaMalloc((void**)&dep_k0, sizeof(unsigned long long) * c));
-    NB_CUDA(cudaMalloc((void**)&dep_k1, sizeof(unsigned long long) * c));
-    NB_CUDA(cudaMalloc((void**)&dep_i0, sizeof(int32_t) * c));
-    NB_CUDA(cudaMalloc((void**)&dep_i1, sizeof(int32_t) * c));
-    NB_CUDA(cudaMalloc((void**)&dep_buf, sizeof(double) * 12 * c));
-    dep_cap = c;
-  }
-  size_t b = 0;
-  cub::DeviceRadixSort::SortPairs((void*)nullptr, b, (unsigned long long*)nullptr,
-                                  (unsigned long long*)nullptr, (int32_t*)nullptr,
-                                  (int32_t*)nullptr, (int)dep_cap);
-  return ensure_cub(b);
-}
-
-int Engine::ensure_shells(int64_t m) {
-  Engine& E = *this;
-  if (m <= cap_shells && dep_shells) return 0;
-  if (dep_shells) cudaFree(dep_shells);
-  dep_shells = nullptr;
-  NB_CUDA(cudaMalloc(&dep_shells, 2 * sizeof(double) * m));
-  cap_shells = m;
-  return 0;
-}
-
-int Engine::ensure_bricks(int64_t nbricks) {
-  Engine& E = *this;
-  if (!dep_count) NB_CUDA(cudaMalloc((void**)&dep_count, 4 * sizeof(int64_t)));
-  if (nbricks <= cap_bricks && brick_off) return 0;
-  int64_t c = 0;
-  NB_TRY(grow(E, brick_count, c, nbricks));
-  c = 0;
-  NB_TRY(grow(E, brick_cursor, c, nbricks));
-  c = 0;
-  NB_TRY(grow(E, brick_off, c, nbricks + 1));
-  cap_bricks = nbricks;
-  return 0;
-}
-
-int Engine::ensure_brick_lists(int64_t pairs, int64_t tasks) {
-  Engine& E = *this;
-  NB_TRY(grow(E, brick_pairs, cap_brick_pairs, pairs));
-  return grow(E, brick_tasks, cap_brick_tasks, tasks);
-}
-
-int Engine::ensure_sort_keys(int64_t m) {
-  Engine& E = *this;
-  NB_TRY(grow(E, sort_keys, cap_sort, m));
-  return ensure_cub(cub_bytes_needed(cap_n, m));
-}
-
-void Engine::release() {
-  void* ps[] = {dep_k0, dep_k1, dep_i0, dep_i1, dep_buf, d_err, bbox, bbox_part, keys_a, keys_b, vals_a, counts, node_lo, node_hi, sub_lo, sub_hi, node_q, sub_q,
-                cub_tmp, sort_keys, red, lists.perm, lists.inv_perm, lists.spos, lists.off,
-                lists.idx, d_rowmax, tidx, leaf_cbase, leaf_bbase, leaf_ibase, leaf_ncand, cands, masks, items, part_count,
-                dep_shells, dep_count, brick_count, brick_cursor, brick_off, brick_pairs, brick_tasks};
-  for (void* p : ps)
-    if (p) cudaFree(p);
-  if (h_err) cudaFreeHost(h_err);
-  if (h_build) cudaFreeHost(h_build);
-  prof.release();
-  if (h_red) cudaFreeHost(h_red);
-  ws.release();
-}
-
 int check_device_error(Engine& E, cudaStream_t st) {
   NB_CUDA(cudaMemcpyAsync(E.h_err, E.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
   NB_CUDA(host_sync(st));
@@ -720,91 +509,14 @@ __global__ void k_max_rows(int64_t nrows, const int64_t* __restrict__ rows, cons
 }
 
 // ---------------------------------------------------------------- cache + density
-int Workspace::ensure(Engine& E, int64_t n) {
-  if (n <= cap && d_a) return 0;
-  release();
-  int64_t c = std::max<int64_t>(n + n / 4, 1024);
-  double** dd[] = {&d_a, &d_b, &d_c, &d_hg, &d_hs, &d_heff, &d_hlim, &d_disp, &d_P, &d_cs,
-                   &d_vsig, &d_ddudt, &d_dm, &d_tmp, &d_uh};
-  for (double** p : dd) NB_CUDA(cudaMalloc((void**)p, sizeof(double) * c));
-  double** d3[] = {&v_flow, &v_pred, &v_eval, &v_dacc, &v_tmp};
-  for (double** p : d3) NB_CUDA(cudaMalloc((void**)p, sizeof(double) * 3 * c));
-  double4** d4[] = {&pk0, &pk1, &pk2, &pk3};
-  for (double4** p : d4) NB_CUDA(cudaMalloc((void**)p, sizeof(double4) * c));
-  NB_CUDA(cudaMalloc((void**)&pk32, sizeof(float4) * 2 * c));
-  NB_CUDA(cudaMalloc((void**)&pf1, sizeof(float4) * 2 * c));
-  float4** f4s[] = {&pf2, &pf3};
-  for (float4** p : f4s) NB_CUDA(cudaMalloc((void**)p, sizeof(float4) * c));
-  int64_t** i8[] = {&rows, &rows_s, &rows2, &iters, &flags, &need, &i_tmp, &pairs, &i_lvl, &i_tmp2};
-  for (int64_t** p : i8) NB_CUDA(cudaMalloc((void**)p, sizeof(int64_t) * (c + 1)));
-  uint8_t** u1[] = {&m_rows, &m_done, &m_need, &m_tmp, &m_x, &m_sorted, &m_smark};
-  for (uint8_t** p : u1) NB_CUDA(cudaMalloc((void**)p, c));
-  NB_CUDA(cudaMalloc((void**)&i32a, sizeof(int32_t) * c));
-  NB_CUDA(cudaMalloc((void**)&i32b, sizeof(int32_t) * c));
-  NB_CUDA(cudaMalloc((void**)&dk_b, sizeof(double) * c));
-  const int64_t tk = (c / TOPK_CHUNK + 2) * TOPK;
-  NB_CUDA(cudaMalloc((void**)&tk_key0, sizeof(unsigned long long) * tk));
-  NB_CUDA(cudaMalloc((void**)&tk_key1, sizeof(unsigned long long) * tk));
-  NB_CUDA(cudaMalloc((void**)&tk_idx0, sizeof(int32_t) * tk));
-  NB_CUDA(cudaMalloc((void**)&tk_idx1, sizeof(int32_t) * tk));
-  NB_CUDA(cudaMalloc((void**)&d_int, sizeof(int) * 16));
-  NB_CUDA(cudaMalloc((void**)&d_i64, sizeof(int64_t) * 16));
-  NB_CUDA(cudaMallocHost((void**)&h_int, sizeof(int) * 16));
-  NB_CUDA(cudaMallocHost((void**)&h_i64, sizeof(int64_t) * 16));
-  NB_CUDA(cudaMallocHost((void**)&h_dbl, sizeof(double) * 80));
-  NB_CUDA(cudaMalloc((void**)&d_scal_i, sizeof(int64_t) * 16));
-  d_scal = reinterpret_cast<double*>(d_scal_i + 8);
-  NB_CUDA(cudaMallocHost((void**)&h_scal, sizeof(int64_t) * 16));
-  cap = c;
-  if (cache.cap < c) {
-    if (cache.x_ref) cudaFree(cache.x_ref);
-    if (cache.hs) cudaFree(cache.hs);
-    NB_CUDA(cudaMalloc((void**)&cache.x_ref, sizeof(double) * 3 * c));
-    NB_CUDA(cudaMalloc((void**)&cache.hs, sizeof(double) * c));
-    cache.cap = c;
-    cache.valid = false;
-  }
-  size_t need = cub_bytes_needed(c, 0);
-  size_t a = 0;
+// temporary storage of the runtime's sorts, selections and reductions over n particles
+size_t workspace_cub_bytes(int64_t n) {
+  size_t a = 0, b = 0, d = 0;
   cub::DeviceRadixSort::SortPairsDescending((void*)nullptr, a, (double*)nullptr, (double*)nullptr,
-                                            (int32_t*)nullptr, (int32_t*)nullptr, (int)c);
-  size_t b = 0;
-  cub::DeviceReduce::Min((void*)nullptr, b, (int64_t*)nullptr, (int64_t*)nullptr, (int)c);
-  size_t d = 0;
-  cub::DeviceReduce::Sum((void*)nullptr, d, (double*)nullptr, (double*)nullptr, (int)c);
-  return E.ensure_cub(std::max(std::max(need, a), std::max(b, d)) + 4096);
-}
-
-int Workspace::ensure_grad(Engine& E, int64_t n) {
-  if (n <= gcap && gvel) return 0;
-  if (pk4) cudaFree(pk4);
-  if (gvel) cudaFree(gvel);
-  if (gvel32) cudaFree(gvel32);
-  pk4 = nullptr;
-  gvel = nullptr;
-  gvel32 = nullptr;
-  gcap = 0;
-  const int64_t c = std::max<int64_t>(cap, n);
-  NB_CUDA(cudaMalloc((void**)&pk4, sizeof(double4) * c));
-  NB_CUDA(cudaMalloc((void**)&gvel, sizeof(double) * 9 * c));
-  NB_CUDA(cudaMalloc((void**)&gvel32, sizeof(float) * 9 * c));
-  gcap = c;
-  return 0;
-}
-
-void Workspace::release() {
-  void* ps[] = {pk4, gvel, gvel32, d_a, d_b, d_c, d_hg, d_hs, d_heff, d_hlim, d_disp, d_P, d_cs, d_vsig, d_ddudt,
-                d_dm, d_tmp, d_uh, v_flow, v_pred, v_eval, v_dacc, v_tmp, pk0, pk1, pk2, pk3, pk32,
-                pf1, pf2, pf3, m_x, m_sorted, m_smark,
-                rows, rows_s, rows2, iters, flags, need, i_tmp, pairs, i_lvl, i_tmp2, m_rows, m_done, m_need,
-                m_tmp, i32a, i32b, dk_b, d_int, d_i64, tk_key0, tk_key1, tk_idx0, tk_idx1, d_scal_i};
-  for (void* p : ps)
-    if (p) cudaFree(p);
-  if (h_int) cudaFreeHost(h_int);
-  if (h_i64) cudaFreeHost(h_i64);
-  if (h_dbl) cudaFreeHost(h_dbl);
-  if (h_scal) cudaFreeHost(h_scal);
-  *this = Workspace{cache};
+                                            (int32_t*)nullptr, (int32_t*)nullptr, (int)n);
+  cub::DeviceReduce::Min((void*)nullptr, b, (int64_t*)nullptr, (int64_t*)nullptr, (int)n);
+  cub::DeviceReduce::Sum((void*)nullptr, d, (double*)nullptr, (double*)nullptr, (int)n);
+  return std::max(std::max(cub_bytes_needed(n, 0), a), std::max(b, d)) + 4096;
 }
 
 // sum of a[rows] into E.ws.h_i64[0] (profiling only)

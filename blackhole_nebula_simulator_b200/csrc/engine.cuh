@@ -14,6 +14,9 @@
 namespace nbk {
 
 constexpr int MAX_LEVELS = 16;
+// the reuse test looks at the TOPK = 65 largest displacements (its fast sets hold at most 64)
+constexpr int TOPK = 65;
+constexpr int TOPK_CHUNK = 2048;
 
 // Symmetric lists of the last build, in sorted (Hilbert-curve) order: row k belongs to the particle
 // perm[k] of the caller's order; entries are sorted positions.
@@ -172,7 +175,7 @@ struct Engine {
   double4* sub_hi = nullptr;
   void *node_q = nullptr, *sub_q = nullptr;  // the boxes' 32-byte records of the candidate walk
   int64_t cap_sub = 0;
-  void* cub_tmp = nullptr;
+  void* cub_tmp = nullptr;  // null or cub_bytes large
   size_t cub_bytes = 0;
   int64_t* sort_keys = nullptr;
   // particle -> grid deposition: spatial sort keys / indices (double buffers) and the gathered
@@ -229,7 +232,6 @@ struct Engine {
 
   int ensure_n(int64_t n);
   int ensure_nodes(int64_t m);
-  int grow2(int64_t m);
   int ensure_sub(int64_t m);
   int ensure_list_capacity(int64_t m);
   int ensure_sort_keys(int64_t m);
@@ -238,7 +240,11 @@ struct Engine {
   void release();
 };
 
+// temporary storage of the library's sorts and scans: lists of n particles (m exported entries), the
+// step runtime, the log grid's deposition
 size_t cub_bytes_needed(int64_t n, int64_t m);
+size_t workspace_cub_bytes(int64_t n);
+size_t deposit_cub_bytes(int64_t n);
 struct MlpHull;
 // learned cooling (mlp.cu): u_out = cooled u of n particles (dt per particle or dt_scalar)
 int mlp_cool(Engine& E, int64_t n, const double* u, const double* rho, const double* dt,

@@ -536,14 +536,18 @@ BremsParams brems_of_mlp(const nb_mlp_params* mp) {
 
 int mlp_state(Engine& E, MlpState** out) {
   MlpState& M = g_mlp_state[E.device & 63];
-  if (!M.w) {
-    NB_CUDA(cudaMalloc((void**)&M.w, sizeof(float) * MLP_NPARAM));
-    NB_CUDA(cudaMemset(M.w, 0, sizeof(float) * MLP_NPARAM));
-    NB_CUDA(cudaMalloc((void**)&M.stats, sizeof(double) * 3));
-    NB_CUDA(cudaMemset(M.stats, 0, sizeof(double) * 3));
-    NB_CUDA(cudaMalloc((void**)&M.counts, sizeof(unsigned long long) * 2));
-    NB_CUDA(cudaMemset(M.counts, 0, sizeof(unsigned long long) * 2));
-  }
+  // each by itself: what an allocation that failed left out, the next call makes
+  auto zeroed = [&E](auto*& p, size_t bytes) -> int {
+    void* got = nullptr;
+    if (p) return 0;
+    NB_CUDA(cudaMalloc(&got, bytes));
+    p = static_cast<std::remove_reference_t<decltype(p)>>(got);
+    NB_CUDA(cudaMemset(got, 0, bytes));
+    return 0;
+  };
+  NB_TRY(zeroed(M.w, sizeof(float) * MLP_NPARAM));
+  NB_TRY(zeroed(M.stats, sizeof(double) * 3));
+  NB_TRY(zeroed(M.counts, sizeof(unsigned long long) * 2));
   *out = &M;
   return 0;
 }

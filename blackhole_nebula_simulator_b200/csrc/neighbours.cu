@@ -1051,6 +1051,7 @@ int build_lists(Engine& E, int64_t n, const double* pos, const double* hs, cudaS
   }
   Lists& L = E.lists;
   L.gen += 1;
+  L.n = 0;  // no lists until these are whole
   E.prof.begin(st);
   // bounding box and Hilbert keys
   int nbb = (int)std::min<int64_t>(grid_for(n), 1184);
