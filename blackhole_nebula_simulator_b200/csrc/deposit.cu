@@ -134,16 +134,17 @@ __device__ __forceinline__ LogParticle log_particle(const LogGeom& g, int64_t p,
 
 // render/gasgrid.py:316-412 (_nb_log_kernel_pass) over those candidates, dealt to `size` threads:
 // MODE 0 sums f V and counts the centres inside the support, MODE 1 adds the normalised weights
-// and the mass beyond the grid.  q < 2 is decided on d^2 against (2h)^2 with a relative margin of
-// 1e-12 (sqrt(d^2) / h only inside the margin); the weights take q = sqrt(d^2) (1 / h), within an ulp
-// of the reference's quotient.
+// and the mass beyond the grid.  d^2 is a few fused operations from (rc sin th) cos ph - x and its
+// like, as the reference forms them: within 12 u |d| (r + |d|), u = 2^-53.  A centre ten times that
+// close to (2h)^2 is decided by the reference's own arithmetic, which counts it for the kernel's or
+// the trilinear weights; the weights take q = sqrt(d^2) (1 / h), within rounding of its quotient.
 template <int MODE>
 __device__ __forceinline__ void log_pass(const LogGeom& g, const double2* __restrict__ shells,
                                          const LogParticle& q, int rank, int size, int kid,
                                          double inv, const double* vals, double* acc,
                                          double& wsum, int& n_in, double& outside) {
   const double big = 2.0 * q.h, big2 = big * big;
-  const double in2 = big2 * (1.0 - 1e-12), out2 = big2 * (1.0 + 1e-12);
+  const double edge = 1e-12 * big2 + 1.4e-14 * big * q.rr, in2 = big2 - edge, out2 = big2 + edge;
   const double ih = 1.0 / q.h;
   const int dj = size / q.nk, dk = size % q.nk;
   int j = q.j0 + rank / q.nk, c = rank % q.nk;
@@ -162,9 +163,12 @@ __device__ __forceinline__ void log_pass(const LogGeom& g, const double2* __rest
         const double dxc = fma(sh.x, ux, -q.x), dyc = fma(sh.x, uy, -q.y), dzc = fma(sh.x, cth, -q.z);
         const double dd = fma(dzc, dzc, fma(dyc, dyc, dxc * dxc));
         if (dd >= out2) continue;
-        const double r = sqrt(dd);
-        if (dd >= in2 && !(r / q.h < 2.0)) continue;
-        const double f = kernel_f<double>(r * ih, kid) * (sh.y * dvol);
+        if (dd >= in2) {
+          const double rst = sh.x * sth;
+          const double ex = rst * cph - q.x, ey = rst * sph - q.y, ez = sh.x * cth - q.z;
+          if (!(sqrt(d2_exact(ex, ey, ez)) / q.h < 2.0)) continue;
+        }
+        const double f = kernel_f<double>(sqrt(dd) * ih, kid) * (sh.y * dvol);
         if (MODE == 0) {
           n_in += 1;
           wsum += f;
