@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(128, LOG_B) k_deposit_log_heavy(
 //   k_box_weights   a warp (a block for the wide ones) per listed particle: the kernel sum, the
 //                   part of it outside the box, the trilinear fallback below 8 centres; the
 //                   record of the particle and the number of particles per brick of 8^3 cells
-//   k_box_fill      the bricks' particle lists
+//   k_box_lists     the bricks' particle lists, BOX_PAIRS entries at a time
 //   k_box_bricks    a block per brick and stretch of its list, a warp per 2 x 4 x 4 cells, a cell
 //                   per lane, the six sums in registers: no atomic add per (particle, cell)
 // Bound by the FP64 pipe (a kernel value per lane of every sub-brick a support reaches, about a
@@ -356,6 +356,10 @@ constexpr int BRICK_STAGE = 128;    // records staged in shared memory at a time
 constexpr int BRICK_CHUNK = 512;    // records of one block's stretch of a brick's list
 constexpr int BOX_REC = 12;         // doubles per record: x, y, z, h, 1/h, -, six weighted fields
 constexpr int BOX_WIDE = 16384;     // candidate cells from which a block takes the particle
+
+// Entries of the bricks' lists held at once (1 GiB): twice what a frame of ten million particles
+// of twenty-odd bricks each needs, so only supports far wider than a brick are taken in parts.
+constexpr int64_t BOX_PAIRS = int64_t(1) << 28;
 
 struct BoxGeom {
   double x0, y0, z0, dx;
@@ -605,19 +609,24 @@ __global__ void k_box_tasks(int64_t nbricks, const unsigned long long* __restric
   for (unsigned k = 0; k < nt; ++k) tasks[at + k] = make_int2((int)b, (int)k);
 }
 
-__global__ void __launch_bounds__(NB_THREADS) k_box_fill(
-    int64_t n, BoxGeom g, const unsigned long long* __restrict__ nlist,
-    const double* __restrict__ rec, const int64_t* __restrict__ brick_off,
-    unsigned* __restrict__ cursor, int32_t* __restrict__ pairs) {
+// the work list's entries [w0, w1): counted per brick (a part of the list), or put in its list
+template <bool FILL>
+__global__ void __launch_bounds__(NB_THREADS) k_box_lists(
+    int64_t n, BoxGeom g, int64_t w0, int64_t w1, const unsigned long long* __restrict__ nlist,
+    const double* __restrict__ rec, unsigned long long* __restrict__ count,
+    const int64_t* __restrict__ brick_off, unsigned* __restrict__ cursor, int32_t* __restrict__ pairs) {
   const int lane = threadIdx.x & 31;
-  const int64_t small = (int64_t)nlist[0], all = small + (int64_t)nlist[1];
-  for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < all;
+  const int64_t small = (int64_t)nlist[0], all = min(small + (int64_t)nlist[1], w1);
+  for (int64_t w = w0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5); w < all;
        w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     const int64_t slot = w < small ? w : n - 1 - (w - small);
     const double* r = rec + BOX_REC * slot;
     if (r[3] < 0.0) continue;  // trilinear
     for_bricks(g, r[0], r[1], r[2], 2.0 * r[3], lane, 32, [&](int64_t brick) {
-      pairs[brick_off[brick] + atomicAdd(cursor + brick, 1u)] = (int32_t)slot;
+      if (FILL)
+        pairs[brick_off[brick] + atomicAdd(cursor + brick, 1u)] = (int32_t)slot;
+      else
+        atomicAdd(count + brick, 1ull);
     });
   }
 }
@@ -727,20 +736,53 @@ int deposit_box(Engine& E, int64_t n, const double* x, const double* h, const do
   NB_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp, reinterpret_cast<int64_t*>(bcount),
                                         E.brick_off + 1, (int)nbricks, st));
   NB_TRY(E.ensure_cub(tmp));
-  tmp = E.cub_bytes;
-  NB_CUDA(cub::DeviceScan::InclusiveSum(E.cub_tmp, tmp, reinterpret_cast<int64_t*>(bcount),
-                                        E.brick_off + 1, (int)nbricks, st));
-  NB_CUDA(cudaMemcpyAsync(E.h_build, E.brick_off + nbricks, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  // the bricks' offsets from their counts, and the number of pairs on the host
+  auto offsets = [&](int64_t* pairs) -> int {
+    tmp = E.cub_bytes;
+    NB_CUDA(cub::DeviceScan::InclusiveSum(E.cub_tmp, tmp, reinterpret_cast<int64_t*>(bcount),
+                                          E.brick_off + 1, (int)nbricks, st));
+    NB_CUDA(cudaMemcpyAsync(E.h_build, E.brick_off + nbricks, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    NB_CUDA(host_sync(st));
+    *pairs = E.h_build[0];
+    return 0;
+  };
+  // the lists of the entries [w0, w1) and their bricks' sums
+  auto gather = [&](int64_t pairs, int64_t w0, int64_t w1) -> int {
+    if (pairs == 0) return 0;
+    NB_TRY(E.ensure_brick_lists(pairs, pairs / BRICK_CHUNK + nbricks));
+    count_launch(), k_box_tasks<<<grid_for(nbricks), NB_THREADS, 0, st>>>(nbricks, bcount, E.brick_cursor,
+                                                                           E.brick_tasks, counters + 2);
+    count_launch(), k_box_lists<true><<<warps, NB_THREADS, 0, st>>>(
+        n, g, w0, w1, counters, E.dep_buf, bcount, E.brick_off, E.brick_cursor, E.brick_pairs);
+    count_launch(), k_box_bricks<<<(unsigned)(sms * 2), BRICK_WARPS * 32, 0, st>>>(
+        g, kid, E.dep_buf, bcount, E.brick_off, E.brick_pairs, E.brick_tasks, counters + 2, acc);
+    return 0;
+  };
+  int64_t pairs = 0;
+  NB_TRY(offsets(&pairs));
+  if (pairs <= BOX_PAIRS) return gather(pairs, 0, n);
+  // Wide supports reach so many bricks that their lists would take gigabytes: part of the work list
+  // at a time, of twice the mean's room; one that still does not fit is halved, down to the length
+  // that fits whatever it holds.
+  NB_CUDA(cudaMemcpyAsync(E.h_build, counters, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   NB_CUDA(host_sync(st));
-  const int64_t pairs = E.h_build[0];
-  if (pairs == 0) return 0;
-  NB_TRY(E.ensure_brick_lists(pairs, pairs / BRICK_CHUNK + nbricks));
-  count_launch(), k_box_tasks<<<grid_for(nbricks), NB_THREADS, 0, st>>>(nbricks, bcount, E.brick_cursor,
-                                                                         E.brick_tasks, counters + 2);
-  count_launch(), k_box_fill<<<warps, NB_THREADS, 0, st>>>(n, g, counters, E.dep_buf, E.brick_off,
-                                                           E.brick_cursor, E.brick_pairs);
-  count_launch(), k_box_bricks<<<(unsigned)(sms * 2), BRICK_WARPS * 32, 0, st>>>(
-      g, kid, E.dep_buf, bcount, E.brick_off, E.brick_pairs, E.brick_tasks, counters + 2, acc);
+  const int64_t all = E.h_build[0] + E.h_build[1];
+  const int64_t least = std::max<int64_t>(BOX_PAIRS / nbricks, 1);
+  int64_t part = std::max<int64_t>(least, (int64_t)((double)all * BOX_PAIRS / (2.0 * pairs)));
+  for (int64_t w = 0; w < all;) {
+    const int64_t end = std::min(all, w + part);
+    count_launch(), k_box_zero<<<grid_for(nbricks), NB_THREADS, 0, st>>>(nbricks, bcount, E.brick_off);
+    count_launch(), k_box_lists<false><<<warps, NB_THREADS, 0, st>>>(
+        n, g, w, end, counters, E.dep_buf, bcount, E.brick_off, E.brick_cursor, nullptr);
+    NB_TRY(offsets(&pairs));
+    if (pairs > BOX_PAIRS && part > least) {
+      part = std::max(least, part / 2);
+      continue;
+    }
+    NB_CUDA(cudaMemsetAsync(counters + 2, 0, sizeof(unsigned long long), st));
+    NB_TRY(gather(pairs, w, end));
+    w = end;
+  }
   return 0;
 }
 
