@@ -601,11 +601,11 @@ int nb_deposit_box(nb_ctx* ctx, int64_t n, const double* x, const double* h, con
   if (nb < 1 || !(dx > 0.0)) return nbk::set_host_error(E, "bad box"), NB_ERR_INPUT;
   if (!outside || !n_trilinear) return nbk::set_host_error(E, "outputs missing"), NB_ERR_INPUT;
   cudaStream_t st = S(stream);
-  NB_TRY(E.ws.ensure(E, std::max<int64_t>(E.ws.cap, 1024)));
-  NB_TRY(deposit_zero(E, acc, (int64_t)nb * nb * nb, st));
-  NB_TRY(nbk::deposit_box(E, n, x, h, m, t, v, x0, y0, z0, dx, nb, kernel_id, acc, E.ws.d_scal,
-                          (unsigned long long*)E.ws.d_i64, st));
-  return deposit_finish_host(E, 1, outside, n_trilinear, nullptr, st);
+  NB_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * nbk::DEP_FIELDS * nb * nb * nb, st));
+  NB_TRY(nbk::deposit_box(E, n, x, h, m, t, v, x0, y0, z0, dx, nb, kernel_id, acc, outside,
+                          n_trilinear, st));
+  NB_CUDA(cudaGetLastError());
+  return 0;
 }
 
 int nb_grid_finish(nb_ctx* ctx, int64_t ncell, const double* acc, const double* vol,

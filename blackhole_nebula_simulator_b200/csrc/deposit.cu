@@ -702,36 +702,55 @@ __global__ void __launch_bounds__(BRICK_WARPS * 32, 2) k_box_bricks(
   }
 }
 
+// the bricks' counts; the four work counters, the mass outside and the trilinear count with the first
 __global__ void k_box_zero(int64_t nbricks, unsigned long long* __restrict__ count,
-                           int64_t* __restrict__ brick_off) {
+                           int64_t* __restrict__ brick_off, unsigned long long* __restrict__ counters,
+                           double* __restrict__ outside, unsigned long long* __restrict__ n_tri) {
   const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (b < nbricks) count[b] = 0;
-  if (b == 0) brick_off[0] = 0;
+  if (b == 0) {
+    brick_off[0] = 0;
+    if (outside) {
+      for (int k = 0; k < 4; ++k) counters[k] = 0;
+      *outside = 0.0;
+      *n_tri = 0;
+    }
+  }
 }
 
-// acc, *outside (a device double) and *n_tri are zeroed by the caller
+// acc is zeroed by the caller; the mass outside and the number of trilinear particles come back with
+// the lists' length, so a call whose particles reach no cell by the kernel waits once (a thousand
+// supports of 0.2 cells into 32^3: 0.146 ms, 0.163 with a wait of their own and four clears).
+// The context's buffers are free again on return.
 int deposit_box(Engine& E, int64_t n, const double* x, const double* h, const double* m,
                 const double* t, const double* v, double x0, double y0, double z0, double dx,
-                int nb, int kid, double* acc, double* outside, unsigned long long* n_tri,
+                int nb, int kid, double* acc, double* outside_out, int64_t* n_tri_out,
                 cudaStream_t st) {
+  *outside_out = 0.0;
+  *n_tri_out = 0;
   if (n <= 0) return 0;
   BoxGeom g{x0, y0, z0, dx, nb, (nb + BRICK - 1) / BRICK};
   const int64_t nbricks = (int64_t)g.bricks * g.bricks * g.bricks;
+  Workspace& W = E.ws;
+  NB_TRY(W.ensure(E, std::max<int64_t>(W.cap, 1024)));
   NB_TRY(E.ensure_deposit(n));
   NB_TRY(E.ensure_bricks(nbricks));
   int sms = 0;
   NB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, E.device));
+  double* outside = W.d_scal;
+  unsigned long long* n_tri = reinterpret_cast<unsigned long long*>(W.d_i64);
   // small and wide particles listed, and the tasks
   unsigned long long* counters = reinterpret_cast<unsigned long long*>(E.dep_count);
-  NB_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), st));
   unsigned long long* bcount = E.brick_count;
-  count_launch(), k_box_zero<<<grid_for(nbricks), NB_THREADS, 0, st>>>(nbricks, bcount, E.brick_off);
+  count_launch(), k_box_zero<<<grid_for(nbricks), NB_THREADS, 0, st>>>(nbricks, bcount, E.brick_off, counters, outside, n_tri);
   count_launch(), k_box_classify<<<grid_for(n), NB_THREADS, 0, st>>>(n, x, h, m, g, E.dep_i0, counters, outside);
   const unsigned warps = (unsigned)std::min<int64_t>(grid_for(n * 32), (int64_t)sms * 8);
   count_launch(), k_box_weights<32><<<warps, NB_THREADS, 0, st>>>(
       n, x, h, m, t, v, g, kid, E.dep_i0, counters, E.dep_buf, bcount, acc, outside, n_tri);
   count_launch(), k_box_weights<NB_THREADS><<<(unsigned)std::min<int64_t>(n, (int64_t)sms * 4), NB_THREADS, 0, st>>>(
       n, x, h, m, t, v, g, kid, E.dep_i0, counters, E.dep_buf, bcount, acc, outside, n_tri);
+  NB_CUDA(cudaMemcpyAsync(W.h_dbl, outside, sizeof(double), cudaMemcpyDeviceToHost, st));
+  NB_CUDA(cudaMemcpyAsync(W.h_i64, n_tri, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   size_t tmp = 0;
   NB_CUDA(cub::DeviceScan::InclusiveSum(nullptr, tmp, reinterpret_cast<int64_t*>(bcount),
                                         E.brick_off + 1, (int)nbricks, st));
@@ -760,7 +779,14 @@ int deposit_box(Engine& E, int64_t n, const double* x, const double* h, const do
   };
   int64_t pairs = 0;
   NB_TRY(offsets(&pairs));
-  if (pairs <= BOX_PAIRS) return gather(pairs, 0, n);
+  *outside_out = W.h_dbl[0];
+  *n_tri_out = W.h_i64[0];
+  if (pairs == 0) return 0;
+  if (pairs <= BOX_PAIRS) {
+    NB_TRY(gather(pairs, 0, n));
+    NB_CUDA(host_sync(st));
+    return 0;
+  }
   // Wide supports reach so many bricks that their lists would take gigabytes: part of the work list
   // at a time, of twice the mean's room; one that still does not fit is halved, down to the length
   // that fits whatever it holds.
@@ -771,7 +797,7 @@ int deposit_box(Engine& E, int64_t n, const double* x, const double* h, const do
   int64_t part = std::max<int64_t>(least, (int64_t)((double)all * BOX_PAIRS / (2.0 * pairs)));
   for (int64_t w = 0; w < all;) {
     const int64_t end = std::min(all, w + part);
-    count_launch(), k_box_zero<<<grid_for(nbricks), NB_THREADS, 0, st>>>(nbricks, bcount, E.brick_off);
+    count_launch(), k_box_zero<<<grid_for(nbricks), NB_THREADS, 0, st>>>(nbricks, bcount, E.brick_off, nullptr, nullptr, nullptr);
     count_launch(), k_box_lists<false><<<warps, NB_THREADS, 0, st>>>(
         n, g, w, end, counters, E.dep_buf, bcount, E.brick_off, E.brick_cursor, nullptr);
     NB_TRY(offsets(&pairs));
@@ -783,6 +809,7 @@ int deposit_box(Engine& E, int64_t n, const double* x, const double* h, const do
     NB_TRY(gather(pairs, w, end));
     w = end;
   }
+  NB_CUDA(host_sync(st));
   return 0;
 }
 

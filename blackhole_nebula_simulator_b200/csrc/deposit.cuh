@@ -24,10 +24,11 @@ int deposit_log(Engine& E, int64_t n, const double* x, const double* h, const do
                 const double* t, const double* v, const LogGeom& fine, const LogGeom* coarse,
                 double wide_cells, int kid, double* acc, double* acc_c, double* scal,
                 unsigned long long* ints, cudaStream_t st);
-// the box' sums (acc, *outside and *n_tri zeroed by the caller); waits for the stream once
+// the box' sums (acc zeroed by the caller), the mass outside and the trilinear count on the host;
+// waits for the stream
 int deposit_box(Engine& E, int64_t n, const double* x, const double* h, const double* m,
                 const double* t, const double* v, double x0, double y0, double z0, double dx,
-                int nb, int kid, double* acc, double* outside, unsigned long long* n_tri,
+                int nb, int kid, double* acc, double* outside, int64_t* n_trilinear,
                 cudaStream_t st);
 void launch_grid_finish(int64_t ncell, const double* acc, const double* vol, int64_t per,
                         double* mass, float* rho, float* t_mass, float* t_em, float* vel,
