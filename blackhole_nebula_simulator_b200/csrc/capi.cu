@@ -194,6 +194,7 @@ int nb_find_neighbours(nb_ctx* ctx, int64_t n, const double* pos, const double* 
   NB_TRY(begin(ctx));
   Engine& E = ctx->E;
   if (n < 0 || n > 2000000000) return nbk::set_host_error(E, "n out of range"), NB_ERR_INPUT;
+  E.ws.cache.valid = false;  // these take the place of the lists a run would reuse
   NB_TRY(nbk::build_lists(E, n, pos, h, S(stream)));
   *total = E.lists.total;
   if (n == 0) {

@@ -1293,8 +1293,9 @@ int cell_geometry(Engine& E, int64_t n, const double* pos, const double* h, doub
   if (n <= 0) return set_host_error(E, "the cell grid needs at least one particle");
   NB_TRY(E.ensure_n(n));
   int nbb = (int)std::min<int64_t>(grid_for(n), 1184);
+  double* span6 = E.red;  // not E.bbox: the FP32 records of a run on its cached lists are in that box
   count_launch(), k_bbox_partial<<<nbb, NB_THREADS, 0, st>>>(n, pos, E.bbox_part);
-  count_launch(), k_bbox_final<<<1, NB_THREADS, 0, st>>>(nbb, E.bbox_part, E.bbox);
+  count_launch(), k_bbox_final<<<1, NB_THREADS, 0, st>>>(nbb, E.bbox_part, span6);
   double* h_sorted = reinterpret_cast<double*>(E.keys_b);
   size_t tmp = 0;
   NB_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, tmp, h, h_sorted, (int)n, 0, 64, st));
@@ -1302,7 +1303,7 @@ int cell_geometry(Engine& E, int64_t n, const double* pos, const double* h, doub
   tmp = E.cub_bytes;
   NB_CUDA(cub::DeviceRadixSort::SortKeys(E.cub_tmp, tmp, h, h_sorted, (int)n, 0, 64, st));
   double box[6], mid[2];
-  NB_CUDA(cudaMemcpyAsync(box, E.bbox, sizeof(box), cudaMemcpyDeviceToHost, st));
+  NB_CUDA(cudaMemcpyAsync(box, span6, sizeof(box), cudaMemcpyDeviceToHost, st));
   NB_CUDA(cudaMemcpyAsync(mid, h_sorted + (n - 1) / 2, sizeof(double) * (n % 2 ? 1 : 2),
                           cudaMemcpyDeviceToHost, st));
   NB_CUDA(host_sync(st));
