@@ -289,7 +289,6 @@ static int forces_impl(nb_ctx* ctx, int64_t n, const double* pos, const double* 
   fp.beta = beta;
   fp.alpha_u = alpha_u;
   fp.use_disc = 0;
-  fp.tighten = 0;
   if (grad_v && fp.use_visc) {
     if (gate < 0 || gate > 2) return nbk::set_host_error(E, "bad reconstruction gate"), NB_ERR_INPUT;
     fp.use_recon = 1;
@@ -405,7 +404,6 @@ int nb_disc_forces(nb_ctx* ctx, int64_t n, const double* pos, const double* vel,
   fp.use_sph = 0;
   fp.use_disc = 1;
   fp.disc_alpha_av = alpha_av;
-  fp.tighten = 0;
   nbk::ForceOut fo;
   fo.dacc = acc;
   fo.ddudt = dudt;

@@ -37,7 +37,6 @@ int check_device_error(Engine& E, cudaStream_t st) {
     case ERR_BAD_INDEX: msg = "index outside [0, n)"; ret = NB_ERR_INPUT; break;
     case ERR_NONPOSITIVE_U: msg = "non-positive internal energy"; ret = NB_ERR_NONPOSITIVE_U; break;
     case ERR_LEVEL: msg = "a particle needs a level beyond K_MAX = 40"; ret = NB_ERR_LEVEL; break;
-    case ERR_LIMITER: msg = "level limiter did not settle"; ret = -3; break;
     case ERR_DT: msg = "time steps must be positive"; ret = NB_ERR_DT; break;
     case ERR_EOS_RANGE: msg = "u outside the EOS bracket [1, 1e13] K"; ret = NB_ERR_EOS_RANGE; break;
     case ERR_EOS_CONVERGE: msg = "gas + radiation EOS: temperature did not converge"; ret = NB_ERR_EOS; break;
@@ -989,7 +988,6 @@ int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, in
   fp.alpha_u = prm->alpha_u;
   fp.use_disc = prm->disc_alpha_av > 0;
   fp.disc_alpha_av = prm->disc_alpha_av;
-  fp.tighten = 1;
   const bool want_tight = sk.want_tight && prm->limiter && rows == W.rows;
   W.tight_ver = -1;
   // the FP32 form without the reconstruction walks the lists in a launch of its own that writes

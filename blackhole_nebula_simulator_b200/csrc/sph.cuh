@@ -20,7 +20,6 @@ struct ForceParams {
   double beta, alpha_u;
   int use_disc;   // disc viscosity (Lodato-Price AV form on every pair)
   double disc_alpha_av;
-  int tighten;    // skip list entries with r >= 2 max(h_a, h_b)
   // velocity reconstruction in the viscosity (physics/viscosity.py:116-158): the velocity
   // gradients of every particle the pass reads, in the pass's index space: 9 floats per particle
   // (row-major dv^i/dx^j) for the FP32 form, the symmetric part in 8 doubles (two records: xx, yy,

@@ -34,7 +34,7 @@ void launch_forces32(int64_t nrows, const int64_t* rows, const float4* pos, cons
   Pos32 geo{pos, 0.f, box6};
   const unsigned grid = grid_for(nrows * 8);
   if (prm.use_recon && prm.use_visc) {
-    count_launch(), k_forces_recon32<float, Pos32, I, float4><<<grid, NB_THREADS, 0, st>>>(
+    count_launch(), k_forces_recon32<I><<<grid, NB_THREADS, 0, st>>>(
         nrows, rows, geo, vm, hydro, aux, off, idx, prm, out_map, out);
     return;
   }

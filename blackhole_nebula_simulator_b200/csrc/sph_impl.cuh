@@ -91,21 +91,6 @@ __device__ __forceinline__ float sqdist(float dx, float dy, float dz) {
   return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
 
-template <typename R>
-struct Acc;
-template <>
-struct Acc<double> {
-  double s = 0.0;
-  __device__ __forceinline__ void add(double v) { s += v; }
-  __device__ __forceinline__ double get() const { return s; }
-};
-template <>
-struct Acc<float> {
-  Kahan k;
-  __device__ __forceinline__ void add(float v) { k.add(v); }
-  __device__ __forceinline__ double get() const { return (double)k.s; }
-};
-
 // ---------------------------------------------------------------- density
 // Reference sim/sph.py:215-297 (_sums, _distances, _density_kernel): Newton-Raphson on
 // f(h) = sum_j m_j W(r_ij, h) - m_i (eta/h)^3 inside a bisection bracket, tol * h0, at most 50
@@ -121,13 +106,10 @@ __device__ __forceinline__ double group_total(double v) {
   for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-template <int L = 8>
-__device__ __forceinline__ double group_total(const Acc<double>& a) { return group_total<L>(a.s); }
-template <int L = 8>
-__device__ __forceinline__ double group_total(const Acc<float>& a) {
-  float s = a.k.s, k = -a.k.c;
+__device__ __forceinline__ double group_total(const Kahan& a) {
+  float s = a.s, k = -a.c;
 #pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) {
+  for (int o = 4; o > 0; o >>= 1) {
     float s2 = __shfl_xor_sync(0xffffffffu, s, o);
     float k2 = __shfl_xor_sync(0xffffffffu, k, o);
     float t = __fadd_rn(s, s2);
@@ -240,7 +222,7 @@ __global__ void __launch_bounds__(DENSITY_THREADS, DENSITY_BLOCKS)
   int evals = 0;
   // kernel sums at h of the rows whose `active` is set; every lane takes part in the reductions
   auto sums = [&](float h, bool active, double& rs_out, double& dws_out) {
-    Acc<float> rs, dws;
+    Kahan rs, dws;
     if (active) {
       float inv_h = 1.0f / h;
       float ih2 = inv_h * inv_h;
@@ -602,12 +584,6 @@ __global__ void __launch_bounds__(DENSITY_THREADS, 6)
 // ---------------------------------------------------------------- forces
 // Reference sim/sph.py:519-652 (_forces_kernel, no reconstruction) and sim/sph.py:1084-1117
 // (_disc_kernel).  r_ab = x_a - x_b; F(h) = dW/dr; pair terms antisymmetric.
-template <typename R>
-__device__ __forceinline__ R dwdr(R r, R h, int kid, R cnorm) {
-  R h2 = h * h;
-  return cnorm / (h2 * h2) * kernel_df<R>(r / h, kid);
-}
-
 constexpr int FORCE_QUEUE = 64;  // interacting entries a row queues before its lanes drain them
 constexpr int FORCE_UNROLL = 4;  // rounds of eight entries a walk issues at once
 
@@ -710,7 +686,7 @@ static __global__ void __launch_bounds__(NB_THREADS, 4)
   const int kid = prm.kid;
   const R ih_a = ha.x;
   const R cn4_a = cn * (ih_a * ih_a) * (ih_a * ih_a);
-  Acc<R> ax, ay, az, work, heat, vheat, cheat, dax, day, daz, dheat;
+  Kahan ax, ay, az, work, heat, vheat, cheat, dax, day, daz, dheat;
   R vmax = prm.use_visc ? cs_a : R(0);
   int npairs = 0;
   auto pair = [&](int b) {
@@ -822,15 +798,15 @@ static __global__ void __launch_bounds__(NB_THREADS, 4)
 // viscosity) in one launch, eight lanes per row (lanes 8g .. 8g+7 of a warp); the walk queues the
 // interacting entries in shared memory and drains them into the pair terms as it goes.  Two
 // blocks per SM: with two 3x3 gradients per pair more would spill.
-template <typename R, typename PosT, typename I, typename V4>
+template <typename I>
 __global__ void __launch_bounds__(NB_THREADS, 2)
-    k_forces_recon32(int64_t nrows, const int64_t* __restrict__ rows, PosT geo_in,
-             const V4* __restrict__ vm,    // (vx, vy, vz, mass)
-             const V4* __restrict__ hydro, // (h, rho, omega, P)
-             const V4* __restrict__ aux,   // (u, c_s, alpha, unused)
+    k_forces_recon32(int64_t nrows, const int64_t* __restrict__ rows, Pos32 geo,
+             const float4* __restrict__ vm,    // (vx, vy, vz, mass)
+             const float4* __restrict__ hydro, // (h, rho, omega, P)
+             const float4* __restrict__ aux,   // (u, c_s, alpha, unused)
              const int64_t* __restrict__ off, const I* __restrict__ idx, ForceParams prm,
              const int32_t* __restrict__ out_map, ForceOut out) {
-  PosT geo = geo_in;
+  using R = float;
   geo.ready();
   const unsigned FULL = 0xffffffffu;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -843,15 +819,15 @@ __global__ void __launch_bounds__(NB_THREADS, 2)
     a = rows ? rows[q] : q;
     o = out_map ? (int64_t)out_map[a] : q;
   }
-  const V4 va = vm[a], ha = hydro[a], xa = aux[a];
+  const float4 va = vm[a], ha = hydro[a], xa = aux[a];
   const R h_a = (R)ha.x, rho_a = (R)ha.y, om_a = (R)ha.z, P_a = (R)ha.w;
   const R inv_or_a = R(1) / (om_a * rho_a);
   const R inv_orr_a = R(1) / (om_a * rho_a * rho_a);
-  const R cs_a = (R)xa.y, al_a = (R)xa.z, u_a = (R)xa.x;
+  const R cs_a = (R)xa.y, al_a = (R)xa.z;
   const R beta = (R)prm.beta, alpha_u = (R)prm.alpha_u, aav = (R)prm.disc_alpha_av;
   const R cn = (R)prm.cnorm;
   const int kid = prm.kid;
-  Acc<R> ax, ay, az, work, heat, vheat, cheat, dax, day, daz, dheat;
+  Kahan ax, ay, az, work, heat, vheat, cheat, dax, day, daz, dheat;
   R vmax = prm.use_visc ? cs_a : R(0);
   int64_t npairs = 0;
   // the row's list in rounds of eight entries: lanes test their entry, the interacting ones are
@@ -875,7 +851,7 @@ __global__ void __launch_bounds__(NB_THREADS, 2)
   }
   const R eta_crit = (R)prm.eta_crit, eta_fold = (R)prm.eta_fold;
   auto recon_visc = [&](int64_t b, R dx0, R dx1, R dx2, R r, R rx, R ry, R rz, R h_b, R vdotr,
-                        const V4& vb, const V4& xb, R rho_b, R m_b, R fa, R& num_a, R& num_b) {
+                        const float4& vb, const float4& xb, R rho_b, R m_b, R fa, R& num_a, R& num_b) {
     R Gb[9];
 #pragma unroll
     for (int e = 0; e < 9; ++e) Gb[e] = prm.gv32[9 * b + e];
@@ -932,11 +908,11 @@ __global__ void __launch_bounds__(NB_THREADS, 2)
   auto pair_fast = [&](int64_t b) {
     R ddx, ddy, ddz;
     geo.diff(a, b, ddx, ddy, ddz);  // x_b - x_a
-    const V4 hb4 = hydro[b];
+    const float4 hb4 = hydro[b];
     const R h_b = (R)hb4.x;
     const R d2 = sqdist(ddx, ddy, ddz);
     npairs += 1;
-    const V4 vb = vm[b];
+    const float4 vb = vm[b];
     const R rho_b = (R)hb4.y, om_b = (R)hb4.z, P_b = (R)hb4.w;
     const R m_b = (R)vb.w;
     const R inv_r = rsqrtf(d2);
@@ -949,31 +925,29 @@ __global__ void __launch_bounds__(NB_THREADS, 2)
     const R vdotr = dvx * rx + dvy * ry + dvz * rz;
     R num_a = P_a, num_b = P_b;
     const R inv_orr_b = __frcp_rn(om_b * rho_b * rho_b);
-    if (prm.use_sph) {
-      if (prm.use_visc) {
-        const V4 xb = aux[b];
-        recon_visc(b, -ddx, -ddy, -ddz, r, rx, ry, rz, h_b, vdotr, vb, xb, rho_b, m_b, fa, num_a,
-                   num_b);
-        if (prm.use_cond) {
-          R vu;
-          if (prm.cond_signal == 0)
-            vu = sqrt(fabs(P_a - P_b) * __frcp_rn(R(0.5) * (rho_a + rho_b)));
-          else
-            vu = fabs(vdotr);
-          R dc = m_b * alpha_u * vu * (R)(xa.x - xb.x) * R(0.5) *
-                 (fa * inv_or_a + fb * inv_orr_b * rho_b);
-          heat.add(dc);
-          cheat.add(dc);
-        }
+    if (prm.use_visc) {
+      const float4 xb = aux[b];
+      recon_visc(b, -ddx, -ddy, -ddz, r, rx, ry, rz, h_b, vdotr, vb, xb, rho_b, m_b, fa, num_a,
+                 num_b);
+      if (prm.use_cond) {
+        R vu;
+        if (prm.cond_signal == 0)
+          vu = sqrt(fabs(P_a - P_b) * __frcp_rn(R(0.5) * (rho_a + rho_b)));
+        else
+          vu = fabs(vdotr);
+        R dc = m_b * alpha_u * vu * (R)(xa.x - xb.x) * R(0.5) *
+               (fa * inv_or_a + fb * inv_orr_b * rho_b);
+        heat.add(dc);
+        cheat.add(dc);
       }
-      R f = m_b * (num_a * inv_orr_a * fa + num_b * inv_orr_b * fb);
-      ax.add(-f * rx);
-      ay.add(-f * ry);
-      az.add(-f * rz);
-      work.add(m_b * vdotr * fa);
     }
+    R f = m_b * (num_a * inv_orr_a * fa + num_b * inv_orr_b * fb);
+    ax.add(-f * rx);
+    ay.add(-f * ry);
+    az.add(-f * rz);
+    work.add(m_b * vdotr * fa);
     if (prm.use_disc) {
-      const V4 xb = aux[b];
+      const float4 xb = aux[b];
       const R vdr = vdotr;  // v_ab . (x_a - x_b) / r
       R qa = -rho_a * h_a * R(0.5) * inv_r * aav * cs_a * vdr * inv_orr_a;
       R qb = -rho_b * h_b * R(0.5) * inv_r * aav * (R)xb.y * vdr * inv_orr_b;
@@ -1013,19 +987,16 @@ __global__ void __launch_bounds__(NB_THREADS, 2)
       tight[u] = false;
       if (b >= 0) {
         if (b != a) {
-          bool tk = true;
-          if (prm.tighten) {
-            R ddx, ddy, ddz, h_b;
-            geo.diff_h(geo.own(a), b, ddx, ddy, ddz, h_b);
-            R rr = R(2) * (h_a > h_b ? h_a : h_b);
-            const R d2 = sqdist(ddx, ddy, ddz), r2 = rr * rr;
-            tk = d2 < r2;
-            if (prm.pos64 && d2 > r2 * R(1.0 - 1e-5) && d2 < r2 * R(1.0 + 1e-5)) {
-              const double4 pa = prm.pos64[a], pb = prm.pos64[b];
-              const double e2 = d2_exact(pb.x - pa.x, pb.y - pa.y, pb.z - pa.z);
-              const double er = 2.0 * fmax(pa.w, pb.w);
-              tk = e2 < er * er;
-            }
+          R ddx, ddy, ddz, h_b;
+          geo.diff_h(geo.own(a), b, ddx, ddy, ddz, h_b);
+          R rr = R(2) * (h_a > h_b ? h_a : h_b);
+          const R d2 = sqdist(ddx, ddy, ddz), r2 = rr * rr;
+          bool tk = d2 < r2;
+          if (prm.pos64 && d2 > r2 * R(1.0 - 1e-5) && d2 < r2 * R(1.0 + 1e-5)) {
+            const double4 pa = prm.pos64[a], pb = prm.pos64[b];
+            const double e2 = d2_exact(pb.x - pa.x, pb.y - pa.y, pb.z - pa.z);
+            const double er = 2.0 * fmax(pa.w, pb.w);
+            tk = e2 < er * er;
           }
           take[u] = tk;
           tight[u] = tk;
@@ -1051,17 +1022,10 @@ __global__ void __launch_bounds__(NB_THREADS, 2)
   drain();
   if (prm.tcnt && live && gl == 0) prm.tcnt[q] = m_tot;
   // sums over the row's eight lanes (uniform flags: every lane takes part in every reduction)
-  double s_ax = 0, s_ay = 0, s_az = 0, s_work = 0, s_heat = 0, s_vheat = 0, s_cheat = 0;
   double s_dax = 0, s_day = 0, s_daz = 0, s_dheat = 0;
-  if (prm.use_sph) {
-    s_ax = group_total(ax);
-    s_ay = group_total(ay);
-    s_az = group_total(az);
-    s_work = group_total(work);
-    s_heat = group_total(heat);
-    s_vheat = group_total(vheat);
-    s_cheat = group_total(cheat);
-  }
+  const double s_ax = group_total(ax), s_ay = group_total(ay), s_az = group_total(az);
+  const double s_work = group_total(work), s_heat = group_total(heat);
+  const double s_vheat = group_total(vheat), s_cheat = group_total(cheat);
   if (prm.use_disc) {
     s_dax = group_total(dax);
     s_day = group_total(day);
@@ -1075,18 +1039,16 @@ __global__ void __launch_bounds__(NB_THREADS, 2)
     npairs += __shfl_xor_sync(FULL, npairs, of);
   }
   if (!live || gl != 0) return;
-  if (prm.use_sph) {
-    double du = (double)P_a * (double)inv_or_a / (double)rho_a * s_work + s_heat;
-    if (out.acc) {
-      out.acc[3 * o + 0] = s_ax;
-      out.acc[3 * o + 1] = s_ay;
-      out.acc[3 * o + 2] = s_az;
-    }
-    if (out.dudt) out.dudt[o] = du;
-    if (out.vsig) out.vsig[o] = (double)vmax;
-    if (out.vheat) out.vheat[o] = s_vheat;
-    if (out.cheat) out.cheat[o] = s_cheat;
+  const double du = (double)P_a * (double)inv_or_a / (double)rho_a * s_work + s_heat;
+  if (out.acc) {
+    out.acc[3 * o + 0] = s_ax;
+    out.acc[3 * o + 1] = s_ay;
+    out.acc[3 * o + 2] = s_az;
   }
+  if (out.dudt) out.dudt[o] = du;
+  if (out.vsig) out.vsig[o] = (double)vmax;
+  if (out.vheat) out.vheat[o] = s_vheat;
+  if (out.cheat) out.cheat[o] = s_cheat;
   if (prm.use_disc) {
     if (out.dacc) {
       out.dacc[3 * o + 0] = s_dax;
