@@ -1,7 +1,8 @@
 """Build recipe of libnebula_b200.so: every CUDA source compiled for sm_100a with nvcc.
 
-FP64 sources are compiled without fused multiply-add so the double-precision path rounds like
-the reference; the FP32 pair passes keep fused multiply-add.  The library is written in place
+FP64 sources are compiled without contraction, so an operation is fused only where the source says
+fma (never where the result must round like the reference's: list tests, the flow, the counts of a
+deposition); the FP32 pair passes let the compiler fuse.  The library is written in place
 (next to this file) so it travels with the source tree.
 """
 

@@ -4,8 +4,9 @@
 // weights in index space over the 8 nearest centres.  Weight beyond the grid goes to the
 // `outside` total.  On the log grid a thread (a warp for wide supports) walks a particle's candidate
 // centres twice (sum of weights, then the atomic adds); the box is gathered brick by brick; the
-// cell sums are FP64.  Compiled without fused multiply-add, so a
-// particle's weights round like the reference's (the order of the atomic adds does not).
+// cell sums are FP64.  Which centres count towards the choice of weights is the reference's own
+// arithmetic (compiled without contraction); the weights themselves are within rounding of it, and the
+// order of the additions is not its order.
 #include <cub/cub.cuh>
 
 #include "common.cuh"
@@ -264,9 +265,7 @@ __device__ __forceinline__ double log_one(const LogTarget& T, const LogParticle&
 // launch: a serial walk of thousands of centres would be a tail of its own, and a small input with
 // wide supports would leave the chip idle.  Bound by L2's FP64 adds (eight a centre) and the walk's
 // FP64 arithmetic.  The whole call for the disc sampled by 1,000,003 particles (cubic) 0.90 ms; 2.08
-// with a thread for every particle over the reference's wider windows, one grid after the other, and
-// 1.51 with an atomic count per particle beyond the kernel's reach and candidate boxes a centre wider
-// on each side.  20,000 / 150,000 / 2,000,000 particles 1.1 / 0.73 / 1.35 ms (8.1 / 3.87 / 2.38).
+// with a thread for every particle over the reference's wider windows, one grid after the other.  20,000 / 150,000 / 2,000,000 particles 1.1 / 0.73 / 1.35 ms (8.1 / 3.87 / 2.38).
 // LOG_WIDE 64 / 128 / 256 differ by 2 % but for 50,000 Wendland particles: 1.56 / 1.60 / 1.71 ms.  Blocks
 // an SM of the first launch, 4 / 5 / 6: 0.905 / 0.894 / 0.926 ms at 1,000,003.
 // Particles from n_narrow on are the second grid's (the coarser one of very wide particles).
@@ -346,9 +345,9 @@ __global__ void __launch_bounds__(128, LOG_B) k_deposit_log_heavy(
 //                   per lane, the six sums in registers: no atomic add per (particle, cell)
 // Bound by the FP64 pipe (a kernel value per lane of every sub-brick a support reaches, about a
 // third to a half of the lanes inside).  The 1,048,576-particle torus into 160^3 cells takes
-// 3.75 ms (bricks 1.40, weights 1.37 + 0.66 for the wide particles); one thread per particle
+// 3.73 ms (bricks 1.40, weights 1.37 + 0.66 for the wide particles); one thread per particle
 // walking its support with six atomic adds per cell kept 5 of 32 lanes busy, sent 1.8e9
-// reductions to L2 and took 61 ms.  A particle of BOX_WIDE = 25^3 candidate cells or more takes a
+// reductions to L2 and took 61 ms.  A particle of BOX_WIDE candidate cells (25.4^3) or more takes a
 // block, so that none keeps a warp alone for a millisecond.
 constexpr int BRICK = 8;            // cells per brick edge
 constexpr int BRICK_WARPS = 16;     // sub-bricks of 2 x 4 x 4 cells
@@ -366,7 +365,8 @@ struct BoxGeom {
   int nb, bricks;  // cells and bricks per axis
 };
 
-// (int)floor of the reference's index expressions; a NaN gives 0, as the conversion does
+// (int)floor of the reference's index expressions; a NaN gives the lowest int (the conversion of a
+// double does), a cell beyond the box
 __device__ __forceinline__ int cell_of(double v, double lo, double dx) {
   return (int)floor((v - lo) / dx);
 }

@@ -673,7 +673,7 @@ static int density_on_lists(Engine& E, int64_t n, const double* x, const double*
   } else {
     // the rows are the mask's (their number is known), sorted beside the active rows' copy, which
     // the force pass then finds still valid: eight launches less per block step on reused lists (20
-    // steps of 300,000 particles 15.6 -> 14.9 ms)
+    // steps of 300,000 particles 15.6 -> 15.1 ms)
     count_launch(), k_sorted_mask<<<grid_for(n), NB_THREADS, 0, st>>>(n, L.perm, mask, W.m_smark);
     size_t tmp = E.cub_bytes;
     NB_CUDA(cub::DeviceSelect::Flagged(E.cub_tmp, tmp, thrust::counting_iterator<int64_t>(0), W.m_smark,

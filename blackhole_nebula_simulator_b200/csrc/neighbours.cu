@@ -278,13 +278,11 @@ __device__ __forceinline__ double box_gap2(double4 alo, double4 ahi, double4 blo
 }
 
 // The rows of one query leaf of LEAF consecutive sorted particles, one lane per particle, tested
-// tile by tile.  The warp walks the tree of boxes with an explicit stack in shared memory (entries
-// (level << 40) | index; children pushed highest first, so candidate leaves are reached in
-// ascending order) and takes, in ascending order, the sub-leaves whose boxes lie within reach of
-// the query leaf's box.  Every 4 of them (32 candidates) are staged in shared memory, one
-// candidate per lane with coalesced loads, as float offsets from the query leaf's centre, and
-// every lane tests its own particle against all 32: the whole warp stays busy on the same
-// candidates, with no per-lane queues.
+// tile by tile.  The leaf's candidates are the sub-leaves whose boxes lie within its reach, in
+// ascending order.  Every 4 of them (32 candidates) are staged in shared memory, one candidate per
+// lane with coalesced loads, as float offsets from the query leaf's centre, and every lane tests its
+// own particle against all 32: the whole warp stays busy on the same candidates, with no per-lane
+// queues.
 //
 // The test is the reference's FP64 r^2 < (2 h_i)^2 or r^2 < (2 h_j)^2 decided in FP32 with a
 // rigorous band.  With D the largest offset component of the query lanes and the staged batch
@@ -298,11 +296,12 @@ __device__ __forceinline__ double box_gap2(double4 alo, double4 ahi, double4 blo
 // the exact FP64 test (no fused multiply-add) from the double positions.  So the lists are the
 // reference's bit for bit.
 //
-// Three passes share the traversal: k_lists_cand counts each query leaf's candidate sub-leaves
-// (so every leaf gets its own slice of the candidate and mask buffers), k_lists_test runs the
-// tests once, storing each lane's 32-bit hit mask per batch and its row's entry count, and
-// k_lists_expand turns the masks into the CSR entries at the rows' offsets, each row ascending
-// (batches come in ascending candidate order, a mask's bits from the lowest slot up).
+// Three passes: k_lists_cand finds the candidates of each query leaf, level by level through the tree
+// of boxes (k_lists_wide for the leaves whose frontiers outgrow a warp's buffer, and in it a
+// depth-first walk for those that outgrow a block's), each in its own slice of the candidate and mask
+// buffers; k_lists_test runs the tests once, storing each lane's 32-bit hit mask per batch and its
+// row's entry count; k_lists_expand turns the masks into the CSR entries at the rows' offsets, each
+// row ascending (batches come in ascending candidate order, a mask's bits from the lowest slot up).
 
 constexpr float BAND_U = 192.0f / 16777216.0f;  // 192 u, u = 2^-24
 
@@ -322,7 +321,8 @@ __device__ __forceinline__ QueryLeaf query_leaf(const TreeView& tv, int64_t leaf
   return q;
 }
 
-// Walk the tree for one query leaf; on_subs(s0, mask) is called warp-uniformly for every
+// Depth-first walk of the tree for one query leaf by one warp, with a stack in shared memory (entries
+// (level << 40) | index, children pushed highest first); on_subs(s0, mask) is called warp-uniformly for every
 // candidate leaf with its first sub-leaf s0 and the ballot of its sub-leaves within reach of the
 // query leaf's box (bit c: sub-leaf s0 + c), in ascending order.  Returns false if the stack
 // overflowed.
@@ -653,11 +653,11 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 
 // Pass 2: the tests, on each work item's batches of candidates.  Each batch's final hit masks go
 // to masks[(batch base + b) * 32 + lane], the item's entries per row to part_count and, added up,
-// to counts (zeroed before).  Bound by issue (71 %) and by the broadcast loads of the staged
-// candidates (LSU 69 %, but four rows by eight candidates a lane, with a quarter of those loads,
-// gain 1 %): 0.83 ms on the 1M torus.  Two candidates per packed instruction, the whole batch
-// unrolled, two blocks per SM (three spill); with scalar tests, a warp alone on its leaf whatever the
-// leaf's number of batches and candidates by the leaf's box alone, 1.30 ms.
+// to counts (zeroed before).  Bound by issue (60 % active, cold, at two blocks of 120 registers an SM;
+// four rows by eight candidates a lane, with a quarter of the shared loads, gain 1 %): 0.83 ms on the
+// 1M torus.  Two candidates per packed instruction, the whole batch unrolled (three blocks spill);
+// with scalar tests, a warp alone on its leaf whatever the leaf's number of batches and candidates by
+// the leaf's box alone, 1.30 ms.
 #ifndef TEST_BLOCKS_PER_SM
 #define TEST_BLOCKS_PER_SM 2
 #endif
@@ -801,11 +801,11 @@ __global__ void __launch_bounds__(NB_THREADS, TEST_BLOCKS_PER_SM) k_lists_test(
 // lane c holds candidate c of each batch, and for every row with a hit in them the lanes whose bit
 // is set in the row's mask store their candidates at the row's next positions (a bit's rank in
 // the mask), so a row's entries come ascending.
-// Bound by issue, about ten instructions per row and batch: 0.65 ms on the 1M torus (160M entries),
-// 0.52 on a 400,000-particle Wendland torus, 12 us on a 4,096-particle cloud.  Each lane appending a
-// row's entries to a ring in shared memory that the warp empties in aligned stretches of 32 took
-// 0.78, 0.75 ms and 22 us (fewer stores, but a loop over the longest of 32 masks).  Batches at a
-// time 2 / 4 / 8: 0.65 / 0.65 / 0.68 ms.  The candidates culled by sub-leaf (pass 1) leave 0.59, 0.51 ms, 12 us.
+// Bound by issue (73 % active, about ten instructions per row and batch): 0.59 ms on the 1M torus
+// (160M entries), 0.51 on a 400,000-particle Wendland torus, 12 us on a 4,096-particle cloud.  Rings in
+// shared memory that the warp empties in aligned stretches of 32 (fewer stores, but a loop over the
+// longest of 32 masks) took 0.78, 0.75 ms and 22 us; batches at a time 2 / 4 / 8: 0.65 / 0.65 / 0.68 ms,
+// before the candidates were culled by sub-leaf.
 constexpr int EXPAND_WARPS = 4;
 constexpr int EXPAND_BATCHES = 4;
 
@@ -973,10 +973,10 @@ __device__ __forceinline__ void export_row(const int32_t* __restrict__ src, int 
 }
 
 // Rows in the caller's order and numbering, each ascending: one warp per row, sorted in registers.
-// Bound by the network's shuffles and minima; the entries are read and written once.  Building
-// and exporting the lists of the 1M torus (160M entries) takes 5.56 ms, of a 4,096-particle
-// cloud 0.52 ms; with rows filled by one thread each and sorted as 64-bit keys by a segmented
-// device sort it was 76.5 and 0.90 ms.  The network is chosen by the row's length; a row over
+// Bound by the network's shuffles and minima; the entries are read and written once: 1.03 ms on the 1M
+// torus (160M entries).  With rows filled by one thread each and sorted as 64-bit keys by a segmented
+// device sort, building and exporting those lists took 76.5 ms, of a 4,096-particle cloud 0.90 ms;
+// with this kernel in its place, on the list build of then, 5.56 and 0.52 ms (3.19 and 0.33 now).  The network is chosen by the row's length; a row over
 // EXPORT_MAX entries (the registers of the largest network) goes unsorted to `keys` and into the
 // segment list, for the device sort.
 constexpr int EXPORT_MAX = 1024;

@@ -1,4 +1,4 @@
-// Parameters and launchers of the SPH pair passes (sph.cu).
+// Parameters and launchers of the SPH pair passes (sph_impl.cuh, sph64.cu, sph32.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

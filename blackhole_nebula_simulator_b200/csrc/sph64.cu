@@ -1,5 +1,5 @@
-// FP64 instantiations of the pair passes (compiled without fused multiply-add: the FP64 path
-// rounds like the reference).
+// FP64 instantiations of the pair passes.  Compiled without contraction, so that an operation is fused
+// only where an fma is written: the list tests round like the reference, the sums' terms do not.
 #include <type_traits>
 
 #include "sph_impl.cuh"
@@ -21,11 +21,14 @@ void launch_density64(int64_t nrows, const int64_t* rows, const double4* pos, co
         iters, flags, work);
   };
   using std::integral_constant;
-  // Cubic: 8 lanes per row once the rows fill the GPU (262,144 cloud rows 447 us against 646 with
-  // 32 lanes; 300,000 torus rows 607 against 721), 32 for fewer (30,000 rows 150 us against 186,
-  // 3,000 rows 84 against 113).  Wendland C4: 32 lanes at any size, whose block keeps 4 rows'
-  // caches (11 KB) instead of 16 rows' (43 KB) out of L1 (200,001 torus rows 0.98 ms against
-  // 1.24 with 16 lanes and 1.94 with 8).
+  // Cubic: 8 lanes per row once the rows fill the GPU, 32 for fewer, whose rows are then in flight
+  // together.  Where the two meet depends on the gas and the guess; from the last step's h, call
+  // times in us with 8 / 32 lanes: a cloud of 10,000 rows 93 / 94, 30,000 130 / 142, 60,000 169 / 203,
+  // 262,144 458 / 649; a torus of 30,000 210 / 156, 60,000 268 / 229, 100,000 314 / 306, 200,000
+  // 465 / 516.  The line lies between the two gases.  (From a guess far off, 32 lanes stay ahead
+  // on a torus: 200,000 rows 3,367 / 2,104.)  Wendland C4: 32 lanes at any size, whose block keeps 4
+  // rows' caches (11 KB) instead of 16 rows' (43 KB) out of L1 (200,001 torus rows 0.98 ms
+  // against 1.24 with 16 lanes and 1.94 with 8).
   if (prm.kid != 0)
     run(integral_constant<int, 1>{}, integral_constant<int, 32>{});
   else if (nrows >= 65536)
@@ -41,7 +44,8 @@ void launch_forces64(int64_t nrows, const int64_t* rows, const double4* pos, con
   if (nrows <= 0) return;
   auto run = [&](auto sph, auto disc, auto recon) {
     constexpr bool S = decltype(sph)::value, D = decltype(disc)::value, R = decltype(recon)::value;
-    // the caller-order lists come tightened, the engine's sorted lists are tested by the walk
+    // the operators' int64 lists are taken as they are, every entry a pair, as their reference does;
+    // the engine's int32 lists hold the search radius' entries, which the walk tests
     constexpr bool T = sizeof(I) == 4;
     count_launch(), k_forces64<S, D, R, T, I><<<grid_for(nrows * 8, F64_THREADS), F64_THREADS, 0, st>>>(
         nrows, rows, pos, vm, hydro, aux, prm.gs64, off, idx, prm, out_map, out);

@@ -1,12 +1,12 @@
 // SPH pair passes on neighbour lists (implementation, included by sph64.cu and sph32.cu): the h-rho Newton solve and the fused pressure + artificial
 // viscosity (+ conductivity, + disc viscosity) force and du/dt pass.
 //
-// The density solve runs 8 (FP32) or 16 (FP64) lanes per row with a shared-memory cache of the
-// inner entries; the force pass eight lanes per row.  Both walk CSR lists.  They are templated on the list index type so the
-// same code serves the caller-order int64 lists of the operator API and the engine's sorted int32
-// lists, and on the arithmetic: FP64 (every pair term in double) or FP32 (positions as float
-// offsets from cell centres, float pair terms, Kahan-compensated sums, the Newton update and all
-// per-particle state in double).
+// The density solve runs 8 lanes per row (FP64: 8 or 32, see launch_density64) with a shared-memory
+// cache of the inner entries; the force pass eight lanes per row.  Both walk CSR lists.  They are
+// templated on the list index type so the same code serves the caller-order int64 lists of the
+// operator API and the engine's sorted int32 lists.  The FP64 kernels form every pair term in double;
+// the FP32 ones take positions as float offsets from cell centres, float pair terms and
+// Kahan-compensated sums, with the Newton update and all per-particle state in double.
 #pragma once
 #include "common.cuh"
 #include "engine.cuh"
@@ -141,9 +141,9 @@ constexpr int DENSITY_UNROLL = 4, DENSITY_WALK = 2, DENSITY_BLOCKS = 9;
 // holds re-walk their list in every sum.  (The compensated float sums depend on the order of
 // their terms in the eighth digit: which lane adds which entry when is part of the result, and so
 // are the fused operations of a term, written out below where a rearrangement changed them.)
-// Bound by issue (65 % active, about 900 warp instructions per row) and by the gathers (LSU 68 %).
-// With a square root per list entry, three loads per record, divergent kernel branches and
-// conflicting cache rows the two launches above took 51.5 and 5.49 ms.
+// Bound by issue (74 % active, about 820 warp instructions per row of a 1M torus step, at half the
+// warp slots).  With a square root per list entry, three loads per record, divergent kernel branches
+// and conflicting cache rows the two launches above took 51.5 and 5.49 ms.
 template <int KID, typename I>
 __global__ void __launch_bounds__(DENSITY_THREADS, DENSITY_BLOCKS)
     k_density32(int64_t nrows, const int64_t* __restrict__ rows, Pos32 geo,
@@ -393,10 +393,9 @@ struct DensityTerm {
 // (2 h > r_in), or has shrunk enough that the entries of a row too long for the cache may fit, the
 // cache is filled again at the present h.  A row with more entries inside 2.1 h than the cache
 // holds walks its list in every sum.
-// Bound by issue and by the gathers' latency (54 % issue active, L1 54 %, FP64 pipe 35 % at 16
-// lanes; a row needs about 800 warp instructions with 8 lanes).  With one thread per row, the list
-// read uncoalesced and walked again in every sum, 262,144 cloud particles took 1.69 ms per call;
-// 0.45 ms now.
+// Bound by issue and by the gathers' latency (8 lanes, 262,144 cloud rows: 55 % issue active, L1 66 %,
+// FP64 pipe 36 %, 35 % of the warp slots; 920 warp instructions per row).  With one thread per row,
+// the list read uncoalesced and walked again in every sum, that call took 1.69 ms; 0.45 ms now.
 // Entries kept: about 67 lie inside 2.1 h with the cubic kernel, 159 with Wendland C4.
 template <int KID>
 constexpr int D64_CAP = KID == 0 ? 128 : 224;

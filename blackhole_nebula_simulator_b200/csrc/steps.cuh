@@ -35,11 +35,12 @@ int compute_density(Engine& E, int64_t n, const double* x, const double* mass, d
                     const uint8_t* rows_mask = nullptr, int first_fail = -1);
 int reuse_first_test(Engine& E, int64_t n, const double* x, const double* hg_in,
                      const uint8_t* mask, int* fail, cudaStream_t st);
-// out = the indices of mask's set entries, ascending; count read on the host (with W.d_i64[1]
-// into *also when given)
+// out = 0 .. n - 1
 void launch_iota(int64_t n, int64_t* out, cudaStream_t st);
 // one device word, with the pending checks
 int read_word(Engine& E, const int64_t* d, int64_t* out, cudaStream_t st);
+// out = the indices of mask's set entries, ascending; count read on the host (with W.d_i64[1]
+// into *also when given)
 int select_mask(Engine& E, int64_t n, const uint8_t* mask, int64_t* out, int64_t* count,
                 cudaStream_t st, int64_t* also = nullptr);
 int engine_forces(Engine& E, nb_state* s, const double* vel, const double* u, int64_t nrows,
