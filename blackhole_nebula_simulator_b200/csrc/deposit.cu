@@ -371,6 +371,11 @@ __device__ __forceinline__ int cell_of(double v, double lo, double dx) {
   return (int)floor((v - lo) / dx);
 }
 
+// d^2 of a centre, in one arithmetic for the weights' sum and for the bricks: only so do a particle's
+// weights add up to one where its centres all lie close to the support's edge
+__device__ __forceinline__ double box_yz2(double dy, double dz) { return fma(dz, dz, dy * dy); }
+__device__ __forceinline__ double box_d2(double dx, double yz2) { return fma(dx, dx, yz2); }
+
 struct BoxRange {
   int a0, a1, b0, b1, c0, c1;
 };
@@ -497,24 +502,23 @@ __global__ void __launch_bounds__(NB_THREADS) k_box_weights(
     double w_in = 0.0, w_out = 0.0;
     bool eight = box_holds_eight(xp, yp, zp, big, dx);
     if (eight) {
-      // columns of the support along x, one (b, c) per thread; lane l of a warp keeps the
-      // squared x distance of plane a + l, so a centre costs one addition before its weight
+      // columns of the support along x, one (b, c) per thread; lane l of a warp keeps the x
+      // distance of plane a + l, so a centre costs one fused operation before its weight
       for (int64_t e0 = rank - lane; e0 < plane; e0 += GROUP) {
         const int64_t e = e0 + lane;
         // (a warp's support has less than BOX_WIDE cells: 32-bit quotients)
         const int64_t eb = GROUP > 32 ? e / ncc : (int64_t)((unsigned)e / (unsigned)ncc);
         const int b = (int)(r.b0 + eb), c = (int)(r.c0 + (e - eb * ncc));
         const double dy = g.y0 + (b + 0.5) * dx - yp, dz = g.z0 + (c + 0.5) * dx - zp;
-        const double yz2 = e < plane ? dy * dy + dz * dz : INFINITY;
+        const double yz2 = e < plane ? box_yz2(dy, dz) : INFINITY;
         const bool in_bc = b >= 0 && b < g.nb && c >= 0 && c < g.nb;
         if (!__any_sync(FULL, yz2 < big2)) continue;
         double s_in = 0.0, s_all = 0.0;
         for (int64_t a32 = r.a0; a32 <= r.a1; a32 += 32) {
           const double da = g.x0 + ((double)(a32 + lane) + 0.5) * dx - xp;
-          const double a2 = da * da;
           const int na = (int)min((int64_t)32, (int64_t)r.a1 - a32 + 1);
           for (int k = 0; k < na; ++k) {
-            const double dd = yz2 + __shfl_sync(FULL, a2, k);
+            const double dd = box_d2(__shfl_sync(FULL, da, k), yz2);
             if (dd < big2) {
               const double f = kernel_f<double>(sqrt(dd) * ih, kid);
               s_all += f;
@@ -540,10 +544,10 @@ __global__ void __launch_bounds__(NB_THREADS) k_box_weights(
           const int b = r.b0 + (int)(e / ncc), c = r.c0 + (int)(e % ncc);
           const double dyc = g.y0 + (b + 0.5) * dx - yp, dzc = g.z0 + (c + 0.5) * dx - zp;
           const double dd = dxc * dxc + dyc * dyc + dzc * dzc;
-          const bool in = dd < in2 || (dd < out2 && sqrt(dd) / hp < 2.0);
-          if (!in) continue;
-          n_in += 1.0;
-          const double f = kernel_f<double>(sqrt(dd) * ih, kid);
+          if (dd < in2 || (dd < out2 && sqrt(dd) / hp < 2.0)) n_in += 1.0;
+          const double df = box_d2(dxc, box_yz2(dyc, dzc));
+          if (!(df < big2)) continue;
+          const double f = kernel_f<double>(sqrt(df) * ih, kid);
           if (a >= 0 && a < g.nb && b >= 0 && b < g.nb && c >= 0 && c < g.nb)
             w_in += f;
           else
@@ -552,11 +556,14 @@ __global__ void __launch_bounds__(NB_THREADS) k_box_weights(
       }
       eight = group_sum<GROUP>(n_in, red) >= (double)DEP_MIN_CELLS;
     }
+    w_in = group_sum<GROUP>(w_in, red);
+    w_out = group_sum<GROUP>(w_out, red);
     double vals[DEP_FIELDS];
     particle_vals(p, m, t, v, vals);
-    if (!eight) {
-      // trilinear weights over the eight nearest centres, one per lane
-      if (rank == 0) atomicAdd(n_tri, 1ull);
+    if (!eight || !(w_in + w_out > 0.0)) {
+      // trilinear weights over the eight nearest centres, one per lane (also, uncounted, where every
+      // centre is a rounding from the edge and has no weight)
+      if (rank == 0 && !eight) atomicAdd(n_tri, 1ull);
       const double fa = (xp - g.x0) / dx - 0.5, fb = (yp - g.y0) / dx - 0.5,
                    fc = (zp - g.z0) / dx - 0.5;
       const int ia = (int)floor(fa), ib = (int)floor(fb), ic = (int)floor(fc);
@@ -573,8 +580,6 @@ __global__ void __launch_bounds__(NB_THREADS) k_box_weights(
       if (rank == 0) rec[BOX_REC * slot + 3] = -1.0;  // nothing for the bricks
       continue;
     }
-    w_in = group_sum<GROUP>(w_in, red);
-    w_out = group_sum<GROUP>(w_out, red);
     const double inv = 1.0 / (w_in + w_out);
     if (rank == 0 && w_out != 0.0) out_all += w_out * inv * vals[0];
     if (rank < BOX_REC) {
@@ -683,7 +688,7 @@ __global__ void __launch_bounds__(BRICK_WARPS * 32, 2) k_box_bricks(
         for (unsigned mk = __ballot_sync(FULL, reach); mk; mk &= mk - 1) {
           const double* q = stage[k0 + __ffs(mk) - 1];
           const double ddx = cx - q[0], ddy = cy - q[1], ddz = cz - q[2];
-          const double dd = fma(ddz, ddz, fma(ddy, ddy, ddx * ddx));
+          const double dd = box_d2(ddx, box_yz2(ddy, ddz));
           const double big = 2.0 * q[3];
           if (dd < big * big) {
             const double w = kernel_f<double>(sqrt(dd) * q[4], kid);
