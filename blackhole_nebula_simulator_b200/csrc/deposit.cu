@@ -252,10 +252,11 @@ __device__ __forceinline__ double log_one(const LogTarget& T, const LogParticle&
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, d);
   }
-  if (n_in >= DEP_MIN_CELLS) {
+  // (where every centre is a rounding from the edge none has a weight: trilinear too, not counted)
+  if (n_in >= DEP_MIN_CELLS && wsum > 0.0) {
     log_pass<1>(T.g, T.shells, q, rank, SIZE, kid, 1.0 / wsum, vals, T.acc, wsum, n_in, out);
   } else if (rank == 0) {
-    tri = true;
+    tri = n_in < DEP_MIN_CELLS;
     log_trilinear(T.g, q, vals, T.acc, out);
   }
   return out;
